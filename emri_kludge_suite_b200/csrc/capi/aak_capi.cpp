@@ -81,6 +81,7 @@ struct aak_ctx {
   std::vector<int32_t> tile_knot;  // 2 per tile: first knot of the tile window, knots in it
   std::vector<int64_t> kofs;       // nsrc + 1 prefix of knots (the sources' knots stay in their plans)
   std::vector<int64_t> spl_blk;    // nsrc + 1 prefix of the device spline solve's blocks
+  int spl_len = kSplineBlockShort; // knots per block of the device spline solve
   bool want_pinned = true;         // plans' knot arrays in page-locked memory
   std::vector<int32_t> bessel;
   int64_t total_samples = 0, total_tiles = 0, total_knots = 0;
@@ -238,9 +239,10 @@ int pack(aak_ctx *ctx, const std::vector<aak_params> &P, int nthreads) {
     kofs[s + 1] = kofs[s] + (ok ? (int64_t)ctx->plans[s].knot_t.size() : 0);
     bofs[s + 1] = bofs[s] + (ok ? ctx->plans[s].nmodes : 0);
   }
+  ctx->spl_len = spline_block(knots);
   ctx->spl_blk.assign(n + 1, 0);
   for (int s = 0; s < n; ++s)
-    ctx->spl_blk[s + 1] = ctx->spl_blk[s] + (ctx->status[s] == AAK_OK ? spline_blocks((int)ctx->plans[s].knot_t.size()) : 0);
+    ctx->spl_blk[s + 1] = ctx->spl_blk[s] + (ctx->status[s] == AAK_OK ? spline_blocks((int)ctx->plans[s].knot_t.size(), ctx->spl_len) : 0);
   ctx->tile_pairs.assign(2 * (size_t)n, 0);
   for (int s = 0; s < n; ++s) ctx->tile_pairs[2 * s + 1] = ctx->tile_start[s + 1] - ctx->tile_start[s];
   ctx->tile_knot.assign(2 * std::max<int64_t>(ctx->total_tiles, 1), 0);
@@ -789,7 +791,7 @@ int upload(aak_ctx *ctx, cudaStream_t st, bool wait_pinned = true) {
       return r;
   }
   // spline coefficients of every source, solved on the device
-  launch_spline_coeffs(ctx->d_src.ptr, n, ctx->d_spl_blk.ptr, ctx->spl_blk[n], ctx->d_knot_t.ptr, ctx->d_knot_y.ptr,
+  launch_spline_coeffs(ctx->d_src.ptr, n, ctx->d_spl_blk.ptr, ctx->spl_blk[n], ctx->spl_len, ctx->d_knot_t.ptr, ctx->d_knot_y.ptr,
                        ctx->d_knot_c.ptr, st);
   if ((r = cuda_ok(cudaGetLastError())) != AAK_OK) return r;
   // copies from page-locked memory run asynchronously: finish them before the
@@ -881,7 +883,7 @@ int run_graph(aak_ctx *ctx, double *hI, double *hII, int precision, cudaStream_t
     // the whole dense stage: natural-spline solve of every source's knots
     // (idempotent: the same knots give the same coefficients), then the clears
     // and the waveform kernel
-    launch_spline_coeffs(ctx->d_src.ptr, ctx->nsrc, ctx->d_spl_blk.ptr, ctx->spl_blk[ctx->nsrc], ctx->d_knot_t.ptr,
+    launch_spline_coeffs(ctx->d_src.ptr, ctx->nsrc, ctx->d_spl_blk.ptr, ctx->spl_blk[ctx->nsrc], ctx->spl_len, ctx->d_knot_t.ptr,
                          ctx->d_knot_y.ptr, ctx->d_knot_c.ptr, ctx->cap_stream);
     launch_dense(bv, ctx->num_sms, ctx->cap_stream, nullptr, precision);
     const cudaError_t launch_err = cudaGetLastError();
@@ -1627,7 +1629,7 @@ int aak_batch_run_noalloc(aak_ctx *ctx, void *d_plan, int64_t plan_bytes, int64_
       return r;
   }
   launch_spline_coeffs(reinterpret_cast<const SourceDesc *>(base), ctx->nsrc, reinterpret_cast<const int64_t *>(base + o_sb),
-                       ctx->spl_blk[ctx->nsrc], reinterpret_cast<const double *>(base + o_kt),
+                       ctx->spl_blk[ctx->nsrc], ctx->spl_len, reinterpret_cast<const double *>(base + o_kt),
                        reinterpret_cast<const double4 *>(base + o_ky), reinterpret_cast<double4 *>(base + o_kc), st);
   if ((r = cuda_ok(cudaGetLastError())) != AAK_OK) return r;
   if (ctx->want_pinned && (r = cuda_ok(cudaStreamSynchronize(st))) != AAK_OK) return r;  // host arrays reusable on return

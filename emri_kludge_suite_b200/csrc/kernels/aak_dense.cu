@@ -2110,12 +2110,12 @@ __global__ void __launch_bounds__(128) k_spline_coeffs(const SourceDesc *src, in
   }
   // interior unknowns 1 .. n-2; this block owns [a, e), the widened window is [wa, wb)
   const int b = (int)(g - blk_start[s]);
-  const int a = 1 + b * kSplineBlock, e = min(a + kSplineBlock, n - 1);
+  const int a = 1 + b * kSplineBlockLong, e = min(a + kSplineBlockLong, n - 1);
   if (a == 1) c[0] = zero;
   if (e == n - 1) c[n - 1] = zero;
   const int wa = max(1, a - kSplineHalo), wb = min(n - 1, e + kSplineHalo);
-  double cp[kSplineBlock + kSplineHalo];
-  double4 dp[kSplineBlock + kSplineHalo];
+  double cp[kSplineBlockLong + kSplineHalo];
+  double4 dp[kSplineBlockLong + kSplineHalo];
   double cprev = 0.0;
   double4 dprev = zero;
   double inv_h0 = 1.0 / (x[wa] - x[wa - 1]);
@@ -2147,11 +2147,111 @@ __global__ void __launch_bounds__(128) k_spline_coeffs(const SourceDesc *src, in
     if (i < e) c[i] = v;
   }
 }
+
+// The same solve with four lanes a block, one per component, and blocks of
+// kSplineBlockShort.  One thread per 256-knot block leaves a batch of a few
+// sources waiting for a serial chain of 336 steps, each with two divisions and
+// a round trip to memory on it.  Here a step's chain is one division (each
+// lane repeats the factorisation, which depends on the knot times alone; the
+// intervals' reciprocals leave the chain, one lane dividing for each of the
+// next four), the knots are read kAhead steps before they are used, and the
+// factors wait in shared memory.  Every unknown takes the operations of the
+// long-block solve in its order.  Bound by the latency of the chain: 1e5 knots
+// 320 -> 10 us; block lengths of 32 to 96 differ by less than 10 %.
+constexpr int kQuadThreads = 32;
+constexpr int kQuadBlocks = kQuadThreads / 4;  // knot blocks of one CTA
+constexpr int kQuadKept = kSplineBlockShort + kSplineHalo;
+__global__ void __launch_bounds__(kQuadThreads) k_spline_coeffs_quad(const SourceDesc *src, int nsrc,
+                                                                     const int64_t *blk_start, int64_t total_blocks,
+                                                                     const double *knot_t, const double4 *knot_y,
+                                                                     double4 *knot_c) {
+  __shared__ double s_cp[kQuadKept][kQuadBlocks];
+  __shared__ double s_dp[kQuadKept][kQuadThreads];
+  constexpr int kAhead = 4;
+  const int qd = threadIdx.x >> 2, comp = threadIdx.x & 3;
+  const int64_t g = (int64_t)blockIdx.x * kQuadBlocks + qd;
+  if (g >= total_blocks) return;
+  const int s = find_source(blk_start, nsrc, g);
+  const SourceDesc &d = src[s];
+  if (d.status != 0) return;  // a failed source has no knots
+  const int n = d.n_knots;
+  const double *x = knot_t + d.knot_offset;
+  const double *y = reinterpret_cast<const double *>(knot_y + d.knot_offset) + comp;
+  double *c = reinterpret_cast<double *>(knot_c + d.knot_offset) + comp;
+  if (n < 3) {
+    for (int i = 0; i < n; ++i) c[4 * i] = 0.0;
+    return;
+  }
+  const int b = (int)(g - blk_start[s]);
+  const int a = 1 + b * kSplineBlockShort, e = min(a + kSplineBlockShort, n - 1);
+  if (a == 1) c[0] = 0.0;
+  if (e == n - 1) c[4 * (int64_t)(n - 1)] = 0.0;
+  const int wa = max(1, a - kSplineHalo), wb = min(n - 1, e + kSplineHalo);
+  const unsigned quad = 0xfu << (threadIdx.x & 28);  // the block's four lanes
+  double cprev = 0.0, dprev = 0.0;
+  double x1 = x[wa], h0 = x1 - x[wa - 1], inv_h0 = 1.0 / h0;
+  double y0 = y[4 * (int64_t)(wa - 1)], y1 = y[4 * (int64_t)wa];
+  double xn[kAhead], yn[kAhead];  // knots i + 1 .. i + kAhead
+#pragma unroll
+  for (int k = 0; k < kAhead; ++k) {
+    const int64_t j = min(wa + 1 + k, n - 1);
+    xn[k] = x[j];
+    yn[k] = y[4 * j];
+  }
+  for (int i0 = wa; i0 < wb; i0 += kAhead) {
+    double xc[kAhead], yc[kAhead];
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) {
+      xc[k] = xn[k];
+      yc[k] = yn[k];
+      const int64_t j = min(i0 + 1 + kAhead + k, n - 1);
+      xn[k] = x[j];
+      yn[k] = y[4 * j];
+    }
+    // lane k of the four divides for interval k (intervals past the window repeat the last knot: not used)
+    const double hk = comp == 0 ? xc[0] - x1 : comp == 1 ? xc[1] - xc[0] : comp == 2 ? xc[2] - xc[1] : xc[3] - xc[2];
+    const double rk = 1.0 / hk;
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) {
+      const int i = i0 + k;
+      const double inv_h1 = __shfl_sync(quad, rk, k, 4);
+      if (i >= wb) continue;
+      const double h1 = xc[k] - x1;
+      const double inv = 1.0 / (2.0 * (h0 + h1) - h0 * cprev);
+      const double cc = (i + 1 < wb) ? h1 * inv : 0.0;
+      const double y2 = yc[k];
+      const double dd = (3.0 * ((y2 - y1) * inv_h1 - (y1 - y0) * inv_h0) - h0 * dprev) * inv;
+      if (i >= a) {
+        if (comp == 0) s_cp[i - a][qd] = cc;
+        s_dp[i - a][threadIdx.x] = dd;
+      }
+      cprev = cc;
+      dprev = dd;
+      inv_h0 = inv_h1;
+      h0 = h1;
+      x1 = xc[k];
+      y0 = y1;
+      y1 = y2;
+    }
+  }
+  __syncwarp(quad);  // lane 0's factors
+  double v = s_dp[wb - 1 - a][threadIdx.x];  // c at wb - 1 (its neighbour beyond the window taken as 0)
+  if (wb - 1 < e) c[4 * (int64_t)(wb - 1)] = v;
+  for (int i = wb - 2; i >= a; --i) {
+    v = s_dp[i - a][threadIdx.x] - s_cp[i - a][qd] * v;
+    if (i < e) c[4 * (int64_t)i] = v;
+  }
+}
 }  // namespace
 
-void launch_spline_coeffs(const SourceDesc *src, int nsrc, const int64_t *blk_start, int64_t total_blocks,
+void launch_spline_coeffs(const SourceDesc *src, int nsrc, const int64_t *blk_start, int64_t total_blocks, int block,
                           const double *knot_t, const double4 *knot_y, double4 *knot_c, cudaStream_t stream) {
   if (total_blocks <= 0) return;
+  if (block == kSplineBlockShort) {
+    k_spline_coeffs_quad<<<(unsigned)((total_blocks + kQuadBlocks - 1) / kQuadBlocks), kQuadThreads, 0, stream>>>(
+        src, nsrc, blk_start, total_blocks, knot_t, knot_y, knot_c);
+    return;
+  }
   const int threads = 128;
   k_spline_coeffs<<<(unsigned)((total_blocks + threads - 1) / threads), threads, 0, stream>>>(
       src, nsrc, blk_start, total_blocks, knot_t, knot_y, knot_c);
