@@ -85,6 +85,7 @@ struct aak_ctx {
   bool want_pinned = true;         // plans' knot arrays in page-locked memory
   std::vector<int32_t> bessel;
   int64_t total_samples = 0, total_tiles = 0, total_knots = 0;
+  int64_t small_tiles = 0;  // first items of the queue: the tiles of the sources of at most kSmallTiles tiles
   int32_t max_nmodes = 0;
   int64_t out_stride = 0;  // > 0: source s writes at s * out_stride (FFT-padded rows)
   bool uploaded = false;
@@ -101,6 +102,9 @@ struct aak_ctx {
   DevBuf<unsigned long long> d_counter;   // [0] work-queue head, [1] device status word
   DevBuf<TilePrep> d_tile_prep;           // tile pre-pass: per-tile parameters
   DevBuf<unsigned char> d_tile_tab;       //   and per-tile Taylor tables
+  DevBuf<unsigned char> d_tile_seg;       // FP64: polynomial segments, one slot per tile
+  DevBuf<int32_t> d_seg_ctl;              //   their counters,
+  DevBuf<double> d_frozen;                //   and the phases at i_plunge, 3 per source
   DevBuf<double> d_out;  // outputs for the host-buffer entry points
   // batched device solve of the Kerr -> AK map (opt-in: parmap_device)
   bool parmap_device = false;
@@ -308,23 +312,26 @@ int pack(aak_ctx *ctx, const std::vector<aak_params> &P, int nthreads) {
   // after the taper's end, min(vlength, i_plunge + i_buffer)).
   ctx->queue.assign(std::max<int64_t>(ctx->total_tiles, 1), QueueItem{});
   int64_t q = 0;
-  for (int k = 0; k < maxT; ++k)
-    for (int s = 0; s < n; ++s)
-      if (k < T[s]) {
-        const SourceDesc &d = ctx->descs[s];
-        const int lt = (k < T[s] - head[s]) ? head[s] + k : T[s] - 1 - k;
-        const int64_t g = ctx->tile_start[s] + lt;
-        const long long neff = std::min<long long>(d.vlength, (long long)d.i_plunge + (long long)d.i_buffer);
-        QueueItem &it = ctx->queue[q++];
-        it.g = (int32_t)g;
-        it.s = s;
-        it.lt = lt;
-        it.k0 = ctx->tile_knot[2 * g];
-        it.nk = ctx->tile_knot[2 * g + 1];
-        it.knot = d.knot_offset + it.k0;
-        it.flags = (d.status != 0 ? kQueueFailed | kQueueNoWave : 0) |
-                   ((long long)lt * kTileSamples >= neff ? kQueueNoWave : 0);
-      }
+  for (int small = 1; small >= 0; --small) {  // the small sources' tiles first (kSmallTiles)
+    for (int k = 0; k < maxT; ++k)
+      for (int s = 0; s < n; ++s)
+        if (k < T[s] && (T[s] <= kSmallTiles) == (small == 1)) {
+          const SourceDesc &d = ctx->descs[s];
+          const int lt = (k < T[s] - head[s]) ? head[s] + k : T[s] - 1 - k;
+          const int64_t g = ctx->tile_start[s] + lt;
+          const long long neff = std::min<long long>(d.vlength, (long long)d.i_plunge + (long long)d.i_buffer);
+          QueueItem &it = ctx->queue[q++];
+          it.g = (int32_t)g;
+          it.s = s;
+          it.lt = lt;
+          it.k0 = ctx->tile_knot[2 * g];
+          it.nk = ctx->tile_knot[2 * g + 1];
+          it.knot = d.knot_offset + it.k0;
+          it.flags = (d.status != 0 ? kQueueFailed | kQueueNoWave : 0) |
+                     ((long long)lt * kTileSamples >= neff ? kQueueNoWave : 0);
+        }
+    if (small == 1) ctx->small_tiles = q;
+  }
   ctx->uploaded = false;
   return AAK_OK;
 }
@@ -808,6 +815,35 @@ BatchView batch_view(aak_ctx *ctx, double *hI, double *hII, double *t, double *t
 // TilePrep and one Taylor-table slot per tile), grown as needed, set in bv.
 void drop_graph(aak_ctx *ctx);
 
+// The buffers of the FP64 polynomial segments, grown as needed, set in bv: the
+// aggregates and the list of direct tiles take the look-back records' and
+// flags' memory, which the segments' launches do not use.
+int tile_segments(aak_ctx *ctx, BatchView &bv) {
+  const int64_t tiles = std::max<int64_t>(ctx->total_tiles, 1);
+  const void *s0 = ctx->d_tile_seg.ptr, *c0 = ctx->d_seg_ctl.ptr;
+  int r;
+  if ((r = ctx->d_tile_seg.reserve(tiles * kSegSlotBytes)) != AAK_OK ||
+      (r = ctx->d_seg_ctl.reserve(seg_ctl_words(ctx->nsrc))) != AAK_OK || (r = ctx->d_frozen.reserve(3 * (size_t)ctx->nsrc)) != AAK_OK)
+    return r;
+  if (ctx->d_tile_seg.ptr != s0 || ctx->d_seg_ctl.ptr != c0) drop_graph(ctx);
+  bv.tile_seg = ctx->d_tile_seg.ptr;
+  bv.seg_ctl = ctx->d_seg_ctl.ptr;
+  bv.frozen = ctx->d_frozen.ptr;
+  bv.tile_agg = reinterpret_cast<SegAgg *>(ctx->d_link.ptr);
+  bv.direct_list = ctx->d_flag.ptr;
+  return AAK_OK;
+}
+
+// Kernels of one dense launch: the in-tile kernel alone; with the pre-pass,
+// split: tile parameters, tables, waveform; FP64: the in-tile kernel for the
+// small sources, and for the others segments, carries (with the tables), the
+// direct tiles and the segments' waveform.
+int dense_launches(const aak_ctx *ctx, int precision) {
+  if (!wave_variant(precision == 1, ctx->variant[precision]).pre) return 1;
+  if (precision == 1) return 3;
+  return (ctx->small_tiles > 0 ? 1 : 0) + (ctx->small_tiles < ctx->total_tiles ? 4 : 0);
+}
+
 int tile_tables(aak_ctx *ctx, int precision, BatchView &bv) {
   const int64_t tiles = std::max<int64_t>(ctx->total_tiles, 1);
   const int64_t slot = tile_table_slot_bytes(ctx->max_nmodes, precision == 1);
@@ -820,7 +856,7 @@ int tile_tables(aak_ctx *ctx, int precision, BatchView &bv) {
   bv.tile_prep = ctx->d_tile_prep.ptr;
   bv.tile_tab = ctx->d_tile_tab.ptr;
   bv.tab_slot = slot;
-  return AAK_OK;
+  return precision == 0 ? tile_segments(ctx, bv) : AAK_OK;
 }
 
 int run(aak_ctx *ctx, double *hI, double *hII, double *t, double *traj, int64_t traj_stride, int precision,
@@ -837,7 +873,7 @@ int run(aak_ctx *ctx, double *hI, double *hII, double *t, double *traj, int64_t 
   if (ctx->profile && !ctx->ev[0])
     for (auto &e : ctx->ev) cudaEventCreate(&e);
   launch_dense(bv, ctx->num_sms, st, ctx->profile ? ctx->ev : nullptr, precision);
-  ctx->last_launches = (bv.tile_prep && wave_variant(precision == 1, bv.variant).pre) ? 3 : 1;
+  ctx->last_launches = bv.tile_prep ? dense_launches(ctx, precision) : 1;
   return cuda_ok(cudaGetLastError());
 }
 
@@ -904,8 +940,7 @@ int run_graph(aak_ctx *ctx, double *hI, double *hII, int precision, cudaStream_t
     ctx->g_gen = ctx->upload_gen;
     ctx->g_variant = ctx->variant[precision];
   }
-  // spline solve, tile parameters and tables (with the pre-pass), waveform kernel
-  ctx->last_launches = wave_variant(precision == 1, ctx->variant[precision]).pre ? 4 : 2;
+  ctx->last_launches = 1 + dense_launches(ctx, precision);  // with the spline solve
   return cuda_ok(cudaGraphLaunch(ctx->gexec, st));
 }
 
@@ -916,6 +951,7 @@ BatchView batch_view(aak_ctx *ctx, double *hI, double *hII, double *t, double *t
   bv.total_tiles = ctx->total_tiles;
   bv.tile_start = ctx->d_tile_start.ptr;
   bv.queue = ctx->d_queue.ptr;
+  bv.small_tiles = ctx->small_tiles;
   bv.tile_knot = ctx->d_tile_knot.ptr;
   bv.knot_t = ctx->d_knot_t.ptr;
   bv.knot_y = ctx->d_knot_y.ptr;
@@ -951,10 +987,12 @@ int run_phase(aak_ctx *ctx, double *out, int64_t stride, cudaStream_t st) {
   if ((r = ctx->d_tile_prep.reserve(std::max<int64_t>(ctx->total_tiles, 1))) != AAK_OK) return r;
   if (ctx->d_tile_prep.ptr != p0) drop_graph(ctx);
   bv.tile_prep = ctx->d_tile_prep.ptr;
+  if ((r = tile_segments(ctx, bv)) != AAK_OK) return r;
   if (ctx->profile && !ctx->ev[0])
     for (auto &e : ctx->ev) cudaEventCreate(&e);
   launch_phase(bv, ctx->num_sms, st, ctx->profile ? ctx->ev : nullptr);
-  ctx->last_launches = 3;
+  // small sources: tile parameters, phase pass, freeze; the others: segments, carries, phase pass
+  ctx->last_launches = (ctx->small_tiles > 0 ? 3 : 0) + (ctx->small_tiles < ctx->total_tiles ? 3 : 0);
   return cuda_ok(cudaGetLastError());
 }
 
@@ -1480,6 +1518,9 @@ void aak_ctx_destroy(aak_ctx *c) {
     c->d_tile_pairs.release();
     c->d_queue.release();
     c->d_spl_blk.release();
+    c->d_tile_seg.release();
+    c->d_seg_ctl.release();
+    c->d_frozen.release();
     c->d_knot_t.release();
     c->d_knot_y.release();
     c->d_knot_c.release();

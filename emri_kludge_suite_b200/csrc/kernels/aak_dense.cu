@@ -14,10 +14,12 @@
 #include <cuda_runtime.h>
 #include <math.h>
 
+#include <algorithm>
 #include <atomic>
 #include <type_traits>
 #include <utility>
 
+#include "../segment_fit.hpp"
 #include "aak_dense.cuh"
 
 namespace aak {
@@ -835,12 +837,14 @@ __device__ __forceinline__ double taylor_tail(double q, int nmodes, int K) {
   for (int k = 1; k <= K + 1; ++k) t *= q / (double)k;
   return t;
 }
+// (FP64: the powers over factorials built once, for all the options)
 __device__ __forceinline__ int taylor_terms_fp64(double q, int nmodes) {
   if (!(q <= 1.0)) return 0;
-  const int opts[5] = {4, 5, 6, 8, 10};
-  for (int i = 0; i < 5; ++i)
-    if (taylor_tail(q, nmodes, opts[i]) < 1e-17) return opts[i];
-  return 0;
+  const double lim = 1e-17 / (8.0 * nmodes * exp(q));
+  const double q2 = q * q, q4 = q2 * q2;
+  const double t5 = q4 * q * (1. / 120.), t6 = t5 * q * (1. / 6.), t7 = t6 * q * (1. / 7.);
+  const double t9 = t7 * q2 * (1. / 72.), t11 = t9 * q2 * (1. / 110.);
+  return t5 < lim ? 4 : t6 < lim ? 5 : t7 < lim ? 6 : t9 < lim ? 8 : t11 < lim ? 10 : 0;
 }
 __device__ __forceinline__ int taylor_terms_fp32(double q, int nmodes) {
   if (!(q <= 1.0)) return 0;
@@ -1328,13 +1332,15 @@ __global__ void __launch_bounds__(128) k_tile_params(BatchView bv) {
   bv.tile_prep[g] = P;
 }
 
+// Table row `id` of the launch: one thread a (tile, harmonic); tiles in batch
+// order, or (FP64: the launch's own tiles) in queue order.
 template <bool kSplit>
-__global__ void __launch_bounds__(128) k_tile_table(BatchView bv, int rows) {
+__device__ __forceinline__ void table_row(const BatchView &bv, int rows, int64_t id) {
   using T = typename std::conditional<kSplit, float, double>::type;
-  const int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const int64_t g = id / rows;
-  if (g >= bv.total_tiles) return;
-  const int n = (int)(id - g * rows) + 1;
+  const int64_t j = id / rows;
+  if (j >= bv.total_tiles) return;
+  const int n = (int)(id - j * rows) + 1;
+  const int64_t g = kSplit ? j : (int64_t)bv.queue[j].g;
   const TilePrep &P = bv.tile_prep[g];
   const int K = P.K;
   if (K <= 0) return;
@@ -1343,6 +1349,12 @@ __global__ void __launch_bounds__(128) k_tile_table(BatchView bv, int rows) {
   T *tab = reinterpret_cast<T *>(static_cast<unsigned char *>(bv.tile_tab) + g * bv.tab_slot);
   build_taylor_row<T>(tab, P.stride, n, d.nmodes, P.ec, K, (n <= d.nmodes) ? bv.bessel_start[d.bessel_offset + n - 1] : 0);
 }
+template <bool kSplit>
+__global__ void __launch_bounds__(128) k_tile_table(BatchView bv, int rows) {
+  table_row<kSplit>(bv, rows, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
+}
+
+#include "aak_segments.cuh"
 
 // ------------------------------------------------------------------ waveform kernel
 // Samples per thread whose harmonic sums run side by side (divides kTileChunks).
@@ -1370,8 +1382,9 @@ constexpr size_t kWaveDynSmem = (size_t)kDynVals * kTileSamples * sizeof(double)
 // sample of each source runs through phase 1, the harmonic sums are skipped,
 // and the tile's samples are written to bv.phase_out as t, phase_r,
 // phase_theta, phase_phi, omega_r, omega_theta, omega_phi, e (the per-sample
-// packing of GenPhase, AAKPhase.cc:346-355).  The phases of the samples
-// after the plunge buffer are frozen afterwards by k_phase_freeze.
+// packing of GenPhase, AAKPhase.cc:346-355).  The samples after the plunge
+// buffer take the phases of sample i_plunge (bv.frozen, summed before the
+// kernel; the small sources': k_phase_freeze after it).
 // kMode 2, the phase grid of the frequency-domain TDI (PNevolutionTDI,
 // AAKTDI.cc:311-469): the same pass writes kTdiRows rows (TdiRow order).
 // kPre (waveform mode with the tile pre-pass): each tile's source record,
@@ -1413,10 +1426,12 @@ __device__ __forceinline__ void issue_stage(const BatchView &bv, const QueueItem
   win[2] = toff;
 }
 
-template <bool kSplit, int kMode = 0, bool kPre = false, int kJointT = 0, int kMinB = AAK_WAVE_MIN_BLOCKS>
+template <bool kSplit, int kMode = 0, bool kPre = false, int kJointT = 0, int kMinB = AAK_WAVE_MIN_BLOCKS,
+          bool kCarry = false>
 __global__ void __launch_bounds__(kTileThreads, kMinB) k_waveform(BatchView bv) {
   constexpr bool kPhase = kMode != 0, kTdi = kMode == 2;
   static_assert(!kPre || kMode != 2, "the pre-pass serves the waveform and phase modes");
+  static_assert(!kCarry || (kPre && !kSplit && kMode != 2), "carries from the segments serve FP64 batches");
   extern __shared__ double s_dyn[];  // [kDynVals][kTileSamples]
   __shared__ double red[2][3][kTileThreads / 32];  // warp totals of the forward and backward scans
   __shared__ long long s_tile;
@@ -1452,12 +1467,52 @@ __global__ void __launch_bounds__(kTileThreads, kMinB) k_waveform(BatchView bv) 
   // ahead cannot stall the chains.  (Fetching at the start of the tile was
   // slower: the CTAs then hold twice as many items, and more of them start
   // while their chain predecessors are still running.)
-  if (tid == 0) s_tile = (long long)atomicAdd(bv.work_counter, 1ull);
+  const auto fetch = [&]() -> long long {
+    if constexpr (kCarry && !kPhase) return atomicAdd(bv.seg_ctl + kCtlDirectQueue, 1);
+    else if constexpr (kCarry) return atomicAdd(bv.seg_ctl + kCtlQueue, 1);
+    else return (long long)atomicAdd(bv.work_counter, 1ull);
+  };
+  const long long items = (kCarry && !kPhase) ? (long long)bv.seg_ctl[kCtlDirectCount] : (long long)bv.total_tiles;
+  if (tid == 0) s_tile = fetch();
   __syncthreads();
   for (;;) {
-    const long long j = s_tile;
+    long long j = s_tile;
     __syncthreads();
-    if (j >= bv.total_tiles) break;
+    if (j >= items) break;
+    if constexpr (kCarry && !kPhase) j = bv.direct_list[j];
+    if constexpr (kCarry && kPhase) {
+      // a tile of polynomial segments: its record, head and coefficients by
+      // bulk copies, its rows straight from them
+      const QueueItem &q = bv.queue[j];
+      const int mode = tile_head(bv, q.g)->mode;
+      if (mode > 0) {
+        if (tid == 0) {
+          fence_proxy_async_smem();
+          const uint32_t nc = (uint32_t)sizeof(TileHead) + 4u * (uint32_t)seg_doubles(mode == 4 ? 4 : 7, true) * 8u;
+          mbar_arrive_expect_tx(&s_mbar[0], (uint32_t)sizeof(SourceDesc) + nc);
+          bulk_copy_g2s(&s_desc, bv.src + q.s, (uint32_t)sizeof(SourceDesc), &s_mbar[0]);
+          bulk_copy_g2s(s_dyn, tile_head(bv, q.g), nc, &s_mbar[0]);
+        }
+        if (tid == 32) s_tile = fetch();
+        const bool ok = mbar_wait_bounded(&s_mbar[0], ph0);
+        ph0 ^= 1u;
+        if (ok) {
+          const TileHead &H = *reinterpret_cast<const TileHead *>(s_dyn);
+          const double2 *co = reinterpret_cast<const double2 *>(reinterpret_cast<const unsigned char *>(s_dyn) + sizeof(TileHead));
+          const int st = q.lt * kTileSamples, en = min(st + kTileSamples, s_desc.vlength);
+          if (mode == 4) phase_rows<4>(bv, s_desc, H, co, st, en, bv.frozen + 3 * q.s);
+          else phase_rows<7>(bv, s_desc, H, co, st, en, bv.frozen + 3 * q.s);
+        }
+        if (__syncthreads_or(!ok)) {
+          if (tid == 0) {
+            atomicExch(bv.device_status, 1u);
+            if (bv.status_report) atomicExch(bv.status_report, 1u);
+          }
+          return;
+        }
+        continue;
+      }
+    }
     // kPre (batches, which have queue items): the tile's record, parameters
     // and knot window are requested first thing, straight from its item
     bool empty = false;
@@ -1490,8 +1545,8 @@ __global__ void __launch_bounds__(kTileThreads, kMinB) k_waveform(BatchView bv) 
       }
       if (tid == 0) {
         const double zero[3] = {0.0, 0.0, 0.0};
-        publish_aggregate(bv, g, zero, 0.0, false);
-        s_tile = (long long)atomicAdd(bv.work_counter, 1ull);
+        if (!kCarry) publish_aggregate(bv, g, zero, 0.0, false);
+        s_tile = fetch();
       }
       __syncthreads();
       continue;
@@ -1591,7 +1646,7 @@ __global__ void __launch_bounds__(kTileThreads, kMinB) k_waveform(BatchView bv) 
     // (raw rate before it not positive) needs the chain's clamped Phidot
     // first: it waits for its whole prefix before phase 1.
     const bool needC = dir > 0 && !(s_rb[1] > 0.0);
-    if (needC) {
+    if (!kCarry && needC) {
       if (tid < 32) {
         double hi[3], lo[3], C;
         look_back_warp(bv, c, 1, hi, lo, C);
@@ -1605,7 +1660,7 @@ __global__ void __launch_bounds__(kTileThreads, kMinB) k_waveform(BatchView bv) 
       }
       __syncthreads();
     }
-    const double Cin = needC ? s_cy[6] : 0.0;
+    const double Cin = needC ? (kCarry ? tile_head(bv, g)->C : s_cy[6]) : 0.0;
 #if !AAK_TABLE_AFTER_SCAN
     // Taylor table rows (one thread per harmonic); its barrier is the first one of phase 1
     if (!kPhase && !kPre && K > 0 && !bv.trajectory_only)
@@ -1781,10 +1836,15 @@ __global__ void __launch_bounds__(kTileThreads, kMinB) k_waveform(BatchView bv) 
       if (bv.traj_out) bv.traj_out[7 * bv.traj_stride + d.out_offset + i] = nuv[k];
     }
     __syncthreads();
-    if (tid == 32) s_tile = (long long)atomicAdd(bv.work_counter, 1ull);  // the next tile, read after the loop's barrier
+    if (tid == 32) s_tile = fetch();  // the next tile, read after the loop's barrier
     // ---------------- chain carries: warp 0 publishes this tile's aggregate,
     // looks back for the exclusive prefix and publishes the inclusive record
-    if (tid < 32) {
+    if (kCarry) {  // the carry is known: summed before this kernel
+      if (tid < 3) {
+        s_cy[tid] = tile_head(bv, g)->hi[tid];
+        s_cy[3 + tid] = tile_head(bv, g)->lo[tid];
+      }
+    } else if (tid < 32) {
       const bool hasF = lim - 1 >= max(c.start, d.i0);  // forward output samples in the tile
       double hi[3] = {0, 0, 0}, lo[3] = {0, 0, 0}, C = 0.0;
       if (needC) {
@@ -1830,7 +1890,24 @@ __global__ void __launch_bounds__(kTileThreads, kMinB) k_waveform(BatchView bv) 
     // the phases of this thread's own samples: X0 + carry + local part
     // (forward), X0 - (carry + increments after the sample) (backward)
     {
-      const double cy_hi[3] = {s_cy[0], s_cy[1], s_cy[2]}, cy_lo[3] = {s_cy[3], s_cy[4], s_cy[5]};
+      double cy_hi[3] = {s_cy[0], s_cy[1], s_cy[2]}, cy_lo[3] = {s_cy[3], s_cy[4], s_cy[5]};
+      if constexpr (kCarry && kPhase) {  // the signed sums: as the chain's own below
+        if (dir < 0)
+          for (int q = 0; q < 3; ++q) {
+            cy_hi[q] = -cy_hi[q];
+            cy_lo[q] = -cy_lo[q];
+          }
+      }
+      // FP64 waveforms take their phases modulo 2 pi (as the segments do), unless the trajectory is wanted
+      const bool mod = !kSplit && !kPhase && !bv.traj_out && !bv.trajectory_only;
+      double base_hi[3], base_lo[3];
+      if constexpr (!kSplit && !kPhase) {
+        for (int q = 0; q < 3; ++q) {
+          base_hi[q] = (dir < 0 && !kCarry) ? -cy_hi[q] : cy_hi[q];
+          base_lo[q] = (dir < 0 && !kCarry) ? -cy_lo[q] : cy_lo[q];
+          if (!kCarry) reduced_base(X0[q], base_hi[q], base_lo[q]);
+        }
+      }
       for (int ch = 0; ch < kTileChunks; ++ch) {
         const int i = c.start + ch * kTileThreads + tid;
         const int sl = ch * kTileThreads + tid;
@@ -1840,6 +1917,13 @@ __global__ void __launch_bounds__(kTileThreads, kMinB) k_waveform(BatchView bv) 
         for (int qq = 0; qq < 3; ++qq) {
           double *sv = s_dyn + (2 + qq) * kTileSamples;
           const double v = sv[sl];
+          if constexpr (!kSplit && !kPhase) {
+            if (mod) {  // the phase modulo 2 pi, from the reduced base
+              X[qq] = (i == d.i0) ? v : base_hi[qq] + (base_lo[qq] + ((i > d.i0) ? v : v - runB[qq]));
+              sv[sl] = X[qq];
+              continue;
+            }
+          }
           if (i > d.i0) X[qq] = X0[qq] + (cy_hi[qq] + (cy_lo[qq] + v));
           else if (i == d.i0) X[qq] = v;
           else X[qq] = X0[qq] - (cy_hi[qq] + (cy_lo[qq] + (runB[qq] - v)));
@@ -1866,6 +1950,8 @@ __global__ void __launch_bounds__(kTileThreads, kMinB) k_waveform(BatchView bv) 
           const int64_t o = d.out_offset + i;
           const int64_t st = bv.phase_stride;
           const double Pd = sv_nu[sl], gd = sv_gd[sl], ad = sv_om[sl];
+          if (kCarry && is_frozen(d, i))
+            for (int qq = 0; qq < 3; ++qq) X[qq] = bv.frozen[3 * c.s + qq];
           bv.phase_out[o] = sample_time(d, i);
           bv.phase_out[st + o] = X[1];
           bv.phase_out[2 * st + o] = X[1] + X[0];
@@ -2267,11 +2353,14 @@ void launch_dense_fp64(const BatchView &bv, int num_sms, cudaStream_t stream, cu
   launch_dense(bv, num_sms, stream, ev, 0);
 }
 
-template <bool kSplit, size_t... I>
-void set_variant_smem(int bytes, std::index_sequence<I...>) {
-  (cudaFuncSetAttribute(k_waveform<kSplit, 0, wave_variant(kSplit, (int)I).pre, wave_variant(kSplit, (int)I).joint,
-                                   wave_variant(kSplit, (int)I).min_blocks>,
+template <size_t... I>
+void set_variant_smem(int bytes, int seg_bytes, std::index_sequence<I...>) {
+  (cudaFuncSetAttribute(k_waveform<true, 0, wave_variant(true, (int)I).pre, wave_variant(true, (int)I).joint,
+                                   wave_variant(true, (int)I).min_blocks>,
                         cudaFuncAttributeMaxDynamicSharedMemorySize, bytes),
+   ...);
+  (cudaFuncSetAttribute(k_wave_segments<std::max(wave_variant(false, (int)I).joint, 1), wave_variant(false, (int)I).min_blocks>,
+                        cudaFuncAttributeMaxDynamicSharedMemorySize, seg_bytes),
    ...);
 }
 
@@ -2284,10 +2373,12 @@ void prepare_dense_launch() {
     const int most = (int)(kWaveDynSmem + (size_t)kTabModes * kRowD * sizeof(double));
     cudaFuncSetAttribute(k_waveform<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
     cudaFuncSetAttribute(k_waveform<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-    set_variant_smem<true>(most, std::make_index_sequence<kNumVariants>{});
-    set_variant_smem<false>(most, std::make_index_sequence<kNumVariants>{});
-    cudaFuncSetAttribute(k_waveform<false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWaveDynSmem);
+    set_variant_smem(most, 2 * (int)(kSegStageBase + (size_t)kTabModes * kRowD * sizeof(double)),
+                     std::make_index_sequence<kNumVariants>{});
+    cudaFuncSetAttribute(k_waveform<false, 0, true, 1, 3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
     cudaFuncSetAttribute(k_waveform<false, 1, true, 0, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)kWaveDynSmem);
+    cudaFuncSetAttribute(k_waveform<false, 1, true, 0, 3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)kWaveDynSmem);
     cudaFuncSetAttribute(k_waveform<false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWaveDynSmem);
     attrs_set.fetch_or(bit);
@@ -2305,39 +2396,92 @@ void launch_persistent(K kernel, const BatchView &bv, int num_sms, size_t dyn, c
   kernel<<<grid, kTileThreads, dyn, stream>>>(bv);
 }
 
-template <bool kSplit, int v>
-void launch_variant(const BatchView &bv, int num_sms, size_t dyn, cudaStream_t stream) {
-  constexpr WaveVariant w = wave_variant(kSplit, v);
-  launch_persistent(k_waveform<kSplit, 0, w.pre, w.joint, w.min_blocks>, bv, num_sms, dyn, stream);
+template <int v>
+void launch_split_variant(const BatchView &bv, int num_sms, size_t dyn, cudaStream_t stream) {
+  constexpr WaveVariant w = wave_variant(true, v);
+  launch_persistent(k_waveform<true, 0, w.pre, w.joint, w.min_blocks>, bv, num_sms, dyn, stream);
+}
+template <size_t... I>
+void launch_split_index(int v, const BatchView &bv, int num_sms, size_t dyn, cudaStream_t stream,
+                        std::index_sequence<I...>) {
+  ((v == (int)I ? launch_split_variant<(int)I>(bv, num_sms, dyn, stream) : void()), ...);
 }
 
-template <bool kSplit, size_t... I>
-void launch_variant_index(int v, const BatchView &bv, int num_sms, size_t dyn, cudaStream_t stream,
-                          std::index_sequence<I...>) {
-  ((v == (int)I ? launch_variant<kSplit, (int)I>(bv, num_sms, dyn, stream) : void()), ...);
+// The segments' waveform kernel as a persistent grid of every CTA that fits.
+template <int v>
+void launch_seg_variant(const BatchView &bv, int num_sms, int rows, cudaStream_t stream) {
+  constexpr WaveVariant w = wave_variant(false, v);
+  constexpr int J = std::max(w.joint, 1);
+  const int stage = (int)(kSegStageBase + (size_t)rows * kRowD * sizeof(double));
+  int resident = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_wave_segments<J, w.min_blocks>, kTileThreads, 2 * stage);
+  resident = std::max(resident, 1);
+  const int grid = (int)std::min<int64_t>(bv.total_tiles, (int64_t)num_sms * resident);
+  k_wave_segments<J, w.min_blocks><<<grid, kTileThreads, 2 * stage, stream>>>(bv, stage);
+}
+template <size_t... I>
+void launch_seg_index(int v, const BatchView &bv, int num_sms, int rows, cudaStream_t stream, std::index_sequence<I...>) {
+  ((v == (int)I ? launch_seg_variant<(int)I>(bv, num_sms, rows, stream) : void()), ...);
+}
+
+// The segments, then the carries (with the Taylor tables of `rows` harmonics, 0: none).
+template <bool kPhase>
+void launch_segments(const BatchView &bv, int num_sms, int rows, cudaStream_t stream, cudaEvent_t *ev) {
+  cudaMemsetAsync(bv.seg_ctl, 0, seg_ctl_words(bv.nsrc) * sizeof(int32_t), stream);
+  if (ev) cudaEventRecord(ev[1], stream);
+  const int64_t tiles = bv.total_tiles, blocks = (tiles + kSegWarps - 1) / kSegWarps;
+  k_tile_segments<kPhase><<<(unsigned)std::min<int64_t>(blocks, 3 * (int64_t)num_sms), kSegWarps * 32, 0, stream>>>(bv);
+  // a block a source, and one an SM for the direct tiles
+  const int carry = std::min(std::max(bv.nsrc, num_sms), 4096);
+  const int64_t table = (tiles * rows + kSegWarps * 32 - 1) / (kSegWarps * 32);
+  k_tile_carries<<<(unsigned)(carry + table), kSegWarps * 32, 0, stream>>>(bv, carry, std::max(rows, 1));
 }
 
 template <bool kSplit>
 void launch_dense_t(const BatchView &bv, int num_sms, cudaStream_t stream, cudaEvent_t *ev) {
   if (ev) cudaEventRecord(ev[0], stream);
-  cudaMemsetAsync(bv.work_counter, 0, sizeof(unsigned long long), stream);
-  cudaMemsetAsync(bv.link_flag, 0, (size_t)bv.total_tiles * sizeof(int32_t), stream);
-  if (ev) cudaEventRecord(ev[1], stream);
   // per-sample values, then the Taylor table sized for the batch's harmonic count
   const int rows = table_rows<typename std::conditional<kSplit, float, double>::type>(
       (bv.max_nmodes > 0 && bv.max_nmodes < kTabModes) ? bv.max_nmodes : kTabModes);
   const size_t dyn = kWaveDynSmem + (size_t)rows * (kSplit ? kRowF * sizeof(float) : kRowD * sizeof(double));
   const int v = (bv.variant >= 0 && bv.variant < kNumVariants) ? bv.variant : 0;
   const bool pre = wave_variant(kSplit, v).pre && bv.tile_prep && bv.tile_tab && bv.queue && !bv.trajectory_only &&
-                   bv.tab_slot >= tile_table_slot_bytes(rows, kSplit);
+                   bv.tab_slot >= tile_table_slot_bytes(rows, kSplit) && (kSplit || bv.tile_seg);
+  const int64_t tiles = bv.total_tiles;
   prepare_dense_launch();
-  if (pre) {
-    const int64_t tiles = bv.total_tiles;
-    k_tile_params<kSplit><<<(unsigned)((tiles + 127) / 128), 128, 0, stream>>>(bv);
-    k_tile_table<kSplit><<<(unsigned)((tiles * rows + 127) / 128), 128, 0, stream>>>(bv, rows);
+  if (!kSplit && pre) {
+    // the small sources' tiles first in the queue, by the kernel that does everything inside the tiles; the rest as
+    // segments (whose list of direct tiles takes the flags' memory afterwards)
+    if (bv.small_tiles > 0) {
+      BatchView sm = bv;
+      sm.total_tiles = bv.small_tiles;
+      cudaMemsetAsync(bv.work_counter, 0, sizeof(unsigned long long), stream);
+      cudaMemsetAsync(bv.link_flag, 0, (size_t)tiles * sizeof(int32_t), stream);
+      if (ev && bv.small_tiles == tiles) cudaEventRecord(ev[1], stream);
+      if (ev && bv.small_tiles == tiles) cudaEventRecord(ev[2], stream);
+      launch_persistent(k_waveform<false>, sm, num_sms, dyn, stream);
+    }
+    if (bv.small_tiles < tiles) {
+      BatchView lg = bv;
+      lg.queue += bv.small_tiles;
+      lg.total_tiles -= bv.small_tiles;
+      launch_segments<false>(lg, num_sms, rows, stream, ev);
+      if (ev) cudaEventRecord(ev[2], stream);
+      launch_persistent(k_waveform<false, 0, true, 1, 3, true>, lg, num_sms, dyn, stream);
+      launch_seg_index(v, lg, num_sms, rows, stream, std::make_index_sequence<kNumVariants>{});
+    }
+    if (ev) cudaEventRecord(ev[3], stream);
+    return;
+  }
+  cudaMemsetAsync(bv.work_counter, 0, sizeof(unsigned long long), stream);
+  cudaMemsetAsync(bv.link_flag, 0, (size_t)bv.total_tiles * sizeof(int32_t), stream);
+  if (ev) cudaEventRecord(ev[1], stream);
+  if (kSplit && pre) {
+    k_tile_params<true><<<(unsigned)((tiles + 127) / 128), 128, 0, stream>>>(bv);
+    k_tile_table<true><<<(unsigned)((tiles * rows + 127) / 128), 128, 0, stream>>>(bv, rows);
   }
   if (ev) cudaEventRecord(ev[2], stream);
-  if (pre) launch_variant_index<kSplit>(v, bv, num_sms, dyn, stream, std::make_index_sequence<kNumVariants>{});
+  if (kSplit && pre) launch_split_index(v, bv, num_sms, dyn, stream, std::make_index_sequence<kNumVariants>{});
   else launch_persistent(k_waveform<kSplit>, bv, num_sms, dyn, stream);
   if (ev) cudaEventRecord(ev[3], stream);
 }
@@ -2354,11 +2498,12 @@ void launch_dense(const BatchView &bv, int num_sms, cudaStream_t stream, cudaEve
 // i.e. the samples from max(i_plunge + i_buffer + 2, i0 + 1) on.  Rows 1-3 of
 // phase_out are sums of those three phases, so they take their own values at
 // i_plunge.  y strides over sources, x over each source's frozen samples.
+// (Small sources; the segments' phase pass writes them itself.)
 __global__ void __launch_bounds__(256) k_phase_freeze(const SourceDesc *__restrict__ src, int nsrc,
                                                       double *__restrict__ out, int64_t st) {
   for (int s = blockIdx.y; s < nsrc; s += gridDim.y) {
     const SourceDesc &d = src[s];
-    if (d.status != 0 || d.i_plunge < 0 || d.i_plunge >= d.vlength) continue;
+    if (d.n_tiles > kSmallTiles || d.status != 0 || d.i_plunge < 0 || d.i_plunge >= d.vlength) continue;
     const long long first = max((long long)d.i_plunge + (long long)d.i_buffer + 2, (long long)d.i0 + 1);
     if (first >= d.vlength) continue;
     const int64_t o = d.out_offset;
@@ -2374,24 +2519,30 @@ __global__ void __launch_bounds__(256) k_phase_freeze(const SourceDesc *__restri
 }
 
 void launch_phase(const BatchView &bv, int num_sms, cudaStream_t stream, cudaEvent_t *ev) {
-  if (bv.total_tiles <= 0 || !bv.phase_out) return;
+  if (bv.total_tiles <= 0 || !bv.phase_out || !bv.tile_prep || !bv.tile_seg || !bv.frozen) return;
   if (ev) cudaEventRecord(ev[0], stream);
-  cudaMemsetAsync(bv.work_counter, 0, sizeof(unsigned long long), stream);
-  cudaMemsetAsync(bv.link_flag, 0, (size_t)bv.total_tiles * sizeof(int32_t), stream);
-  if (ev) {
-    cudaEventRecord(ev[1], stream);
-    cudaEventRecord(ev[2], stream);
-  }
   prepare_dense_launch();
-  if (bv.tile_prep) {
-    // the tile parameters from the pre-pass, each tile's inputs staged by bulk copies
+  if (bv.small_tiles > 0) {
+    // the tile parameters from the pre-pass, each tile's inputs staged by bulk copies, carries by look-back
+    BatchView sm = bv;
+    sm.total_tiles = bv.small_tiles;
+    cudaMemsetAsync(bv.work_counter, 0, sizeof(unsigned long long), stream);
+    cudaMemsetAsync(bv.link_flag, 0, (size_t)bv.total_tiles * sizeof(int32_t), stream);
     k_tile_params<false><<<(unsigned)((bv.total_tiles + 127) / 128), 128, 0, stream>>>(bv);
-    launch_persistent(k_waveform<false, 1, true, 0, 3>, bv, num_sms, kWaveDynSmem, stream);
-  } else {
-    launch_persistent(k_waveform<false, 1>, bv, num_sms, kWaveDynSmem, stream);
+    launch_persistent(k_waveform<false, 1, true, 0, 3>, sm, num_sms, kWaveDynSmem, stream);
+    const dim3 fgrid(64, (unsigned)std::min(std::max(bv.nsrc, 1), 1024));
+    k_phase_freeze<<<fgrid, 256, 0, stream>>>(bv.src, bv.nsrc, bv.phase_out, bv.phase_stride);
   }
-  const dim3 fgrid(64, (unsigned)std::min(std::max(bv.nsrc, 1), 1024));
-  k_phase_freeze<<<fgrid, 256, 0, stream>>>(bv.src, bv.nsrc, bv.phase_out, bv.phase_stride);
+  if (ev) cudaEventRecord(ev[1], stream);
+  if (ev) cudaEventRecord(ev[2], stream);
+  if (bv.small_tiles < bv.total_tiles) {
+    BatchView lg = bv;
+    lg.queue += bv.small_tiles;
+    lg.total_tiles -= bv.small_tiles;
+    launch_segments<true>(lg, num_sms, 0, stream, nullptr);
+    if (ev) cudaEventRecord(ev[2], stream);
+    launch_persistent(k_waveform<false, 1, true, 0, 3, true>, lg, num_sms, kWaveDynSmem, stream);
+  }
   if (ev) cudaEventRecord(ev[3], stream);
 }
 

@@ -52,6 +52,36 @@ struct alignas(16) TilePrep {
 };
 static_assert(sizeof(TilePrep) == 64, "TilePrep is one 64-byte bulk copy");
 
+// FP64 batches: a tile's polynomial segments (aak_segments.cuh), one slot a
+// tile: this head, then per 256-sample segment the coefficients of the three
+// phases and of the rates, amplitude, e and response.
+struct alignas(16) TileHead {
+  // double-double: the three phases at the tile's head modulo 2 pi; the phase product: the signed increments from
+  // t = 0 to there
+  double hi[3], lo[3];
+  double C;             // clamped Phidot before the tile, where its raw value is not positive
+  double sgn;           // 1: the head and the tiles after it; -1: the tiles before it
+  double ec;            // centre of the Bessel table
+  int32_t mode;         // degree of the polynomials (4 or 7); 0: direct, sample by sample; -1: no output
+  int32_t K, stride;    // Bessel table: Taylor terms (0: none), doubles per row
+  int32_t nmodes;
+  int32_t pad[2];
+};
+static_assert(sizeof(TileHead) == 96, "the coefficients after the head stay 16-byte aligned");
+constexpr int64_t kSegSlotBytes = 96 + 4 * 108 * 8;  // head, 4 segments of at most 108 doubles
+// Phase increments of one tile: forward and backward sums, and the clamped
+// Phidot after its last forward sample (kept in the look-back records' memory).
+struct SegAgg {
+  double f[3], b[3];
+  double lastP;
+  int32_t hasP, needC;  // lastP was set in the tile; the sums wait for the clamped Phidot before the tile
+};
+static_assert(sizeof(SegAgg) <= sizeof(TileLink), "an aggregate fits in the tile's look-back record");
+// words of seg_ctl, cleared before every launch: queue heads, direct tiles,
+// then per source its direct tiles, and per source those of them summed
+constexpr int kCtlQueue = 0, kCtlDirectQueue = 1, kCtlDirectCount = 2, kCtlSource = 4;
+inline size_t seg_ctl_words(int nsrc) { return kCtlSource + 2 * (size_t)nsrc; }
+
 // Taylor-table rows: FP64 terms at most (K <= 10) and FP32 terms at most
 // (K <= 6); a tile's FP64 rows hold 3 (K + 1) coefficients of one harmonic,
 // its FP32 rows 6 (K + 1) of a pair of harmonics, padded to 16 bytes.
@@ -71,11 +101,14 @@ inline int64_t tile_table_slot_bytes(int rows, bool split) {
 }
 
 // Launch shapes of the waveform stage, the autotuner's candidates: with the
-// tile pre-pass or tables built inside the tiles, samples per thread whose
+// tile pre-pass or everything inside the tiles, samples per thread whose
 // harmonic sums run side by side, and resident CTAs per SM the register
-// budget is sized for.  Variant 0 is the default of each precision: the
-// autotuner's choice on both the 512-source configuration-1 batch and a
-// 256-template configuration-4 chunk, in both precisions.
+// budget is sized for.  Variant 0 is the default of each precision: split, the
+// autotuner's choice on the 512-source configuration-1 batch and a 256-template
+// configuration-4 chunk; FP64 (polynomial segments), its choice on batches of
+// 30 harmonics (32 sources 4.42 ms against 4.61, 4.66, 4.93, 5.09 of the other
+// segment shapes and 8.68 inside the tiles) and of 11 to 61, within 4 % of the
+// best at 10.
 struct WaveVariant {
   bool pre;
   int joint;
@@ -86,8 +119,16 @@ constexpr WaveVariant wave_variant(bool split, int v) {
   return split ? (v == 1 ? WaveVariant{false, 0, 2} : v == 2 ? WaveVariant{true, 1, 2} : v == 3 ? WaveVariant{true, 4, 2}
                   : v == 4 ? WaveVariant{true, 2, 3} : v == 5 ? WaveVariant{true, 2, 2} : WaveVariant{true, 1, 3})
                : (v == 1 ? WaveVariant{false, 0, 2} : v == 2 ? WaveVariant{true, 2, 2} : v == 3 ? WaveVariant{true, 4, 2}
-                  : v == 4 ? WaveVariant{true, 1, 2} : v == 5 ? WaveVariant{true, 2, 3} : WaveVariant{true, 1, 3});
+                  : v == 4 ? WaveVariant{true, 1, 2} : v == 5 ? WaveVariant{true, 1, 3} : WaveVariant{true, 2, 3});
 }
+
+// FP64 sources of at most this many tiles keep the single kernel that does
+// everything inside the tiles (one launch, the chain carried by look-back):
+// the segments' four launches one after another cost more than the few
+// tiles.  Four sources of 4 to 20 tiles: 41 us against 77; one of 100: 80
+// and 85.  The line is drawn by the source, not by the batch, so that a
+// source's samples do not depend on the batch it comes in.
+constexpr int kSmallTiles = 24;
 
 // One work-queue item: a tile, its place in its source, and what staging it
 // needs, so that a CTA can issue the tile's bulk copies and find its source
@@ -112,6 +153,7 @@ struct BatchView {
   int64_t total_tiles;
   const int64_t *tile_start;    // nsrc + 1 prefix of tiles (device)
   const QueueItem *queue = nullptr;  // work-queue order; null: source by source, each in chain order
+  int64_t small_tiles = 0;      // with a queue: its first items, the tiles of the sources of at most kSmallTiles tiles
   const int32_t *tile_knot;     // 2 per tile: first knot of the tile's window, knots in it
   const double *knot_t;         // knots
   const double4 *knot_y;        // (e, v, M, S) at the knots
@@ -138,6 +180,13 @@ struct BatchView {
   TilePrep *tile_prep = nullptr;
   void *tile_tab = nullptr;
   int64_t tab_slot = 0;
+  // FP64 polynomial segments (with tile_prep; aak_segments.cuh): one slot a
+  // tile, the tiles' aggregates, the queue items of the direct tiles, counters
+  unsigned char *tile_seg = nullptr;
+  SegAgg *tile_agg = nullptr;
+  int32_t *direct_list = nullptr;
+  int32_t *seg_ctl = nullptr;
+  double *frozen = nullptr;  // phase product: 3 per source, the phases at i_plunge
   int32_t variant = 0;  // launch shape of the waveform stage (wave_variant), chosen by the autotuner
 };
 
