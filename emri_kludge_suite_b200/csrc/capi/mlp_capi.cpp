@@ -56,13 +56,17 @@ int train_like(aak_mlp *m, const float *x, const float *y, const int32_t *perm, 
   mlp::launch_reduce_adam(m->md, ntiles, lr, m->beta1, m->beta2, m->eps, bc1, bc2, grad, st);
   if ((r = cuda_status(cudaGetLastError())) != AAK_OK) return r;
   if (loss) {
-    std::vector<float> lp(ntiles);
-    if ((r = cuda_status(cudaMemcpyAsync(lp.data(), m->md.loss_part, ntiles * sizeof(float), cudaMemcpyDeviceToHost,
-                                         st))) != AAK_OK)
+    // the tiles' losses and, right after their array, the error flag: one copy
+    float lp[mlp::kMaxTrainTiles + 1];
+    static_assert(sizeof(lp) == mlp::kMaxTrainTiles * sizeof(float) + sizeof(int), "losses, then the flag");
+    if ((r = cuda_status(cudaMemcpyAsync(lp, m->md.loss_part, sizeof(lp), cudaMemcpyDeviceToHost, st))) != AAK_OK ||
+        (r = cuda_status(cudaStreamSynchronize(st))) != AAK_OK)
       return r;
-    if ((r = check_error_flag(m, st)) != AAK_OK) return r;
+    int err;
+    std::memcpy(&err, &lp[mlp::kMaxTrainTiles], sizeof(err));
+    if (err) return AAK_ERR_DEVICE_TIMEOUT;
     double s = 0.0;
-    for (float v : lp) s += v;
+    for (int i = 0; i < ntiles; ++i) s += lp[i];
     *loss = (float)(s / (3.0 * (double)n));
   }
   return AAK_OK;
@@ -118,9 +122,9 @@ int aak_mlp_create(int32_t device, aak_mlp **out) {
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && sms > 0) m->num_sms = sms;
   const size_t P = mlp::kParams;
   const size_t o_w = 0, o_m = o_w + al256(P * 4), o_v = o_m + al256(P * 4), o_wq = o_v + al256(P * 4),
-               o_img = o_wq + al256(P * 4), o_part = o_img + al256(4 * (size_t)mlp::kImgElems * 2),
+               o_img = o_wq + al256(P * 4), o_part = o_img + al256(2 * (size_t)mlp::kImgElems * 2),
                o_loss = o_part + al256((size_t)mlp::kMaxTrainTiles * mlp::kPartStride * 4),
-               o_err = o_loss + al256(mlp::kMaxTrainTiles * 4), o_grad = o_err + 256, total = o_grad + al256(P * 4);
+               o_err = o_loss + mlp::kMaxTrainTiles * 4, o_grad = al256(o_err + 4), total = o_grad + al256(P * 4);
   unsigned char *b = nullptr;
   if ((r = cuda_status(cudaMalloc(&b, total))) != AAK_OK) {
     delete m;

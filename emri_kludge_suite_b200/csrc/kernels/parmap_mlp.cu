@@ -1,12 +1,15 @@
 // parmap_mlp.cu -- see parmap_mlp.cuh.
 //
-// One CTA of 128 threads owns a tile of 128 batch rows, one thread per row.
 // The 128 x 128 layers are tcgen05.mma (kind::f16, BF16 x BF16 -> FP32,
-// M = N = 128, K = 16 per instruction) issued by one thread on operands staged
-// in shared memory in the K-major, no-swizzle canonical layout, with the FP32
-// accumulators in tensor memory; each thread reads its row back with
-// tcgen05.ld (32x32b: warp w owns TMEM lanes 32w .. 32w + 31 = rows).
+// M = N = 128, K = 16 per instruction) on tiles of 128 batch rows, issued by
+// one thread on operands staged in shared memory in the no-swizzle canonical
+// layout, with the FP32 accumulators in tensor memory; a thread reads its row
+// back with tcgen05.ld (32x32b: warp w owns TMEM lanes 32 (w mod 4) ..  = rows).
 // Activations are rounded to BF16 where they enter a tensor-core product.
+// Inference: a CTA of 512 threads holds both weight images and runs four
+// tiles at a time, one on each group of four warps, so that the products of
+// one overlap the activations of the others.  Training: the 512 threads share
+// one tile, each a row and a quarter of its columns.
 #include "parmap_mlp.cuh"
 
 #include <cuda_bf16.h>
@@ -15,6 +18,9 @@ namespace aak {
 namespace mlp {
 
 namespace {
+
+constexpr int kGroups = 4;                       // groups of four warps a CTA
+constexpr int kThreads = kGroups * kTileRows;    // 512
 
 // ------------------------------------------------------------------ BF16
 __device__ __forceinline__ uint32_t bf16_bits(float x) { return (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(x)); }
@@ -29,29 +35,41 @@ __host__ __device__ __forceinline__ int canon(int r, int k) {
   return (((r >> 3) * 16 + (k >> 3)) << 6) + ((r & 7) << 3) + (k & 7);
 }
 constexpr uint32_t kLBO = 128, kSBO = 2048;
+// The same image read with its columns as the M or N index (MN-major: eight
+// contiguous M or N elements of eight K rows a core): cores adjacent along M or
+// N are 128 B apart (SBO), those along K 2048 B (LBO), and a step of K = 16 is
+// two of the latter.  So one image of activations [row][k] serves the forward
+// product (K = k) and the weight gradient (K = row), and one weight image
+// [out][in] the forward (K = in) and the backward product (K = out).
 // Instruction descriptor (kind::f16): D F32 (bits 4-5 = 1), A BF16 (7-9 = 1),
-// B BF16 (10-12 = 1), both K-major (15, 16 = 0), N >> 3 at 17-22, M >> 4 at 24-28.
+// B BF16 (10-12 = 1), A and B K-major (bits 15, 16 = 0; 1: MN-major), N >> 3 at
+// 17-22, M >> 4 at 24-28.
 constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
 
 __device__ __forceinline__ uint32_t saddr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 // Shared-memory matrix descriptor: start >> 4 (bits 0-13), LBO >> 4 (16-29),
 // SBO >> 4 (32-45), descriptor version 1 (46-47), no swizzle (61-63 = 0).
+template <bool kMN>
 __device__ __forceinline__ uint64_t smem_desc(uint32_t a) {
-  return (uint64_t)((a & 0x3FFFFu) >> 4) | ((uint64_t)(kLBO >> 4) << 16) | ((uint64_t)(kSBO >> 4) << 32) |
-         (1ull << 46);
+  constexpr uint32_t lbo = kMN ? kSBO : kLBO, sbo = kMN ? kLBO : kSBO;
+  return (uint64_t)((a & 0x3FFFFu) >> 4) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(sbo >> 4) << 32) | (1ull << 46);
 }
 
-// D[128 x 128] (+)= A[128 x K] B[128 x K]^T with K = 128 (8 instructions).
-__device__ __forceinline__ void mma_128(uint32_t tmem_d, uint32_t a, uint32_t b, bool accumulate) {
+// D[128 x 128] = A[128 x 128] B[128 x 128]^T over K = 128 (8 instructions);
+// kA, kB: the operand's image is read MN-major.
+template <bool kA, bool kB>
+__device__ __forceinline__ void mma_128(uint32_t tmem_d, uint32_t a, uint32_t b) {
+  constexpr uint32_t idesc = kIdesc | (kA ? 1u << 15 : 0u) | (kB ? 1u << 16 : 0u);
 #pragma unroll
   for (int s = 0; s < 8; ++s) {
-    const uint64_t da = smem_desc(a + s * 256), db = smem_desc(b + s * 256);
-    const uint32_t acc = (s > 0 || accumulate) ? 1u : 0u;
+    const uint64_t da = smem_desc<kA>(a + s * (kA ? 2 * kSBO : 2 * kLBO));
+    const uint64_t db = smem_desc<kB>(b + s * (kB ? 2 * kSBO : 2 * kLBO));
+    const uint32_t acc = (s > 0) ? 1u : 0u;
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d),
-        "l"(da), "l"(db), "r"(kIdesc), "r"(acc)
+        "l"(da), "l"(db), "r"(idesc), "r"(acc)
         : "memory");
   }
 }
@@ -105,11 +123,36 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float v[16]) {
 }
 
 // ------------------------------------------------------------------ activation
-__device__ __forceinline__ float sigm(float z) { return 1.0f / (1.0f + expf(-z)); }
-__device__ __forceinline__ float silu(float z) { return z * sigm(z); }
-__device__ __forceinline__ float dsilu(float z) {
-  const float s = sigm(z);
-  return s * (1.0f + z * (1.0f - s));
+// Sigmoids of a pair.  Training (kFast false): the library's exp and an IEEE
+// division, so that the activations and their BF16 roundings do not move.
+// Inference: one exponential each (ex2.approx of the FP32 product, 2 ulp) and
+// one reciprocal for the two, 1 / a = b / (a b); the argument is bounded at
+// 2^60, so that the product of the two stays finite: below z = -41 the sigmoid
+// is 1e-18, not less.
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+template <bool kFast>
+__device__ __forceinline__ float2 sigm2(float2 z) {
+  if constexpr (!kFast) return make_float2(1.0f / (1.0f + expf(-z.x)), 1.0f / (1.0f + expf(-z.y)));
+  const float2 t = __fmul2_rn(z, make_float2(-1.44269504f, -1.44269504f));
+  const float a = 1.0f + ex2(fminf(t.x, 60.0f)), b = 1.0f + ex2(fminf(t.y, 60.0f));
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a * b));
+  return __fmul2_rn(make_float2(r, r), make_float2(b, a));
+}
+template <bool kFast>
+__device__ __forceinline__ float2 silu2(float2 z) { return __fmul2_rn(z, sigm2<kFast>(z)); }
+// silu' = s (1 + z (1 - s))
+__device__ __forceinline__ float2 dsilu2(float2 z, float2 s) {
+  const float2 one = make_float2(1.0f, 1.0f);
+  return __fmul2_rn(s, __ffma2_rn(z, __ffma2_rn(s, make_float2(-1.0f, -1.0f), one), one));
+}
+__device__ __forceinline__ uint32_t pack_bf16(float2 v) {
+  const __nv_bfloat162 b = __floats2bfloat162_rn(v.x, v.y);
+  return *reinterpret_cast<const uint32_t *>(&b);
 }
 
 __device__ __forceinline__ void features(const Norm &nm, const float *xr, float f[4]) {
@@ -118,36 +161,59 @@ __device__ __forceinline__ void features(const Norm &nm, const float *xr, float 
   for (int k = 0; k < 4; ++k) f[k] = (g[k] - nm.in_shift[k]) * nm.in_scale[k];
 }
 
-__device__ __forceinline__ float layer1(const float *W1, const float *b1, const float f[4], int o) {
-  return b1[o] + W1[4 * o] * f[0] + W1[4 * o + 1] * f[1] + W1[4 * o + 2] * f[2] + W1[4 * o + 3] * f[3];
+// Layer 1 of outputs 2p, 2p + 1, from their weights and biases as pairs: w[0] =
+// (W[k = 0] of the two, W[1]), w[1] = (W[2], W[3]), w[2] = (bias, -).
+__device__ __forceinline__ float2 layer1_pair(const float4 *w, const float f[4]) {
+  const float4 u = w[0], v = w[1], c = w[2];
+  float2 z = make_float2(c.x, c.y);
+  z = __ffma2_rn(make_float2(u.x, u.y), make_float2(f[0], f[0]), z);
+  z = __ffma2_rn(make_float2(u.z, u.w), make_float2(f[1], f[1]), z);
+  z = __ffma2_rn(make_float2(v.x, v.y), make_float2(f[2], f[2]), z);
+  return __ffma2_rn(make_float2(v.z, v.w), make_float2(f[3], f[3]), z);
+}
+// The small layers in the form the threads read them (all threads of the CTA).
+struct SmallLayers {
+  float4 w1[kHid / 2][3];  // layer1_pair
+  float4 w4[kHid];         // W4[0..2][o], b3[o]
+  float b2[kHid];
+  float b4[4];
+};
+__device__ __forceinline__ void load_small(SmallLayers &L, const DeviceModel &md) {
+  float *w1 = reinterpret_cast<float *>(L.w1), *w4 = reinterpret_cast<float *>(L.w4);
+  for (int i = threadIdx.x; i < kHid / 2 * 12; i += blockDim.x) {
+    const int p = i / 12, c = i % 12, o = 2 * p + (c & 1), k = c >> 1;
+    w1[i] = (k < 4) ? md.wq[kOffW1 + kIn * o + k] : (k == 4) ? md.w[kOffB1 + o] : 0.f;
+  }
+  for (int i = threadIdx.x; i < kHid * 4; i += blockDim.x)
+    w4[i] = ((i & 3) < 3) ? md.wq[kOffW4 + (i & 3) * kHid + (i >> 2)] : md.w[kOffB3 + (i >> 2)];
+  for (int i = threadIdx.x; i < kHid; i += blockDim.x) L.b2[i] = md.w[kOffB2 + i];
+  if (threadIdx.x < 4) L.b4[threadIdx.x] = (threadIdx.x < kOut) ? md.w[kOffB4 + threadIdx.x] : 0.f;
 }
 
-// store 8 BF16 (packed in q[4]) at row r, columns k0 .. k0 + 7 of a K-major image
+// store 8 BF16 (packed in q[4]) at row r, columns k0 .. k0 + 7 of an image
 __device__ __forceinline__ void put_row8(uint16_t *img, int r, int k0, const uint32_t q[4]) {
   *reinterpret_cast<uint4 *>(img + canon(r, k0)) = make_uint4(q[0], q[1], q[2], q[3]);
 }
-// store 8 BF16 at rows k0 .. k0 + 7, column c (transposed write)
-__device__ __forceinline__ void put_col8(uint16_t *img, int k0, int c, const uint32_t q[4]) {
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    img[canon(k0 + 2 * j, c)] = (uint16_t)(q[j] & 0xFFFFu);
-    img[canon(k0 + 2 * j + 1, c)] = (uint16_t)(q[j] >> 16);
-  }
-}
 
-__device__ __forceinline__ void copy_img(uint16_t *dst, const uint16_t *src) {
+__device__ __forceinline__ void copy_img(uint16_t *dst, const uint16_t *src, int images) {
   const uint4 *s = reinterpret_cast<const uint4 *>(src);
   uint4 *d = reinterpret_cast<uint4 *>(dst);
-  for (int i = threadIdx.x; i < kImgElems / 8; i += blockDim.x) d[i] = s[i];
+#pragma unroll 8
+  for (int i = threadIdx.x; i < images * kImgElems / 8; i += kThreads) d[i] = s[i];
 }
 
-// One thread waits for the MMA phase; everyone learns the outcome.
-__device__ __forceinline__ bool wait_mma(uint32_t mbar, uint32_t parity, volatile int *flag, int *err) {
-  if (threadIdx.x == 0 && !mbar_wait(mbar, parity)) {
+// Barrier of one group of 128 threads (named barrier 1 + group).
+__device__ __forceinline__ void group_sync(int group) { asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory"); }
+
+// One thread (of the group, or of the CTA: group -1) waits for the MMA phase; all of them learn the outcome.
+__device__ __forceinline__ bool wait_mma(uint32_t mbar, uint32_t parity, volatile int *flag, int *err, int group) {
+  const bool first = (group < 0) ? threadIdx.x == 0 : (threadIdx.x & 127) == 0;
+  if (first && !mbar_wait(mbar, parity)) {
     *flag = 1;
     atomicExch(err, 1);
   }
-  __syncthreads();
+  if (group < 0) __syncthreads();
+  else group_sync(group);
   return *flag == 0;
 }
 
@@ -161,12 +227,10 @@ __device__ __forceinline__ void publish_one(const DeviceModel &md, int p, float 
     const int q = p - kOffW2, o = q >> 7, i = q & 127;
     const uint16_t b = (uint16_t)bf16_bits(w);
     md.img[canon(o, i)] = b;
-    md.img[2 * kImgElems + canon(i, o)] = b;
   } else if (p >= kOffW3 && p < kOffB3) {
     const int q = p - kOffW3, o = q >> 7, i = q & 127;
     const uint16_t b = (uint16_t)bf16_bits(w);
     md.img[kImgElems + canon(o, i)] = b;
-    md.img[3 * kImgElems + canon(i, o)] = b;
   }
 }
 
@@ -180,6 +244,7 @@ __global__ void k_reduce_adam(DeviceModel md, int ntiles, float lr, float beta1,
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= kParams) return;
   float g = 0.0f;
+#pragma unroll 32  // the loads of a batch's tiles in flight together, added in order
   for (int t = 0; t < ntiles; ++t) g += md.partial[(int64_t)t * kPartStride + p];
   if (grad) grad[p] = g;
   if (lr > 0.0f) {
@@ -195,161 +260,169 @@ __global__ void k_reduce_adam(DeviceModel md, int ntiles, float lr, float beta1,
 
 // ------------------------------------------------------------------ inference
 struct FwdSmem {
-  uint16_t A[kImgElems];   // activations of the tile, K-major
-  uint16_t W2[kImgElems];  // W2 image (B operand: N = out, K = in)
-  uint16_t W3[kImgElems];
-  float W1[kHid * kIn];
-  float W4[kOut * kHid];
-  float b1[kHid], b2[kHid], b3[kHid], b4[4];
-  unsigned long long mbar;
+  uint16_t A[kGroups][kImgElems];  // activations of each group's tile, K-major
+  uint16_t W[2][kImgElems];        // W2, W3 images (B operands: N = out, K = in)
+  SmallLayers L;
+  unsigned long long mbar[kGroups];
   uint32_t tmem_slot;
-  int flag;
+  int flag[kGroups];
 };
 
-__global__ void __launch_bounds__(kTileRows) k_forward(DeviceModel md, const float *__restrict__ x,
-                                                       float *__restrict__ y, int64_t n) {
+// The activations cost two special-function operations a value with the
+// library's exp and division beside them; with sigm2 they cost one and a half,
+// and sixteen warps an SM on four tiles keep that pipe busy while a tile waits
+// for its product.  Bound by that pipe (69 % of its rate): 1e6 points 1027 us on
+// 128-thread CTAs, two an SM, 199 us here.
+__global__ void __launch_bounds__(kThreads, 1) k_forward(DeviceModel md, const float *__restrict__ x,
+                                                         float *__restrict__ y, int64_t n) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   FwdSmem &S = *reinterpret_cast<FwdSmem *>(smem_raw);
-  const int t = threadIdx.x, warp = t >> 5;
-  copy_img(S.W2, md.img);
-  copy_img(S.W3, md.img + kImgElems);
-  for (int i = t; i < kHid * kIn; i += kTileRows) S.W1[i] = md.wq[kOffW1 + i];
-  for (int i = t; i < kOut * kHid; i += kTileRows) S.W4[i] = md.wq[kOffW4 + i];
-  S.b1[t] = md.w[kOffB1 + t];
-  S.b2[t] = md.w[kOffB2 + t];
-  S.b3[t] = md.w[kOffB3 + t];
-  if (t < kOut) S.b4[t] = md.w[kOffB4 + t];
-  const uint32_t mbar = saddr(&S.mbar);
+  const int group = threadIdx.x >> 7, t = threadIdx.x & 127, warp = (threadIdx.x >> 5) & 3;
+  copy_img(S.W[0], md.img, 2);
+  load_small(S.L, md);
+  const uint32_t mbar = saddr(&S.mbar[group]);
   if (t == 0) {
     mbar_init(mbar);
-    S.flag = 0;
+    S.flag[group] = 0;
   }
-  if (warp == 0) tmem_alloc(saddr(&S.tmem_slot), 128);
+  if (threadIdx.x < 32) tmem_alloc(saddr(&S.tmem_slot), kGroups * 128);
   fence_async_smem();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = S.tmem_slot;
+  const uint32_t tmem = S.tmem_slot + 128 * group;
   const uint32_t lane = tmem + ((uint32_t)(warp * 32) << 16);
+  uint16_t *A = S.A[group];
   const Norm nm = md.norm;
   uint32_t phase = 0;
   bool ok = true;
   const int64_t ntiles = (n + kTileRows - 1) / kTileRows;
-  for (int64_t g = blockIdx.x; g < ntiles && ok; g += gridDim.x) {
+  // a tile to every CTA before a second one to any
+  for (int64_t g = blockIdx.x + (int64_t)gridDim.x * group; g < ntiles && ok; g += (int64_t)gridDim.x * kGroups) {
     const int64_t row = g * kTileRows + t;
     const bool valid = row < n;
     float f[4] = {0.f, 0.f, 0.f, 0.f};
     if (valid) features(nm, x + 4 * row, f);
     // layer 1 (FP32 pipe) -> A
+#pragma unroll 2
     for (int c = 0; c < 16; ++c) {
       uint32_t q[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int o = 8 * c + 2 * j;
-        const float a0 = valid ? silu(layer1(S.W1, S.b1, f, o)) : 0.f;
-        const float a1 = valid ? silu(layer1(S.W1, S.b1, f, o + 1)) : 0.f;
-        q[j] = bf16_bits(a0) | (bf16_bits(a1) << 16);
-      }
-      put_row8(S.A, t, 8 * c, q);
+      for (int j = 0; j < 4; ++j) q[j] = pack_bf16(silu2<true>(layer1_pair(S.L.w1[4 * c + j], f)));
+      put_row8(A, t, 8 * c, q);
     }
     fence_async_smem();
     tc_fence_before();
-    __syncthreads();
+    group_sync(group);
     if (t == 0) {
       tc_fence_after();
-      mma_128(tmem, saddr(S.A), saddr(S.W2), false);
+      mma_128<false, false>(tmem, saddr(A), saddr(S.W[0]));
       mma_commit(mbar);
     }
-    if (!(ok = wait_mma(mbar, phase, &S.flag, md.error))) break;
+    if (!(ok = wait_mma(mbar, phase, &S.flag[group], md.error, group))) break;
     phase ^= 1;
     tc_fence_after();
     // layer 2 epilogue -> A
+#pragma unroll 1
     for (int c = 0; c < 8; ++c) {
       float v[16];
       tmem_ld16(lane + 16 * c, v);
+      const float4 *b4 = reinterpret_cast<const float4 *>(S.L.b2 + 16 * c);
       uint32_t q[8];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int o = 16 * c + 2 * j;
-        const float a0 = valid ? silu(v[2 * j] + S.b2[o]) : 0.f;
-        const float a1 = valid ? silu(v[2 * j + 1] + S.b2[o + 1]) : 0.f;
-        q[j] = bf16_bits(a0) | (bf16_bits(a1) << 16);
+      for (int j = 0; j < 4; ++j) {
+        const float4 b = b4[j];
+        q[2 * j] = pack_bf16(silu2<true>(__fadd2_rn(make_float2(v[4 * j], v[4 * j + 1]), make_float2(b.x, b.y))));
+        q[2 * j + 1] = pack_bf16(silu2<true>(__fadd2_rn(make_float2(v[4 * j + 2], v[4 * j + 3]), make_float2(b.z, b.w))));
       }
-      put_row8(S.A, t, 16 * c, q);
-      put_row8(S.A, t, 16 * c + 8, q + 4);
+      put_row8(A, t, 16 * c, q);
+      put_row8(A, t, 16 * c + 8, q + 4);
     }
     fence_async_smem();
     tc_fence_before();
-    __syncthreads();
+    group_sync(group);
     if (t == 0) {
       tc_fence_after();
-      mma_128(tmem, saddr(S.A), saddr(S.W3), false);
+      mma_128<false, false>(tmem, saddr(A), saddr(S.W[1]));
       mma_commit(mbar);
     }
-    if (!(ok = wait_mma(mbar, phase, &S.flag, md.error))) break;
+    if (!(ok = wait_mma(mbar, phase, &S.flag[group], md.error, group))) break;
     phase ^= 1;
     tc_fence_after();
     // layer 3 epilogue + output layer (FP32 pipe)
-    float acc[3] = {S.b4[0], S.b4[1], S.b4[2]};
+    float2 acc01 = make_float2(S.L.b4[0], S.L.b4[1]);
+    float acc2 = S.L.b4[2];
+#pragma unroll 1
     for (int c = 0; c < 8; ++c) {
       float v[16];
       tmem_ld16(lane + 16 * c, v);
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const int o = 16 * c + j;
-        const float a = bf16_round(silu(v[j] + S.b3[o]));
-        acc[0] += S.W4[o] * a;
-        acc[1] += S.W4[kHid + o] * a;
-        acc[2] += S.W4[2 * kHid + o] * a;
+      for (int j = 0; j < 8; ++j) {
+        const float4 u = S.L.w4[16 * c + 2 * j], w = S.L.w4[16 * c + 2 * j + 1];
+        const float2 a = silu2<true>(__fadd2_rn(make_float2(v[2 * j], v[2 * j + 1]), make_float2(u.w, w.w)));
+        const uint32_t q = pack_bf16(a);
+        const float a0 = __uint_as_float(q << 16), a1 = __uint_as_float(q & 0xFFFF0000u);
+        acc01 = __ffma2_rn(make_float2(u.x, u.y), make_float2(a0, a0), acc01);
+        acc2 = fmaf(u.z, a0, acc2);
+        acc01 = __ffma2_rn(make_float2(w.x, w.y), make_float2(a1, a1), acc01);
+        acc2 = fmaf(w.z, a1, acc2);
       }
     }
-    if (valid)
-      for (int j = 0; j < 3; ++j) y[3 * row + j] = acc[j] * nm.out_scale[j] + nm.out_shift[j];
+    if (valid) {
+      y[3 * row] = acc01.x * nm.out_scale[0] + nm.out_shift[0];
+      y[3 * row + 1] = acc01.y * nm.out_scale[1] + nm.out_shift[1];
+      y[3 * row + 2] = acc2 * nm.out_scale[2] + nm.out_shift[2];
+    }
+    tc_fence_before();  // this tile's reads of the accumulators, before the next tile's product overwrites them
   }
   if (!ok && t == 0) mbar_wait(mbar, phase);  // let an MMA still in flight drain (bounded)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (warp == 0) tmem_free(tmem, 128);
+  if (threadIdx.x < 32) tmem_free(S.tmem_slot, kGroups * 128);
 }
 
 // ------------------------------------------------------------------ training
+constexpr int kScrStride = kTileRows + 1;  // FP32 dz1 scratch, [out][row], padded against bank conflicts
 struct TrainSmem {
-  uint16_t W[kImgElems];    // weight operand slot
-  uint16_t X0[kImgElems];   // a1, then a2 ([row][in], K-major); then a3 (plain row-major)
-  uint16_t D0[kImgElems];   // dz3, then dz2 ([row][out], K-major); X0|D0: 64 KB FP32 scratch for dz1
-  uint16_t XT1[kImgElems];  // a1^T ([in][row], K-major)
-  uint16_t XT2[kImgElems];  // a2^T
-  uint16_t DT[kImgElems];   // dz^T ([out][row], K-major)
+  uint16_t D[kImgElems];     // dz3, then dz2 [row][out]
+  uint16_t W[2][kImgElems];  // W2, W3
+  uint16_t X1[kImgElems];    // a1 [row][in]; with X2 and A3 at the end the FP32 scratch for dz1
+  uint16_t X2[kImgElems];    // a2
+  uint16_t A3[kImgElems];    // a3
+  SmallLayers L;
   float f[kTileRows][4];
-  float dy[kTileRows][3];
-  float W1[kHid * kIn];
-  float W4[kOut * kHid];
-  float b1[kHid], b2[kHid], b3[kHid], b4[4];
+  float dy[kTileRows][4];
+  float part[kGroups][kTileRows][4];  // output layer, partial over a column quarter; then partial sums of the gradients
   float red[4];
   unsigned long long mbar;
   uint32_t tmem_slot;
   int flag;
 };
+static_assert(3 * kImgElems * 2 >= kHid * kScrStride * 4, "dz1 fits in three images");
 
-__device__ __forceinline__ float sum_row_T(const uint16_t *img, int r) {  // sum over k of image row r
+// Sum over a quarter of the tile's rows (32 quarter .. ) of column o of an image.
+__device__ __forceinline__ float sum_col_quarter(const uint16_t *img, int o, int quarter) {
   float s = 0.f;
-  for (int c = 0; c < 16; ++c) {
-    const uint4 u = *reinterpret_cast<const uint4 *>(img + canon(r, 8 * c));
-    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-    for (int j = 0; j < 4; ++j) s += bf16_val((uint16_t)(w[j] & 0xFFFFu)) + bf16_val((uint16_t)(w[j] >> 16));
-  }
+#pragma unroll 8
+  for (int b = 32 * quarter; b < 32 * quarter + 32; ++b) s += bf16_val(img[canon(b, o)]);
   return s;
 }
 
-__global__ void __launch_bounds__(kTileRows, 1) k_gradients(DeviceModel md, const float *__restrict__ x,
-                                                            const float *__restrict__ yt,
-                                                            const int32_t *__restrict__ perm, int64_t n,
-                                                            float inv_count) {
+// One CTA a tile, thread (row t, column quarter): 64 tiles of a minibatch of
+// 8192 leave most of the chip idle, so what counts is the serial length of a
+// tile.  A quarter of the columns a thread, the operand images read both ways
+// by the products (no transposed copies), conflict-free scratch.  Bound by the
+// latency of its eight barriers and five products: the 64 tiles 126 us on
+// 128-thread CTAs, 34 us here.
+__global__ void __launch_bounds__(kThreads, 1) k_gradients(DeviceModel md, const float *__restrict__ x,
+                                                           const float *__restrict__ yt,
+                                                           const int32_t *__restrict__ perm, int64_t n,
+                                                           float inv_count) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   TrainSmem &S = *reinterpret_cast<TrainSmem *>(smem_raw);
-  const int t = threadIdx.x, warp = t >> 5;
+  const int cg = threadIdx.x >> 7, t = threadIdx.x & 127, warp = (threadIdx.x >> 5) & 3;
+  const int o0 = 32 * cg;  // this thread's columns
   const int64_t g = blockIdx.x;
   const int64_t row = g * kTileRows + t;
   const bool valid = row < n;
@@ -357,35 +430,29 @@ __global__ void __launch_bounds__(kTileRows, 1) k_gradients(DeviceModel md, cons
   float *part = md.partial + g * kPartStride;
   const Norm nm = md.norm;
 
-  copy_img(S.W, md.img);  // W2
-  for (int i = t; i < kHid * kIn; i += kTileRows) S.W1[i] = md.wq[kOffW1 + i];
-  for (int i = t; i < kOut * kHid; i += kTileRows) S.W4[i] = md.wq[kOffW4 + i];
-  S.b1[t] = md.w[kOffB1 + t];
-  S.b2[t] = md.w[kOffB2 + t];
-  S.b3[t] = md.w[kOffB3 + t];
-  if (t < kOut) S.b4[t] = md.w[kOffB4 + t];
+  copy_img(S.W[0], md.img, 2);
+  load_small(S.L, md);
   const uint32_t mbar = saddr(&S.mbar);
-  if (t == 0) {
+  if (threadIdx.x == 0) {
     mbar_init(mbar);
     S.flag = 0;
   }
-  if (warp == 0) tmem_alloc(saddr(&S.tmem_slot), 512);
+  if (threadIdx.x < 32) tmem_alloc(saddr(&S.tmem_slot), 512);
   float f[4] = {0.f, 0.f, 0.f, 0.f};
   if (valid) features(nm, x + 4 * idx, f);
-  for (int k = 0; k < 4; ++k) S.f[t][k] = f[k];
-  __syncthreads();  // W1, b1 staged
-  // layer 1 -> X0 (row t) and XT1 (column t)
-  for (int c = 0; c < 16; ++c) {
+  if (cg == 0)
+    for (int k = 0; k < 4; ++k) S.f[t][k] = f[k];
+  __syncthreads();  // the small layers staged
+  const float on = valid ? 1.f : 0.f;  // rows past the batch contribute nothing
+  const float2 on2 = make_float2(on, on);
+  // layer 1 -> X1
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
     uint32_t q[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int o = 8 * c + 2 * j;
-      const float a0 = valid ? silu(layer1(S.W1, S.b1, f, o)) : 0.f;
-      const float a1 = valid ? silu(layer1(S.W1, S.b1, f, o + 1)) : 0.f;
-      q[j] = bf16_bits(a0) | (bf16_bits(a1) << 16);
-    }
-    put_row8(S.X0, t, 8 * c, q);
-    put_col8(S.XT1, 8 * c, t, q);
+    for (int j = 0; j < 4; ++j)
+      q[j] = valid ? pack_bf16(silu2<false>(layer1_pair(S.L.w1[o0 / 2 + 4 * c + j], f))) : 0u;
+    put_row8(S.X1, t, o0 + 8 * c, q);
   }
   fence_async_smem();
   tc_fence_before();
@@ -393,199 +460,223 @@ __global__ void __launch_bounds__(kTileRows, 1) k_gradients(DeviceModel md, cons
   tc_fence_after();
   const uint32_t tmem = S.tmem_slot;
   const uint32_t T0 = tmem, T1 = tmem + 128, T2 = tmem + 256, T3 = tmem + 384;
-  const uint32_t lane = (uint32_t)(warp * 32) << 16;
+  const uint32_t lane = ((uint32_t)(warp * 32) << 16) + (uint32_t)o0;
   uint32_t phase = 0;
   bool ok = true;
   do {
     // ---- forward: z2 = a1 W2^T -> T0
-    if (t == 0) {
-      mma_128(T0, saddr(S.X0), saddr(S.W), false);
+    if (threadIdx.x == 0) {
+      mma_128<false, false>(T0, saddr(S.X1), saddr(S.W[0]));
       mma_commit(mbar);
     }
-    if (!(ok = wait_mma(mbar, phase, &S.flag, md.error))) break;
+    if (!(ok = wait_mma(mbar, phase, &S.flag, md.error, -1))) break;
     phase ^= 1;
     tc_fence_after();
-    copy_img(S.W, md.img + kImgElems);  // W3
-    for (int c = 0; c < 8; ++c) {
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
       float v[16];
       tmem_ld16(T0 + lane + 16 * c, v);
       uint32_t q[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        const int o = 16 * c + 2 * j;
-        const float a0 = valid ? silu(v[2 * j] + S.b2[o]) : 0.f;
-        const float a1 = valid ? silu(v[2 * j + 1] + S.b2[o + 1]) : 0.f;
-        q[j] = bf16_bits(a0) | (bf16_bits(a1) << 16);
+        const int o = o0 + 16 * c + 2 * j;
+        const float2 z = __fadd2_rn(make_float2(v[2 * j], v[2 * j + 1]), make_float2(S.L.b2[o], S.L.b2[o + 1]));
+        q[j] = valid ? pack_bf16(silu2<false>(z)) : 0u;
       }
-      put_row8(S.X0, t, 16 * c, q);
-      put_row8(S.X0, t, 16 * c + 8, q + 4);
-      put_col8(S.XT2, 16 * c, t, q);
-      put_col8(S.XT2, 16 * c + 8, t, q + 4);
+      put_row8(S.X2, t, o0 + 16 * c, q);
+      put_row8(S.X2, t, o0 + 16 * c + 8, q + 4);
     }
     fence_async_smem();
     tc_fence_before();
     __syncthreads();
     // ---- forward: z3 = a2 W3^T -> T1
-    if (t == 0) {
+    if (threadIdx.x == 0) {
       tc_fence_after();
-      mma_128(T1, saddr(S.X0), saddr(S.W), false);
+      mma_128<false, false>(T1, saddr(S.X2), saddr(S.W[1]));
       mma_commit(mbar);
     }
-    if (!(ok = wait_mma(mbar, phase, &S.flag, md.error))) break;
+    if (!(ok = wait_mma(mbar, phase, &S.flag, md.error, -1))) break;
     phase ^= 1;
     tc_fence_after();
-    // ---- output layer, loss, dy; a3 kept (plain row-major) in X0
-    float acc[3] = {S.b4[0], S.b4[1], S.b4[2]};
-    for (int c = 0; c < 8; ++c) {
-      float v[16];
-      tmem_ld16(T1 + lane + 16 * c, v);
+    // ---- output layer over this thread's columns; a3 kept, silu' in registers
+    float2 ds[16];
+    {
+      float2 acc01 = make_float2(0.f, 0.f);
+      float acc2 = 0.f;
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const int o = 16 * c + j;
-        const float a = bf16_round(silu(v[j] + S.b3[o]));
-        S.X0[t * kHid + o] = (uint16_t)bf16_bits(a);
-        acc[0] += S.W4[o] * a;
-        acc[1] += S.W4[kHid + o] * a;
-        acc[2] += S.W4[2 * kHid + o] * a;
+      for (int c = 0; c < 2; ++c) {
+        float v[16];
+        tmem_ld16(T1 + lane + 16 * c, v);
+        uint32_t q[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float4 u = S.L.w4[o0 + 16 * c + 2 * j], w = S.L.w4[o0 + 16 * c + 2 * j + 1];
+          const float2 z = __fadd2_rn(make_float2(v[2 * j], v[2 * j + 1]), make_float2(u.w, w.w));
+          const float2 sg = sigm2<false>(z);
+          ds[8 * c + j] = dsilu2(z, sg);
+          q[j] = pack_bf16(__fmul2_rn(z, sg));
+          const float a0 = __uint_as_float(q[j] << 16), a1 = __uint_as_float(q[j] & 0xFFFF0000u);
+          acc01 = __ffma2_rn(make_float2(u.x, u.y), make_float2(a0, a0), acc01);
+          acc2 = fmaf(u.z, a0, acc2);
+          acc01 = __ffma2_rn(make_float2(w.x, w.y), make_float2(a1, a1), acc01);
+          acc2 = fmaf(w.z, a1, acc2);
+        }
+        put_row8(S.A3, t, o0 + 16 * c, q);
+        put_row8(S.A3, t, o0 + 16 * c + 8, q + 4);
       }
+      S.part[cg][t][0] = acc01.x;
+      S.part[cg][t][1] = acc01.y;
+      S.part[cg][t][2] = acc2;
     }
+    __syncthreads();
+    // ---- loss, dy
     float dy[3], l = 0.f;
+#pragma unroll
     for (int j = 0; j < 3; ++j) {
-      const float d = valid ? acc[j] - (yt[3 * idx + j] - nm.out_shift[j]) / nm.out_scale[j] : 0.f;
+      const float a = S.L.b4[j] + ((S.part[0][t][j] + S.part[1][t][j]) + (S.part[2][t][j] + S.part[3][t][j]));
+      const float d = valid ? a - (yt[3 * idx + j] - nm.out_shift[j]) / nm.out_scale[j] : 0.f;
       l += d * d;
       dy[j] = 2.0f * d * inv_count;
-      S.dy[t][j] = dy[j];
+      if (cg == 0) S.dy[t][j] = dy[j];
     }
-    for (int off = 16; off > 0; off >>= 1) l += __shfl_xor_sync(0xffffffffu, l, off);
-    if ((t & 31) == 0) S.red[warp] = l;
-    // dz3 = bf16(dy W4 * silu'(z3)) -> D0 (row t), DT (column t)
-    for (int c = 0; c < 8; ++c) {
-      float v[16];
-      tmem_ld16(T1 + lane + 16 * c, v);
-      uint32_t q[8];
+    if (cg == 0) {
+      for (int off = 16; off > 0; off >>= 1) l += __shfl_xor_sync(0xffffffffu, l, off);
+      if ((t & 31) == 0) S.red[warp] = l;
+    }
+    // dz3 = bf16(dy W4 * silu'(z3)) -> D
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        float dz[2];
+    for (int c = 0; c < 4; ++c) {
+      uint32_t q[4];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int o = 16 * c + 2 * j + h;
-          const float da = dy[0] * S.W4[o] + dy[1] * S.W4[kHid + o] + dy[2] * S.W4[2 * kHid + o];
-          dz[h] = valid ? da * dsilu(v[2 * j + h] + S.b3[o]) : 0.f;
-        }
-        q[j] = bf16_bits(dz[0]) | (bf16_bits(dz[1]) << 16);
+      for (int j = 0; j < 4; ++j) {
+        const float4 u = S.L.w4[o0 + 8 * c + 2 * j], w = S.L.w4[o0 + 8 * c + 2 * j + 1];
+        const float2 da = make_float2(dy[0] * u.x + dy[1] * u.y + dy[2] * u.z, dy[0] * w.x + dy[1] * w.y + dy[2] * w.z);
+        q[j] = valid ? pack_bf16(__fmul2_rn(da, ds[4 * c + j])) : 0u;
       }
-      put_row8(S.D0, t, 16 * c, q);
-      put_row8(S.D0, t, 16 * c + 8, q + 4);
-      put_col8(S.DT, 16 * c, t, q);
-      put_col8(S.DT, 16 * c + 8, t, q + 4);
+      put_row8(S.D, t, o0 + 8 * c, q);
     }
-    copy_img(S.W, md.img + 3 * kImgElems);  // W3^T
     fence_async_smem();
     tc_fence_before();
     __syncthreads();
     // ---- dW3 = dz3^T a2 -> T2 ; da2 = dz3 W3 -> T3
-    if (t == 0) {
+    if (threadIdx.x == 0) {
       tc_fence_after();
-      mma_128(T2, saddr(S.DT), saddr(S.XT2), false);
-      mma_128(T3, saddr(S.D0), saddr(S.W), false);
+      mma_128<true, true>(T2, saddr(S.D), saddr(S.X2));
+      mma_128<false, true>(T3, saddr(S.D), saddr(S.W[1]));
       mma_commit(mbar);
       md.loss_part[g] = (S.red[0] + S.red[1]) + (S.red[2] + S.red[3]);
     }
-    // meanwhile: output-layer gradients and db3 from shared memory
+    // meanwhile: output-layer gradients and db3 (column t, a quarter of the rows a thread)
     {
       float s0 = 0.f, s1 = 0.f, s2 = 0.f;
-      for (int b = 0; b < kTileRows; ++b) {
-        const float a = bf16_val(S.X0[b * kHid + t]);
+#pragma unroll 8
+      for (int b = 32 * cg; b < 32 * cg + 32; ++b) {
+        const float a = bf16_val(S.A3[canon(b, t)]);
         s0 += S.dy[b][0] * a;
         s1 += S.dy[b][1] * a;
         s2 += S.dy[b][2] * a;
       }
-      part[kOffW4 + t] = s0;
-      part[kOffW4 + kHid + t] = s1;
-      part[kOffW4 + 2 * kHid + t] = s2;
-      if (t < kOut) {
-        float s = 0.f;
-        for (int b = 0; b < kTileRows; ++b) s += S.dy[b][t];
-        part[kOffB4 + t] = s;
-      }
-      part[kOffB3 + t] = sum_row_T(S.DT, t);
+      float *p = S.part[cg][t];
+      p[0] = s0;
+      p[1] = s1;
+      p[2] = s2;
+      p[3] = sum_col_quarter(S.D, t, cg);
     }
-    if (!(ok = wait_mma(mbar, phase, &S.flag, md.error))) break;
+    if (!(ok = wait_mma(mbar, phase, &S.flag, md.error, -1))) break;
     phase ^= 1;
     tc_fence_after();
-    for (int c = 0; c < 8; ++c) {  // dW3 row t
+    {  // thread (t, cg) writes sum cg of column t: dW4 rows 0-2, db3
+      const float s = (S.part[0][t][cg] + S.part[1][t][cg]) + (S.part[2][t][cg] + S.part[3][t][cg]);
+      part[cg < 3 ? kOffW4 + cg * kHid + t : kOffB3 + t] = s;
+    }
+    if (threadIdx.x < kOut) {
+      float s = 0.f;
+      for (int b = 0; b < kTileRows; ++b) s += S.dy[b][threadIdx.x];
+      part[kOffB4 + threadIdx.x] = s;
+    }
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {  // dW3 row t
       float v[16];
       tmem_ld16(T2 + lane + 16 * c, v);
-      float4 *dst = reinterpret_cast<float4 *>(part + kOffW3 + t * kHid + 16 * c);
+      float4 *dst = reinterpret_cast<float4 *>(part + kOffW3 + t * kHid + o0 + 16 * c);
       for (int j = 0; j < 4; ++j) dst[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
     }
-    // dz2 = bf16(da2 * silu'(z2)) -> D0, DT
-    for (int c = 0; c < 8; ++c) {
+    // dz2 = bf16(da2 * silu'(z2)) -> D
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
       float da[16], z[16];
       tmem_ld16(T3 + lane + 16 * c, da);
       tmem_ld16(T0 + lane + 16 * c, z);
       uint32_t q[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        const int o = 16 * c + 2 * j;
-        const float d0 = valid ? da[2 * j] * dsilu(z[2 * j] + S.b2[o]) : 0.f;
-        const float d1 = valid ? da[2 * j + 1] * dsilu(z[2 * j + 1] + S.b2[o + 1]) : 0.f;
-        q[j] = bf16_bits(d0) | (bf16_bits(d1) << 16);
+        const int o = o0 + 16 * c + 2 * j;
+        const float2 zz = __fadd2_rn(make_float2(z[2 * j], z[2 * j + 1]), make_float2(S.L.b2[o], S.L.b2[o + 1]));
+        q[j] = valid ? pack_bf16(__fmul2_rn(make_float2(da[2 * j], da[2 * j + 1]), dsilu2(zz, sigm2<false>(zz)))) : 0u;
       }
-      put_row8(S.D0, t, 16 * c, q);
-      put_row8(S.D0, t, 16 * c + 8, q + 4);
-      put_col8(S.DT, 16 * c, t, q);
-      put_col8(S.DT, 16 * c + 8, t, q + 4);
+      put_row8(S.D, t, o0 + 16 * c, q);
+      put_row8(S.D, t, o0 + 16 * c + 8, q + 4);
     }
-    copy_img(S.W, md.img + 2 * kImgElems);  // W2^T
     fence_async_smem();
     tc_fence_before();
     __syncthreads();
     // ---- dW2 = dz2^T a1 -> T2 ; da1 = dz2 W2 -> T3
-    if (t == 0) {
+    if (threadIdx.x == 0) {
       tc_fence_after();
-      mma_128(T2, saddr(S.DT), saddr(S.XT1), false);
-      mma_128(T3, saddr(S.D0), saddr(S.W), false);
+      mma_128<true, true>(T2, saddr(S.D), saddr(S.X1));
+      mma_128<false, true>(T3, saddr(S.D), saddr(S.W[0]));
       mma_commit(mbar);
     }
-    part[kOffB2 + t] = sum_row_T(S.DT, t);
-    if (!(ok = wait_mma(mbar, phase, &S.flag, md.error))) break;
+    S.part[cg][t][0] = sum_col_quarter(S.D, t, cg);
+    if (!(ok = wait_mma(mbar, phase, &S.flag, md.error, -1))) break;
     phase ^= 1;
     tc_fence_after();
-    for (int c = 0; c < 8; ++c) {  // dW2 row t
+    if (cg == 0) part[kOffB2 + t] = (S.part[0][t][0] + S.part[1][t][0]) + (S.part[2][t][0] + S.part[3][t][0]);
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {  // dW2 row t
       float v[16];
       tmem_ld16(T2 + lane + 16 * c, v);
-      float4 *dst = reinterpret_cast<float4 *>(part + kOffW2 + t * kHid + 16 * c);
+      float4 *dst = reinterpret_cast<float4 *>(part + kOffW2 + t * kHid + o0 + 16 * c);
       for (int j = 0; j < 4; ++j) dst[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
     }
-    // dz1 = da1 * silu'(z1) in FP32 -> scratch [row][out]
-    float *scr = reinterpret_cast<float *>(S.X0);
-    for (int c = 0; c < 8; ++c) {
+    // dz1 = da1 * silu'(z1) in FP32 -> scratch [out][row] (X1, X2, A3: their last readers are done)
+    float *scr = reinterpret_cast<float *>(S.X1);
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
       float v[16];
       tmem_ld16(T3 + lane + 16 * c, v);
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const int o = 16 * c + j;
-        scr[t * kHid + o] = valid ? v[j] * dsilu(layer1(S.W1, S.b1, f, o)) : 0.f;
+      for (int j = 0; j < 8; ++j) {
+        const int o = o0 + 16 * c + 2 * j;
+        const float2 z = layer1_pair(S.L.w1[o / 2], f);
+        const float2 d = __fmul2_rn(__fmul2_rn(make_float2(v[2 * j], v[2 * j + 1]), dsilu2(z, sigm2<false>(z))), on2);
+        scr[o * kScrStride + t] = d.x;
+        scr[(o + 1) * kScrStride + t] = d.y;
       }
     }
     __syncthreads();
-    {
-      float s[4] = {0.f, 0.f, 0.f, 0.f}, sb = 0.f;
-      for (int b = 0; b < kTileRows; ++b) {
-        const float d = scr[b * kHid + t];
-        sb += d;
-        for (int k = 0; k < 4; ++k) s[k] += d * S.f[b][k];
-      }
-      for (int k = 0; k < 4; ++k) part[kOffW1 + 4 * t + k] = s[k];
-      part[kOffB1 + t] = sb;
+    // column t over a quarter of the rows, then the four quarters (thread (t, cg): input cg; cg = 0 the bias too)
+    float s[4] = {0.f, 0.f, 0.f, 0.f}, sb = 0.f;
+#pragma unroll 8
+    for (int b = 32 * cg; b < 32 * cg + 32; ++b) {
+      const float d = scr[t * kScrStride + b];
+      sb += d;
+      for (int k = 0; k < 4; ++k) s[k] += d * S.f[b][k];
     }
+    float *p = S.part[cg][t];
+    for (int k = 0; k < 4; ++k) p[k] = s[k];
+    __syncthreads();  // the scratch is read: its first words take the bias sums
+    scr[cg * kTileRows + t] = sb;
+    part[kOffW1 + 4 * t + cg] = (S.part[0][t][cg] + S.part[1][t][cg]) + (S.part[2][t][cg] + S.part[3][t][cg]);
+    __syncthreads();
+    if (cg == 0)
+      part[kOffB1 + t] = (scr[t] + scr[kTileRows + t]) + (scr[2 * kTileRows + t] + scr[3 * kTileRows + t]);
   } while (false);
-  if (!ok && t == 0) mbar_wait(mbar, phase);  // let an MMA still in flight drain (bounded)
+  if (!ok && threadIdx.x == 0) mbar_wait(mbar, phase);  // let an MMA still in flight drain (bounded)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (warp == 0) tmem_free(tmem, 512);
+  if (threadIdx.x < 32) tmem_free(tmem, 512);
 }
 
 }  // namespace
@@ -599,8 +690,8 @@ void launch_forward(const DeviceModel &md, const float *x, float *y, int64_t n, 
   const int smem = (int)sizeof(FwdSmem);
   cudaFuncSetAttribute(k_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   const int64_t ntiles = (n + kTileRows - 1) / kTileRows;
-  const int grid = (int)std::min<int64_t>(ntiles, 2 * (int64_t)num_sms);
-  k_forward<<<grid, kTileRows, smem, st>>>(md, x, y, n);
+  const int grid = (int)std::min<int64_t>(ntiles, (int64_t)num_sms);
+  k_forward<<<grid, kThreads, smem, st>>>(md, x, y, n);
 }
 
 void launch_gradients(const DeviceModel &md, const float *x, const float *y_true, const int32_t *perm, int64_t n,
@@ -609,7 +700,7 @@ void launch_gradients(const DeviceModel &md, const float *x, const float *y_true
   const int smem = (int)sizeof(TrainSmem);
   cudaFuncSetAttribute(k_gradients, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   const int ntiles = (int)((n + kTileRows - 1) / kTileRows);
-  k_gradients<<<ntiles, kTileRows, smem, st>>>(md, x, y_true, perm, n, 1.0f / (3.0f * (float)n));
+  k_gradients<<<ntiles, kThreads, smem, st>>>(md, x, y_true, perm, n, 1.0f / (3.0f * (float)n));
 }
 
 void launch_reduce_adam(const DeviceModel &md, int ntiles, float lr, float beta1, float beta2, float eps, float bc1,

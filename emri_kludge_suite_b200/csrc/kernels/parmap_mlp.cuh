@@ -43,7 +43,7 @@ struct DeviceModel {
   float *w;          // kParams FP32 master weights
   float *m, *v;      // Adam moments
   float *wq;         // kParams: weights rounded to BF16 (biases unrounded), as FP32
-  uint16_t *img;     // 4 x kImgElems BF16 operand images (tcgen05 K-major layout): W2, W3, W2^T, W3^T
+  uint16_t *img;     // 2 x kImgElems BF16 operand images (tcgen05 canonical layout): W2, W3
   float *partial;    // kMaxTrainTiles x kPartStride per-tile gradients
   float *loss_part;  // kMaxTrainTiles per-tile loss sums
   int *error;        // nonzero after a bounded wait gave up
