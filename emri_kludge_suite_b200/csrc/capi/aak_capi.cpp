@@ -103,7 +103,8 @@ struct aak_ctx {
   DevBuf<TilePrep> d_tile_prep;           // tile pre-pass: per-tile parameters
   DevBuf<unsigned char> d_tile_tab;       //   and per-tile Taylor tables
   DevBuf<unsigned char> d_tile_seg;       // FP64: polynomial segments, one slot per tile
-  DevBuf<int32_t> d_seg_ctl;              //   their counters,
+  DevBuf<SegAgg> d_seg_agg;               //   the tiles' phase increments,
+  DevBuf<int32_t> d_direct, d_seg_ctl;    //   the direct tiles, counters,
   DevBuf<double> d_frozen;                //   and the phases at i_plunge, 3 per source
   DevBuf<double> d_out;  // outputs for the host-buffer entry points
   // batched device solve of the Kerr -> AK map (opt-in: parmap_device)
@@ -114,6 +115,7 @@ struct aak_ctx {
   DevBuf<double> d_pm_warm, d_pm_map;
   DevBuf<int32_t> d_pm_it;
   cudaStream_t pm_stream = nullptr;
+  DenseSide side;                 // second stream of the FP64 launches
   DevBuf<TdiDesc> d_tdi;        // frequency-domain TDI: per-source stationary-phase records
   DevBuf<int64_t> d_tdi_work;   //   and the prefix of their work items
   int last_launches = 0;
@@ -815,22 +817,24 @@ BatchView batch_view(aak_ctx *ctx, double *hI, double *hII, double *t, double *t
 // TilePrep and one Taylor-table slot per tile), grown as needed, set in bv.
 void drop_graph(aak_ctx *ctx);
 
-// The buffers of the FP64 polynomial segments, grown as needed, set in bv: the
-// aggregates and the list of direct tiles take the look-back records' and
-// flags' memory, which the segments' launches do not use.
+// The buffers of the FP64 polynomial segments, grown as needed, set in bv.
 int tile_segments(aak_ctx *ctx, BatchView &bv) {
   const int64_t tiles = std::max<int64_t>(ctx->total_tiles, 1);
-  const void *s0 = ctx->d_tile_seg.ptr, *c0 = ctx->d_seg_ctl.ptr;
+  const void *s0 = ctx->d_tile_seg.ptr, *c0 = ctx->d_seg_ctl.ptr, *a0 = ctx->d_seg_agg.ptr, *l0 = ctx->d_direct.ptr,
+             *f0 = ctx->d_frozen.ptr;
   int r;
-  if ((r = ctx->d_tile_seg.reserve(tiles * kSegSlotBytes)) != AAK_OK ||
+  if ((r = ctx->d_tile_seg.reserve(tiles * kSegSlotBytes)) != AAK_OK || (r = ctx->d_seg_agg.reserve(tiles)) != AAK_OK ||
+      (r = ctx->d_direct.reserve(tiles)) != AAK_OK ||
       (r = ctx->d_seg_ctl.reserve(seg_ctl_words(ctx->nsrc))) != AAK_OK || (r = ctx->d_frozen.reserve(3 * (size_t)ctx->nsrc)) != AAK_OK)
     return r;
-  if (ctx->d_tile_seg.ptr != s0 || ctx->d_seg_ctl.ptr != c0) drop_graph(ctx);
+  if (ctx->d_tile_seg.ptr != s0 || ctx->d_seg_ctl.ptr != c0 || ctx->d_seg_agg.ptr != a0 || ctx->d_direct.ptr != l0 ||
+      ctx->d_frozen.ptr != f0)
+    drop_graph(ctx);
   bv.tile_seg = ctx->d_tile_seg.ptr;
   bv.seg_ctl = ctx->d_seg_ctl.ptr;
   bv.frozen = ctx->d_frozen.ptr;
-  bv.tile_agg = reinterpret_cast<SegAgg *>(ctx->d_link.ptr);
-  bv.direct_list = ctx->d_flag.ptr;
+  bv.tile_agg = ctx->d_seg_agg.ptr;
+  bv.direct_list = ctx->d_direct.ptr;
   return AAK_OK;
 }
 
@@ -872,7 +876,7 @@ int run(aak_ctx *ctx, double *hI, double *hII, double *t, double *traj, int64_t 
   if (!traj && (r = tile_tables(ctx, precision, bv)) != AAK_OK) return r;
   if (ctx->profile && !ctx->ev[0])
     for (auto &e : ctx->ev) cudaEventCreate(&e);
-  launch_dense(bv, ctx->num_sms, st, ctx->profile ? ctx->ev : nullptr, precision);
+  launch_dense(bv, ctx->num_sms, st, ctx->profile ? ctx->ev : nullptr, precision, &ctx->side);
   ctx->last_launches = bv.tile_prep ? dense_launches(ctx, precision) : 1;
   return cuda_ok(cudaGetLastError());
 }
@@ -921,7 +925,7 @@ int run_graph(aak_ctx *ctx, double *hI, double *hII, int precision, cudaStream_t
     // and the waveform kernel
     launch_spline_coeffs(ctx->d_src.ptr, ctx->nsrc, ctx->d_spl_blk.ptr, ctx->spl_blk[ctx->nsrc], ctx->spl_len, ctx->d_knot_t.ptr,
                          ctx->d_knot_y.ptr, ctx->d_knot_c.ptr, ctx->cap_stream);
-    launch_dense(bv, ctx->num_sms, ctx->cap_stream, nullptr, precision);
+    launch_dense(bv, ctx->num_sms, ctx->cap_stream, nullptr, precision, &ctx->side);
     const cudaError_t launch_err = cudaGetLastError();
     cudaGraph_t g = nullptr;
     const cudaError_t end_err = cudaStreamEndCapture(ctx->cap_stream, &g);
@@ -990,7 +994,7 @@ int run_phase(aak_ctx *ctx, double *out, int64_t stride, cudaStream_t st) {
   if ((r = tile_segments(ctx, bv)) != AAK_OK) return r;
   if (ctx->profile && !ctx->ev[0])
     for (auto &e : ctx->ev) cudaEventCreate(&e);
-  launch_phase(bv, ctx->num_sms, st, ctx->profile ? ctx->ev : nullptr);
+  launch_phase(bv, ctx->num_sms, st, ctx->profile ? ctx->ev : nullptr, &ctx->side);
   // small sources: tile parameters, phase pass, freeze; the others: segments, carries, phase pass
   ctx->last_launches = (ctx->small_tiles > 0 ? 3 : 0) + (ctx->small_tiles < ctx->total_tiles ? 3 : 0);
   return cuda_ok(cudaGetLastError());
@@ -1505,6 +1509,15 @@ int aak_ctx_create(int32_t device, aak_ctx **out) {
   int sms = 0;
   if (device >= 0 && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && sms > 0)
     c->num_sms = sms;
+  if (device >= 0) {
+    int r = cuda_ok(cudaStreamCreateWithFlags(&c->side.stream, cudaStreamNonBlocking));
+    for (cudaEvent_t *e : {&c->side.fork[0], &c->side.fork[1], &c->side.join})
+      if (r == AAK_OK) r = cuda_ok(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+    if (r != AAK_OK) {
+      aak_ctx_destroy(c);
+      return r;
+    }
+  }
   *out = c;
   return AAK_OK;
 }
@@ -1520,6 +1533,11 @@ void aak_ctx_destroy(aak_ctx *c) {
     c->d_spl_blk.release();
     c->d_tile_seg.release();
     c->d_seg_ctl.release();
+    c->d_seg_agg.release();
+    c->d_direct.release();
+    if (c->side.stream) cudaStreamDestroy(c->side.stream);
+    for (cudaEvent_t e : {c->side.fork[0], c->side.fork[1], c->side.join})
+      if (e) cudaEventDestroy(e);
     c->d_frozen.release();
     c->d_knot_t.release();
     c->d_knot_y.release();

@@ -1275,6 +1275,7 @@ __global__ void __launch_bounds__(128) k_tile_params(BatchView bv) {
   if (g >= bv.total_tiles) return;
   const int s = find_source(bv.tile_start, bv.nsrc, g);
   const SourceDesc &d = bv.src[s];
+  if (!kSplit && d.n_tiles > kSmallTiles) return;  // (the phase product's small sources)
   TilePrep P;
   P.ec = 0.0;
   P.K = -1;
@@ -1472,14 +1473,20 @@ __global__ void __launch_bounds__(kTileThreads, kMinB) k_waveform(BatchView bv) 
     else if constexpr (kCarry) return atomicAdd(bv.seg_ctl + kCtlQueue, 1);
     else return (long long)atomicAdd(bv.work_counter, 1ull);
   };
-  const long long items = (kCarry && !kPhase) ? (long long)bv.seg_ctl[kCtlDirectCount] : (long long)bv.total_tiles;
+  // direct tiles: an entry for each chunk of samples (the phase pass is done again for each; a few tiles a batch)
+  const long long items =
+      (kCarry && !kPhase) ? (long long)bv.seg_ctl[kCtlDirectCount] * kTileChunks : (long long)bv.total_tiles;
+  int part = 0;
   if (tid == 0) s_tile = fetch();
   __syncthreads();
   for (;;) {
     long long j = s_tile;
     __syncthreads();
     if (j >= items) break;
-    if constexpr (kCarry && !kPhase) j = bv.direct_list[j];
+    if constexpr (kCarry && !kPhase) {
+      part = (int)(j % kTileChunks);
+      j = bv.direct_list[j / kTileChunks];
+    }
     if constexpr (kCarry && kPhase) {
       // a tile of polynomial segments: its record, head and coefficients by
       // bulk copies, its rows straight from them
@@ -1986,8 +1993,10 @@ __global__ void __launch_bounds__(kTileThreads, kMinB) k_waveform(BatchView bv) 
     static_assert(kTileChunks % kJoint == 0, "joint samples must divide the chunks");
     const T *tab = kSplit ? reinterpret_cast<const T *>(tabF) : reinterpret_cast<const T *>(tabD);
     const int rs = kPre ? (int)s_prep.stride : (kSplit ? 2 * kRowF : kRowD);  // table row (FP32: pair row) stride
+    constexpr bool kParts = kCarry && !kPhase;
+    static_assert(!kParts || kJoint == 1, "a direct entry is one chunk");
 #pragma unroll 1
-    for (int g0 = 0; g0 < kTileChunks; g0 += kJoint) {
+    for (int g0 = kParts ? part : 0; g0 < (kParts ? part + 1 : kTileChunks); g0 += kJoint) {
       SamplePrep<T> P[kJoint];
       T dl[kJoint], c1[kJoint], s1[kJoint], cD[kJoint], sD[kJoint], Sa[kJoint], Sb[kJoint], Sc[kJoint], d0[kJoint];
       double ph[kJoint];
@@ -2416,8 +2425,11 @@ void launch_seg_variant(const BatchView &bv, int num_sms, int rows, cudaStream_t
   int resident = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_wave_segments<J, w.min_blocks>, kTileThreads, 2 * stage);
   resident = std::max(resident, 1);
-  const int grid = (int)std::min<int64_t>(bv.total_tiles, (int64_t)num_sms * resident);
-  k_wave_segments<J, w.min_blocks><<<grid, kTileThreads, 2 * stage, stream>>>(bv, stage);
+  // half tiles where whole ones would leave a last wave nearly empty: below four waves of them
+  const int64_t slots = (int64_t)num_sms * resident;
+  const int parts = (J <= 2 && bv.total_tiles < 4 * slots) ? 2 : 1;
+  const int grid = (int)std::min<int64_t>(bv.total_tiles * parts, slots);
+  k_wave_segments<J, w.min_blocks><<<grid, kTileThreads, 2 * stage, stream>>>(bv, stage, parts);
 }
 template <size_t... I>
 void launch_seg_index(int v, const BatchView &bv, int num_sms, int rows, cudaStream_t stream, std::index_sequence<I...>) {
@@ -2437,8 +2449,21 @@ void launch_segments(const BatchView &bv, int num_sms, int rows, cudaStream_t st
   k_tile_carries<<<(unsigned)(carry + table), kSegWarps * 32, 0, stream>>>(bv, carry, std::max(rows, 1));
 }
 
+// Let work queued on the side stream from here on follow what is on `stream`.
+cudaStream_t fork_side(const DenseSide *side, int k, cudaStream_t stream) {
+  if (!side) return stream;
+  cudaEventRecord(side->fork[k], stream);
+  cudaStreamWaitEvent(side->stream, side->fork[k], 0);
+  return side->stream;
+}
+void join_side(const DenseSide *side, cudaStream_t stream) {
+  if (!side) return;
+  cudaEventRecord(side->join, side->stream);
+  cudaStreamWaitEvent(stream, side->join, 0);
+}
+
 template <bool kSplit>
-void launch_dense_t(const BatchView &bv, int num_sms, cudaStream_t stream, cudaEvent_t *ev) {
+void launch_dense_t(const BatchView &bv, int num_sms, cudaStream_t stream, cudaEvent_t *ev, const DenseSide *side) {
   if (ev) cudaEventRecord(ev[0], stream);
   // per-sample values, then the Taylor table sized for the batch's harmonic count
   const int rows = table_rows<typename std::conditional<kSplit, float, double>::type>(
@@ -2451,15 +2476,20 @@ void launch_dense_t(const BatchView &bv, int num_sms, cudaStream_t stream, cudaE
   prepare_dense_launch();
   if (!kSplit && pre) {
     // the small sources' tiles first in the queue, by the kernel that does everything inside the tiles; the rest as
-    // segments (whose list of direct tiles takes the flags' memory afterwards)
+    // segments.  The small sources beside the segments' pre-pass, the direct tiles beside the segments: each is a
+    // few tiles of latency on a nearly empty chip.
+    bool sided = false;
     if (bv.small_tiles > 0) {
+      const bool only = bv.small_tiles == tiles;
+      const cudaStream_t st = only ? stream : fork_side(side, 0, stream);
+      sided = !only;
       BatchView sm = bv;
       sm.total_tiles = bv.small_tiles;
-      cudaMemsetAsync(bv.work_counter, 0, sizeof(unsigned long long), stream);
-      cudaMemsetAsync(bv.link_flag, 0, (size_t)tiles * sizeof(int32_t), stream);
-      if (ev && bv.small_tiles == tiles) cudaEventRecord(ev[1], stream);
-      if (ev && bv.small_tiles == tiles) cudaEventRecord(ev[2], stream);
-      launch_persistent(k_waveform<false>, sm, num_sms, dyn, stream);
+      cudaMemsetAsync(bv.work_counter, 0, sizeof(unsigned long long), st);
+      cudaMemsetAsync(bv.link_flag, 0, (size_t)tiles * sizeof(int32_t), st);
+      if (ev && only) cudaEventRecord(ev[1], st);
+      if (ev && only) cudaEventRecord(ev[2], st);
+      launch_persistent(k_waveform<false>, sm, num_sms, dyn, st);
     }
     if (bv.small_tiles < tiles) {
       BatchView lg = bv;
@@ -2467,9 +2497,11 @@ void launch_dense_t(const BatchView &bv, int num_sms, cudaStream_t stream, cudaE
       lg.total_tiles -= bv.small_tiles;
       launch_segments<false>(lg, num_sms, rows, stream, ev);
       if (ev) cudaEventRecord(ev[2], stream);
-      launch_persistent(k_waveform<false, 0, true, 1, 3, true>, lg, num_sms, dyn, stream);
+      launch_persistent(k_waveform<false, 0, true, 1, 3, true>, lg, num_sms, dyn, fork_side(side, 1, stream));
       launch_seg_index(v, lg, num_sms, rows, stream, std::make_index_sequence<kNumVariants>{});
+      sided = true;
     }
+    if (sided) join_side(side, stream);
     if (ev) cudaEventRecord(ev[3], stream);
     return;
   }
@@ -2486,10 +2518,11 @@ void launch_dense_t(const BatchView &bv, int num_sms, cudaStream_t stream, cudaE
   if (ev) cudaEventRecord(ev[3], stream);
 }
 
-void launch_dense(const BatchView &bv, int num_sms, cudaStream_t stream, cudaEvent_t *ev, int precision) {
+void launch_dense(const BatchView &bv, int num_sms, cudaStream_t stream, cudaEvent_t *ev, int precision,
+                  const DenseSide *side) {
   if (bv.total_tiles <= 0) return;
-  if (precision == 1) launch_dense_t<true>(bv, num_sms, stream, ev);
-  else launch_dense_t<false>(bv, num_sms, stream, ev);
+  if (precision == 1) launch_dense_t<true>(bv, num_sms, stream, ev, side);
+  else launch_dense_t<false>(bv, num_sms, stream, ev, side);
 }
 
 // The phases of the samples after the plunge buffer hold their values at
@@ -2518,20 +2551,22 @@ __global__ void __launch_bounds__(256) k_phase_freeze(const SourceDesc *__restri
   }
 }
 
-void launch_phase(const BatchView &bv, int num_sms, cudaStream_t stream, cudaEvent_t *ev) {
+void launch_phase(const BatchView &bv, int num_sms, cudaStream_t stream, cudaEvent_t *ev, const DenseSide *side) {
   if (bv.total_tiles <= 0 || !bv.phase_out || !bv.tile_prep || !bv.tile_seg || !bv.frozen) return;
   if (ev) cudaEventRecord(ev[0], stream);
   prepare_dense_launch();
   if (bv.small_tiles > 0) {
     // the tile parameters from the pre-pass, each tile's inputs staged by bulk copies, carries by look-back
+    const bool only = bv.small_tiles == bv.total_tiles;
+    const cudaStream_t st = only ? stream : fork_side(side, 0, stream);
     BatchView sm = bv;
     sm.total_tiles = bv.small_tiles;
-    cudaMemsetAsync(bv.work_counter, 0, sizeof(unsigned long long), stream);
-    cudaMemsetAsync(bv.link_flag, 0, (size_t)bv.total_tiles * sizeof(int32_t), stream);
-    k_tile_params<false><<<(unsigned)((bv.total_tiles + 127) / 128), 128, 0, stream>>>(bv);
-    launch_persistent(k_waveform<false, 1, true, 0, 3>, sm, num_sms, kWaveDynSmem, stream);
+    cudaMemsetAsync(bv.work_counter, 0, sizeof(unsigned long long), st);
+    cudaMemsetAsync(bv.link_flag, 0, (size_t)bv.total_tiles * sizeof(int32_t), st);
+    k_tile_params<false><<<(unsigned)((bv.total_tiles + 127) / 128), 128, 0, st>>>(bv);
+    launch_persistent(k_waveform<false, 1, true, 0, 3>, sm, num_sms, kWaveDynSmem, st);
     const dim3 fgrid(64, (unsigned)std::min(std::max(bv.nsrc, 1), 1024));
-    k_phase_freeze<<<fgrid, 256, 0, stream>>>(bv.src, bv.nsrc, bv.phase_out, bv.phase_stride);
+    k_phase_freeze<<<fgrid, 256, 0, st>>>(bv.src, bv.nsrc, bv.phase_out, bv.phase_stride);
   }
   if (ev) cudaEventRecord(ev[1], stream);
   if (ev) cudaEventRecord(ev[2], stream);
@@ -2542,6 +2577,7 @@ void launch_phase(const BatchView &bv, int num_sms, cudaStream_t stream, cudaEve
     launch_segments<true>(lg, num_sms, 0, stream, nullptr);
     if (ev) cudaEventRecord(ev[2], stream);
     launch_persistent(k_waveform<false, 1, true, 0, 3, true>, lg, num_sms, kWaveDynSmem, stream);
+    if (bv.small_tiles > 0) join_side(side, stream);
   }
   if (ev) cudaEventRecord(ev[3], stream);
 }

@@ -70,13 +70,12 @@ struct alignas(16) TileHead {
 static_assert(sizeof(TileHead) == 96, "the coefficients after the head stay 16-byte aligned");
 constexpr int64_t kSegSlotBytes = 96 + 4 * 108 * 8;  // head, 4 segments of at most 108 doubles
 // Phase increments of one tile: forward and backward sums, and the clamped
-// Phidot after its last forward sample (kept in the look-back records' memory).
+// Phidot after its last forward sample.
 struct SegAgg {
   double f[3], b[3];
   double lastP;
   int32_t hasP, needC;  // lastP was set in the tile; the sums wait for the clamped Phidot before the tile
 };
-static_assert(sizeof(SegAgg) <= sizeof(TileLink), "an aggregate fits in the tile's look-back record");
 // words of seg_ctl, cleared before every launch: queue heads, direct tiles,
 // then per source its direct tiles, and per source those of them summed
 constexpr int kCtlQueue = 0, kCtlDirectQueue = 1, kCtlDirectCount = 2, kCtlSource = 4;
@@ -198,10 +197,18 @@ struct BatchView {
 // shared memory with bulk copies.  ev (optional, 4 events): ev[0]..ev[1]
 // bracket the clears, ev[1]..ev[2] the pre-pass (empty without it),
 // ev[2]..ev[3] the waveform kernel.
+// side: a second stream for the parts of an FP64 launch that depend on one
+// another only through `stream` (forked from it and joined to it by events, so
+// that a captured launch stays one graph); null: everything on `stream`.
+struct DenseSide {
+  cudaStream_t stream = nullptr;
+  cudaEvent_t fork[2] = {nullptr, nullptr}, join = nullptr;
+};
 void launch_dense_fp64(const BatchView &bv, int num_sms, cudaStream_t stream, cudaEvent_t *ev);
 // precision 0: FP64 throughout; 1: split (FP64 phases and reductions, FP32
 // geometry, response, Bessel evaluation and harmonic recurrence).
-void launch_dense(const BatchView &bv, int num_sms, cudaStream_t stream, cudaEvent_t *ev, int precision);
+void launch_dense(const BatchView &bv, int num_sms, cudaStream_t stream, cudaEvent_t *ev, int precision,
+                  const DenseSide *side = nullptr);
 // ------------------------------------------------------------------ frequency-domain TDI
 // Rows of the TDI phase grid that launch_tdi_grid writes to bv.phase_out
 // (kTdiRows x phase_stride, indexed by src.out_offset + i): the grid time,
@@ -246,7 +253,8 @@ void launch_tdi_spa(const TdiArgs &a, cudaStream_t stream);
 // pass over all samples (no harmonic sums), then the freeze of the phases
 // after the plunge buffer.  ev (optional, 4 events) as launch_dense, ev[3]
 // after the freeze.
-void launch_phase(const BatchView &bv, int num_sms, cudaStream_t stream, cudaEvent_t *ev);
+void launch_phase(const BatchView &bv, int num_sms, cudaStream_t stream, cudaEvent_t *ev,
+                  const DenseSide *side = nullptr);
 
 // Plain FP64 per-source harmonic sum: the per-sample algorithm of the
 // reference's CUDA port (src/cuda/kernel.cu:374-555) -- five Bessel functions

@@ -803,32 +803,35 @@ __device__ __forceinline__ int2 seg_stage(const BatchView &bv, int64_t j, unsign
 // the tile before it runs, and a thread needs no other barrier: its slot m is
 // the same in every segment, so x is a constant of the thread.  Bound by FP64
 // issue: at 30 harmonics (K = 5) 20 of 29 instructions of a sample are the mode
-// sums, J samples a thread share their table loads.
+// sums, J samples a thread share their table loads.  parts (1, or 2 where J
+// divides half a tile): queue entries a tile, each with its share of the
+// segments, so that a small batch fills the chip.
 template <int J, int kMinB>
-__global__ void __launch_bounds__(kTileThreads, kMinB) k_wave_segments(BatchView bv, int stage_bytes) {
+__global__ void __launch_bounds__(kTileThreads, kMinB) k_wave_segments(BatchView bv, int stage_bytes, int parts) {
   extern __shared__ __align__(16) unsigned char s_stage[];
   __shared__ __align__(8) uint64_t s_bar[2];
   __shared__ long long s_next[2];
   __shared__ int2 s_what[2];  // place in the source, mode
   const int tid = threadIdx.x;
   const double x = ((double)tid - kSegMid) * (1.0 / kSegHalf);
+  const long long units = (long long)bv.total_tiles * parts;
   if (tid == 0) {
     mbar_init(&s_bar[0], 1);
     mbar_init(&s_bar[1], 1);
     mbar_init_fence();
     const long long j = (long long)atomicAdd(bv.seg_ctl + kCtlQueue, 1);
     s_next[0] = j;
-    if (j < bv.total_tiles) s_what[0] = seg_stage(bv, j, s_stage, &s_bar[0]);
+    if (j < units) s_what[0] = seg_stage(bv, j / parts, s_stage, &s_bar[0]);
   }
   __syncthreads();
   uint32_t parity = 0u;  // bit b: phase of barrier b
   for (int b = 0;; b ^= 1) {
     const long long j = s_next[b];
-    if (j >= bv.total_tiles) break;
+    if (j >= units) break;
     if (tid == 0) {
       const long long jn = (long long)atomicAdd(bv.seg_ctl + kCtlQueue, 1);
       s_next[b ^ 1] = jn;
-      if (jn < bv.total_tiles) s_what[b ^ 1] = seg_stage(bv, jn, s_stage + (b ^ 1) * stage_bytes, &s_bar[b ^ 1]);
+      if (jn < units) s_what[b ^ 1] = seg_stage(bv, jn / parts, s_stage + (b ^ 1) * stage_bytes, &s_bar[b ^ 1]);
     }
     const int mode = s_what[b].y;
     const int start = s_what[b].x * kTileSamples;
@@ -851,8 +854,9 @@ __global__ void __launch_bounds__(kTileThreads, kMinB) k_wave_segments(BatchView
     const int lim = (mode > 0) ? min(end, n_eff(d)) : start;
     const int K = H.K;
     const int sd2 = seg_doubles(mode == 4 ? 4 : 7, false) / 2;
+    const int first = (int)(j % parts) * (kTileChunks / parts), past = first + kTileChunks / parts;
 #pragma unroll 1
-    for (int g0 = 0; g0 < kTileChunks; g0 += J) {
+    for (int g0 = first; g0 < past; g0 += J) {
       if (start + 256 * g0 >= end) break;
       double dl[J], c1[J], s1[J], cD[J], sD[J], Sa[J], Sb[J], Sc[J];
 #pragma unroll
