@@ -77,8 +77,12 @@ struct aak_ctx {
   std::vector<SourceDesc> descs;
   std::vector<int64_t> tile_start;
   std::vector<int64_t> tile_pairs;  // per source {0, its tiles}: the tile prefix of a one-source view
-  std::vector<QueueItem> queue;     // work-queue order of the tiles, with what staging each needs
-  std::vector<int32_t> tile_knot;  // 2 per tile: first knot of the tile window, knots in it
+  // work-queue order (the queue itself and the tiles' knot windows are made on
+  // the device): per source its place in a chain step, then per class (small
+  // sources, the others) the first queue entry of every chain step
+  std::vector<int32_t> queue_rank;
+  std::vector<int64_t> queue_step;
+  int32_t large_steps = 0;  // index in queue_step of the second class
   std::vector<int64_t> kofs;       // nsrc + 1 prefix of knots (the sources' knots stay in their plans)
   std::vector<int64_t> spl_blk;    // nsrc + 1 prefix of the device spline solve's blocks
   int spl_len = kSplineBlockShort; // knots per block of the device spline solve
@@ -91,9 +95,9 @@ struct aak_ctx {
   bool uploaded = false;
   // device buffers
   DevBuf<SourceDesc> d_src;
-  DevBuf<int64_t> d_tile_start, d_tile_pairs, d_spl_blk;
+  DevBuf<int64_t> d_tile_start, d_tile_pairs, d_spl_blk, d_queue_step;
   DevBuf<QueueItem> d_queue;
-  DevBuf<int32_t> d_tile_knot;
+  DevBuf<int32_t> d_tile_knot, d_queue_rank;
   DevBuf<double> d_knot_t;
   DevBuf<double4> d_knot_y, d_knot_c;
   DevBuf<int32_t> d_bessel;
@@ -251,7 +255,6 @@ int pack(aak_ctx *ctx, const std::vector<aak_params> &P, int nthreads) {
     ctx->spl_blk[s + 1] = ctx->spl_blk[s] + (ctx->status[s] == AAK_OK ? spline_blocks((int)ctx->plans[s].knot_t.size(), ctx->spl_len) : 0);
   ctx->tile_pairs.assign(2 * (size_t)n, 0);
   for (int s = 0; s < n; ++s) ctx->tile_pairs[2 * s + 1] = ctx->tile_start[s + 1] - ctx->tile_start[s];
-  ctx->tile_knot.assign(2 * std::max<int64_t>(ctx->total_tiles, 1), 0);
   parallel_for(n, nthreads, [&](int64_t s64) {
     const int s = (int)s64;
     SourceDesc d;
@@ -271,69 +274,37 @@ int pack(aak_ctx *ctx, const std::vector<aak_params> &P, int nthreads) {
     d.tile_offset = ctx->tile_start[s];
     d.n_tiles = (int32_t)(ctx->tile_start[s + 1] - ctx->tile_start[s]);
     ctx->descs[s] = d;
-    if (ctx->status[s] != AAK_OK) return;
-    // knot window of every tile: knots bracketing samples start-1 .. start+1024.
-    // k0 is the last knot in [k0, nk - 2] with kt[k0] <= ta (kept at least at
-    // its previous value), k1 the same for tb; found by binary search, so the
-    // cost follows the tiles, not the knots (sources may have thousands of
-    // knots per tile)
-    const double *kt = pl.knot_t.data();
-    const int nk = d.n_knots;
-    auto tsample = [&](int i) { return (i == 0) ? d.t_first : (double)(i - d.i0) * d.dt; };
-    auto last_le = [&](int lo, double x) {  // largest k in [lo, nk - 2] with kt[k] <= x, else lo
-      if (lo + 1 > nk - 2) return lo;
-      return (int)(std::upper_bound(kt + lo + 1, kt + nk - 1, x) - kt) - 1;
-    };
-    int k0 = 0, k1 = 0;
-    for (int64_t t = 0; t < d.n_tiles; ++t) {
-      const int start = (int)(t * kTileSamples);
-      const double ta = tsample(std::max(start - 1, 0));
-      const double tb = tsample(std::min(start + kTileSamples, d.vlength - 1));
-      k0 = last_le(k0, ta);
-      k1 = last_le(std::max(k1, k0), tb);
-      ctx->tile_knot[2 * (d.tile_offset + t)] = k0;
-      ctx->tile_knot[2 * (d.tile_offset + t) + 1] = k1 + 2 - k0;
-    }
   });
-  // work-queue order: chain step major, source minor.  Step 0 of a source is
-  // its head tile (the one holding t = 0), then come its later tiles in
-  // increasing order, then its earlier ones in decreasing order; interleaving
-  // the sources puts a tile's chain predecessor a whole batch row earlier in
-  // the queue, so that on many-source batches it is finished when the tile
-  // looks back at it.  The head rule is the waveform kernel's.
-  std::vector<int> T(n), head(n);
-  int maxT = 0;
-  for (int s = 0; s < n; ++s) {
-    T[s] = (int)(ctx->tile_start[s + 1] - ctx->tile_start[s]);
-    const int i0 = ctx->descs[s].i0;
-    head[s] = (i0 <= 0 || T[s] == 0) ? 0 : std::min(i0 / kTileSamples, T[s] - 1);
-    maxT = std::max(maxT, T[s]);
-  }
-  // Each item also carries the tile's knot window and whether it has output
-  // (the waveform kernel's test: a failed source, or a tile that starts at or
-  // after the taper's end, min(vlength, i_plunge + i_buffer)).
-  ctx->queue.assign(std::max<int64_t>(ctx->total_tiles, 1), QueueItem{});
+  // work-queue order: the small sources' tiles (kSmallTiles) before the others',
+  // in each class chain step major, source minor.  Step 0 of a source is its
+  // head tile (the one holding t = 0), then come its later tiles in increasing
+  // order, then its earlier ones in decreasing order; interleaving the sources
+  // puts a tile's chain predecessor a whole batch row earlier in the queue, so
+  // that on many-source batches it is finished when the tile looks back at it.
+  // Inside a step the sources are ranked by their number of tiles, so that
+  // those still running at a step are its first ones and a source's rank is
+  // the same in each of its steps.
+  ctx->queue_rank.assign(std::max(n, 1), 0);
+  ctx->queue_step.clear();
   int64_t q = 0;
-  for (int small = 1; small >= 0; --small) {  // the small sources' tiles first (kSmallTiles)
-    for (int k = 0; k < maxT; ++k)
-      for (int s = 0; s < n; ++s)
-        if (k < T[s] && (T[s] <= kSmallTiles) == (small == 1)) {
-          const SourceDesc &d = ctx->descs[s];
-          const int lt = (k < T[s] - head[s]) ? head[s] + k : T[s] - 1 - k;
-          const int64_t g = ctx->tile_start[s] + lt;
-          const long long neff = std::min<long long>(d.vlength, (long long)d.i_plunge + (long long)d.i_buffer);
-          QueueItem &it = ctx->queue[q++];
-          it.g = (int32_t)g;
-          it.s = s;
-          it.lt = lt;
-          it.k0 = ctx->tile_knot[2 * g];
-          it.nk = ctx->tile_knot[2 * g + 1];
-          it.knot = d.knot_offset + it.k0;
-          it.flags = (d.status != 0 ? kQueueFailed | kQueueNoWave : 0) |
-                     ((long long)lt * kTileSamples >= neff ? kQueueNoWave : 0);
-        }
+  for (int small = 1; small >= 0; --small) {
+    std::vector<int> order;
+    for (int s = 0; s < n; ++s)
+      if ((ctx->descs[s].n_tiles <= kSmallTiles) == (small == 1)) order.push_back(s);
+    std::stable_sort(order.begin(), order.end(),
+                     [&](int x, int y) { return ctx->descs[x].n_tiles > ctx->descs[y].n_tiles; });
+    for (size_t i = 0; i < order.size(); ++i) ctx->queue_rank[order[i]] = (int32_t)i;
+    if (small == 0) ctx->large_steps = (int32_t)ctx->queue_step.size();
+    size_t live = order.size();
+    const int steps = order.empty() ? 0 : ctx->descs[order[0]].n_tiles;
+    for (int k = 0; k < steps; ++k) {
+      while (live > 0 && ctx->descs[order[live - 1]].n_tiles <= k) --live;
+      ctx->queue_step.push_back(q);
+      q += (int64_t)live;
+    }
     if (small == 1) ctx->small_tiles = q;
   }
+  if (ctx->queue_step.empty()) ctx->queue_step.push_back(0);
   ctx->uploaded = false;
   return AAK_OK;
 }
@@ -766,8 +737,11 @@ int upload(aak_ctx *ctx, cudaStream_t st, bool wait_pinned = true) {
   if ((r = select_device(ctx->device)) != AAK_OK) return r;
   const int n = ctx->nsrc;
   if ((r = ctx->d_src.reserve(n)) || (r = ctx->d_tile_start.reserve(n + 1)) ||
-      (r = ctx->d_tile_knot.reserve(ctx->tile_knot.size())) || (r = ctx->d_tile_pairs.reserve(ctx->tile_pairs.size())) ||
-      (r = ctx->d_queue.reserve(ctx->queue.size())) || (r = ctx->d_spl_blk.reserve(ctx->spl_blk.size())) ||
+      (r = ctx->d_tile_knot.reserve(2 * std::max<int64_t>(ctx->total_tiles, 1))) ||
+      (r = ctx->d_tile_pairs.reserve(ctx->tile_pairs.size())) ||
+      (r = ctx->d_queue.reserve(std::max<int64_t>(ctx->total_tiles, 1))) ||
+      (r = ctx->d_queue_rank.reserve(ctx->queue_rank.size())) || (r = ctx->d_queue_step.reserve(ctx->queue_step.size())) ||
+      (r = ctx->d_spl_blk.reserve(ctx->spl_blk.size())) ||
       // knot times: two entries of slack past the last knot (a window's bulk
       // copy starts on a 16-byte boundary and may read one element beyond it)
       (r = ctx->d_knot_t.reserve(std::max<int64_t>(ctx->total_knots, 1) + 2)) ||
@@ -783,9 +757,9 @@ int upload(aak_ctx *ctx, cudaStream_t st, bool wait_pinned = true) {
   };
   if ((r = cp(ctx->d_src.ptr, ctx->descs.data(), n * sizeof(SourceDesc))) ||
       (r = cp(ctx->d_tile_start.ptr, ctx->tile_start.data(), (n + 1) * sizeof(int64_t))) ||
-      (r = cp(ctx->d_tile_knot.ptr, ctx->tile_knot.data(), ctx->tile_knot.size() * sizeof(int32_t))) ||
+      (r = cp(ctx->d_queue_rank.ptr, ctx->queue_rank.data(), ctx->queue_rank.size() * sizeof(int32_t))) ||
+      (r = cp(ctx->d_queue_step.ptr, ctx->queue_step.data(), ctx->queue_step.size() * sizeof(int64_t))) ||
       (r = cp(ctx->d_tile_pairs.ptr, ctx->tile_pairs.data(), ctx->tile_pairs.size() * sizeof(int64_t))) ||
-      (r = cp(ctx->d_queue.ptr, ctx->queue.data(), ctx->queue.size() * sizeof(QueueItem))) ||
       (r = cp(ctx->d_spl_blk.ptr, ctx->spl_blk.data(), ctx->spl_blk.size() * sizeof(int64_t))) ||
       (r = cp(ctx->d_bessel.ptr, ctx->bessel.data(), ctx->bessel.size() * sizeof(int32_t))))
     return r;
@@ -799,7 +773,9 @@ int upload(aak_ctx *ctx, cudaStream_t st, bool wait_pinned = true) {
         (r = cp(ctx->d_knot_y.ptr + ko, pl.knot_y.data(), nk * sizeof(double4))))
       return r;
   }
-  // spline coefficients of every source, solved on the device
+  // the tiles' knot windows and the work queue, and the spline coefficients of every source, made on the device
+  launch_tile_layout(ctx->d_src.ptr, n, ctx->d_tile_start.ptr, ctx->total_tiles, ctx->d_knot_t.ptr, ctx->d_tile_knot.ptr,
+                     ctx->d_queue.ptr, ctx->d_queue_rank.ptr, ctx->d_queue_step.ptr, ctx->large_steps, st);
   launch_spline_coeffs(ctx->d_src.ptr, n, ctx->d_spl_blk.ptr, ctx->spl_blk[n], ctx->spl_len, ctx->d_knot_t.ptr, ctx->d_knot_y.ptr,
                        ctx->d_knot_c.ptr, st);
   if ((r = cuda_ok(cudaGetLastError())) != AAK_OK) return r;
@@ -1528,6 +1504,8 @@ void aak_ctx_destroy(aak_ctx *c) {
     c->d_src.release();
     c->d_tile_start.release();
     c->d_tile_knot.release();
+    c->d_queue_rank.release();
+    c->d_queue_step.release();
     c->d_tile_pairs.release();
     c->d_queue.release();
     c->d_spl_blk.release();
@@ -1613,12 +1591,12 @@ int aak_batch_info(aak_ctx *ctx, int64_t *total, int64_t *offsets, int32_t *stat
 int aak_batch_plan_bytes(aak_ctx *ctx, int64_t *bytes) {
   if (!ctx || !bytes) return AAK_ERR_INVALID_PARAM;
   std::lock_guard<std::mutex> lk(ctx->mu);
-  // everything upload() copies: descriptors, tile and queue arrays, knots (t and
+  // everything upload() copies: descriptors, tile prefixes and queue order, knots (t and
   // (e, v, M, S); the spline coefficients are solved on the device), Miller
   // start orders and the spline-block prefix
   *bytes = (int64_t)(ctx->descs.size() * sizeof(SourceDesc) + ctx->tile_start.size() * sizeof(int64_t) +
-                     ctx->tile_knot.size() * sizeof(int32_t) + ctx->tile_pairs.size() * sizeof(int64_t) +
-                     ctx->queue.size() * sizeof(QueueItem) + ctx->total_knots * (sizeof(double) + sizeof(double4)) +
+                     ctx->queue_rank.size() * sizeof(int32_t) + ctx->queue_step.size() * sizeof(int64_t) +
+                     ctx->tile_pairs.size() * sizeof(int64_t) + ctx->total_knots * (sizeof(double) + sizeof(double4)) +
                      ctx->bessel.size() * sizeof(int32_t) + ctx->spl_blk.size() * sizeof(int64_t));
   return AAK_OK;
 }
@@ -1653,7 +1631,7 @@ int aak_batch_run_noalloc(aak_ctx *ctx, void *d_plan, int64_t plan_bytes, int64_
   auto al = [](size_t x) { return (x + 255) / 256 * 256; };
   const size_t o_ts = al(ctx->descs.size() * sizeof(SourceDesc));
   const size_t o_tk = o_ts + al(ctx->tile_start.size() * sizeof(int64_t));
-  const size_t o_kt = o_tk + al(ctx->tile_knot.size() * sizeof(int32_t));
+  const size_t o_kt = o_tk + al(2 * (size_t)std::max<int64_t>(ctx->total_tiles, 1) * sizeof(int32_t));
   const size_t nknots = (size_t)std::max<int64_t>(ctx->total_knots, 1);
   const size_t o_ky = o_kt + al(nknots * sizeof(double));
   const size_t o_kc = o_ky + al(nknots * sizeof(double4));
@@ -1674,7 +1652,6 @@ int aak_batch_run_noalloc(aak_ctx *ctx, void *d_plan, int64_t plan_bytes, int64_
   };
   if ((r = cp(0, ctx->descs.data(), ctx->descs.size() * sizeof(SourceDesc))) ||
       (r = cp(o_ts, ctx->tile_start.data(), ctx->tile_start.size() * sizeof(int64_t))) ||
-      (r = cp(o_tk, ctx->tile_knot.data(), ctx->tile_knot.size() * sizeof(int32_t))) ||
       (r = cp(o_bs, ctx->bessel.data(), ctx->bessel.size() * sizeof(int32_t))) ||
       (r = cp(o_sb, ctx->spl_blk.data(), ctx->spl_blk.size() * sizeof(int64_t))))
     return r;
@@ -1687,6 +1664,9 @@ int aak_batch_run_noalloc(aak_ctx *ctx, void *d_plan, int64_t plan_bytes, int64_
         (r = cp(o_ky + ko * sizeof(double4), pl.knot_y.data(), nk * sizeof(double4))))
       return r;
   }
+  launch_tile_layout(reinterpret_cast<const SourceDesc *>(base), ctx->nsrc, reinterpret_cast<const int64_t *>(base + o_ts),
+                     ctx->total_tiles, reinterpret_cast<const double *>(base + o_kt),
+                     reinterpret_cast<int32_t *>(base + o_tk), nullptr, nullptr, nullptr, 0, st);
   launch_spline_coeffs(reinterpret_cast<const SourceDesc *>(base), ctx->nsrc, reinterpret_cast<const int64_t *>(base + o_sb),
                        ctx->spl_blk[ctx->nsrc], ctx->spl_len, reinterpret_cast<const double *>(base + o_kt),
                        reinterpret_cast<const double4 *>(base + o_ky), reinterpret_cast<double4 *>(base + o_kc), st);

@@ -283,6 +283,14 @@ inline int64_t spline_blocks(int n_knots, int block) { return n_knots < 3 ? 1 : 
 void launch_spline_coeffs(const SourceDesc *src, int nsrc, const int64_t *blk_start, int64_t total_blocks, int block,
                           const double *knot_t, const double4 *knot_y, double4 *knot_c, cudaStream_t stream);
 
+// The knot window of every tile of a batch (tile_knot, 2 per tile: the knots
+// bracketing samples start - 1 .. start + 1024) and, with queue set, its entry
+// in the work queue: entry step[k] + rank[s] for chain step k of source s, step
+// holding the small sources' chain steps and from large_steps on the others'.
+void launch_tile_layout(const SourceDesc *src, int nsrc, const int64_t *tile_start, int64_t tiles, const double *knot_t,
+                        int32_t *tile_knot, QueueItem *queue, const int32_t *rank, const int64_t *step,
+                        int32_t large_steps, cudaStream_t stream);
+
 void launch_plain_waveform(const SourceDesc *src, int s, int vlength, const double *traj, int64_t traj_stride,
                            double *hI, double *hII, cudaStream_t stream);
 
