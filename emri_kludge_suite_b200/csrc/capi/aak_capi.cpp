@@ -2052,6 +2052,7 @@ int aak_genwave(double *t, double *hI, double *hII, double timestep, int32_t vle
 // GPUAAK counterpart (include/AAK_manager.hh:106-153, src/cuda/AAK_manager.cu):
 // templates are generated into FFT-padded rows, transformed in place by a
 // batched cuFFT D2Z plan and reduced against the pre-weighted data.
+constexpr int kUnitsMax = 32;  // planning units of one chunk at most
 struct aak_gpu {
   aak_ctx *ctx = nullptr;
   double T_fit = 1.0, dt = 0.0, init_dt = 0.0;
@@ -2060,29 +2061,44 @@ struct aak_gpu {
   int64_t row = 0;    // doubles per padded template row = 2 * nbins
   DevBuf<double> d_H[2], d_D[2], d_w[2], d_partial, d_out, d_t;
   DevBuf<double> d_fisher;  // Fisher Gram partial sums and the 2 x nd x nd result
-  cufftHandle plan = 0;
-  int plan_batch = 0;
+  // transform plans by kind and batch (exact sizes: a larger plan would
+  // transform stale rows), the oldest replaced; one work area for all (they run
+  // on the likelihood's stream)
+  struct FftPlan {
+    cufftType kind;
+    int batch;
+    size_t work;
+    uint64_t used;
+    cufftHandle handle;
+  };
+  std::vector<FftPlan> plans;
+  uint64_t plan_clock = 0;
+  DevBuf<unsigned char> d_fft_work;
   // precision 2: FP32 template rows, an FP32 R2C transform and the FP32 copies
   // of the data and weights (the compensated FP32 inner products)
   DevBuf<float> d_H32[2], d_D32[2], d_w32[2];
-  cufftHandle plan32 = 0;
-  int plan32_batch = 0;
   bool rows32 = false;   // the rows of the last generation are the FP32 ones
   int32_t count = 0;     // templates currently in the rows
   bool spectral = false; // rows hold spectra (after a likelihood)
+  bool packed = false;   // those spectra are packed (launch_inner_products_packed)
   std::vector<double> like;
   double ms[4] = {0, 0, 0, 0};  // host plan, generate, FFT, reduce of the last batch
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
   // device work of the templates: its own non-blocking stream, so that host
   // planning (and the warm-start model's copies) can overlap it
   cudaStream_t stream = nullptr;
-  // likelihood batches in chunks, double-buffered: chunk c is planned into
-  // ctxs()[c & 1] and uploaded on up_stream while the chunk before it runs
+  // batches in chunks, each planned in units that alternate between two
+  // contexts: a unit is uploaded on up_stream and generated while the next is planned
   aak_ctx *ctx2 = nullptr;
   cudaStream_t up_stream = nullptr;
-  // per parity: upload done, generation done, generation start, transform
-  // done, reduction done, results copied
-  cudaEvent_t pev[2][6] = {{nullptr}};
+  // per parity of the chunk: generation done, transform done, reduction done,
+  // results copied; per planning context: upload done, generation done; and the
+  // start and end of each unit's generation
+  cudaEvent_t pev[2][4] = {{nullptr}};
+  cudaEvent_t uev[2][2] = {{nullptr}};
+  cudaEvent_t tev[2][kUnitsMax][2] = {{{nullptr}}};
+  int units[2] = {0, 0};  // units of the chunk in each slot
+  uint64_t unit = 0;      // units launched so far: unit k plans into context k & 1
   double *h_stage = nullptr;  // page-locked results of the two chunks in flight (2 x 2 x stage_cap)
   int stage_cap = 0;
 };
@@ -2094,19 +2110,6 @@ int gpu_capacity(aak_gpu *g, int B) {
   if ((r = g->d_H[0].reserve((size_t)B * g->row)) || (r = g->d_H[1].reserve((size_t)B * g->row)) ||
       (r = g->d_partial.reserve((size_t)B * kIpBlocksPerTemplate * 2)) || (r = g->d_out.reserve((size_t)B * 2)))
     return r;
-  if (g->plan_batch < B) {
-    if (g->plan) cufftDestroy(g->plan);
-    g->plan = 0;
-    g->plan_batch = 0;
-    int n = g->length;
-    int inembed = (int)g->row, onembed = (int)(g->row / 2);
-    if (cufftPlanMany(&g->plan, 1, &n, &inembed, 1, (int)g->row, &onembed, 1, (int)(g->row / 2), CUFFT_D2Z, B) !=
-        CUFFT_SUCCESS) {
-      g->plan = 0;
-      return AAK_ERR_CUDA;
-    }
-    g->plan_batch = B;
-  }
   return AAK_OK;
 }
 
@@ -2115,19 +2118,49 @@ int gpu_capacity32(aak_gpu *g, int B) {
   if ((r = g->d_H32[0].reserve((size_t)B * g->row)) || (r = g->d_H32[1].reserve((size_t)B * g->row)) ||
       (r = g->d_partial.reserve((size_t)B * kIpBlocksPerTemplate * 2)) || (r = g->d_out.reserve((size_t)B * 2)))
     return r;
-  if (g->plan32_batch != B) {  // an exact-size plan: a larger one would transform stale rows
-    if (g->plan32) cufftDestroy(g->plan32);
-    g->plan32 = 0;
-    g->plan32_batch = 0;
-    int n = g->length;
-    int inembed = (int)g->row, onembed = (int)(g->row / 2);
-    if (cufftPlanMany(&g->plan32, 1, &n, &inembed, 1, (int)g->row, &onembed, 1, (int)(g->row / 2), CUFFT_R2C, B) !=
-        CUFFT_SUCCESS) {
-      g->plan32 = 0;
+  return AAK_OK;
+}
+
+// The in-place transform of the rows for a batch of B, ready on the
+// likelihood's stream: CUFFT_D2Z and CUFFT_R2C of the padded real rows, or
+// CUFFT_Z2Z of half the length (packed).  Kept: a call's full and ragged
+// chunks, a Fisher batch and a likelihood batch each have a size of their own.
+constexpr size_t kFftPlans = 6;
+void drop_fft_plan(aak_gpu *g, size_t k) {
+  cudaStreamSynchronize(g->stream);
+  cufftDestroy(g->plans[k].handle);
+  g->plans.erase(g->plans.begin() + (ptrdiff_t)k);
+}
+int fft_plan(aak_gpu *g, cufftType kind, int B, cufftHandle *out) {
+  size_t k = 0;
+  while (k < g->plans.size() && (g->plans[k].kind != kind || g->plans[k].batch != B)) ++k;
+  if (k == g->plans.size()) {
+    if (g->plans.size() >= kFftPlans) {
+      size_t old = 0;
+      for (size_t i = 1; i < g->plans.size(); ++i)
+        if (g->plans[i].used < g->plans[old].used) old = i;
+      drop_fft_plan(g, old);
+    }
+    aak_gpu::FftPlan p{kind, B, 0, 0, 0};
+    int n = (kind == CUFFT_Z2Z) ? g->length / 2 : g->length;
+    int in = (int)((kind == CUFFT_Z2Z) ? g->row / 2 : g->row), spec = (int)(g->row / 2);
+    if (cufftCreate(&p.handle) != CUFFT_SUCCESS) return AAK_ERR_CUDA;
+    if (cufftSetAutoAllocation(p.handle, 0) != CUFFT_SUCCESS ||
+        cufftMakePlanMany(p.handle, 1, &n, &in, 1, in, &spec, 1, spec, kind, B, &p.work) != CUFFT_SUCCESS) {
+      cufftDestroy(p.handle);
       return AAK_ERR_CUDA;
     }
-    g->plan32_batch = B;
+    g->plans.push_back(p);
+    k = g->plans.size() - 1;
   }
+  aak_gpu::FftPlan &p = g->plans[k];
+  p.used = ++g->plan_clock;
+  const int r = g->d_fft_work.reserve(std::max<size_t>(p.work, 1));
+  if (r != AAK_OK) return r;
+  if (cufftSetWorkArea(p.handle, g->d_fft_work.ptr) != CUFFT_SUCCESS ||
+      cufftSetStream(p.handle, g->stream) != CUFFT_SUCCESS)
+    return AAK_ERR_CUDA;
+  *out = p.handle;
   return AAK_OK;
 }
 
@@ -2252,7 +2285,7 @@ int gpu_launch(aak_gpu *g, int B, bool with_t, bool rows32 = false) {
     if ((r = run_rows32(g->ctx, g->d_H32[0].ptr, g->d_H32[1].ptr, 1, g->stream)) != AAK_OK) return r;
     cudaEventRecord(g->ev[1], g->stream);
     g->count = B;
-    g->spectral = false;
+    g->spectral = g->packed = false;
     g->rows32 = true;
     return AAK_OK;
   }
@@ -2273,7 +2306,7 @@ int gpu_launch(aak_gpu *g, int B, bool with_t, bool rows32 = false) {
     return r;
   cudaEventRecord(g->ev[1], g->stream);
   g->count = B;
-  g->spectral = false;
+  g->spectral = g->packed = false;
   return AAK_OK;
 }
 
@@ -2282,32 +2315,36 @@ int gpu_generate(aak_gpu *g, const double *x, int B, int nthreads, int32_t *stat
   return r != AAK_OK ? r : gpu_launch(g, B, with_t);
 }
 
-// In-place D2Z transforms of the rows of both channels (once per generation).
-int gpu_fft_rows(aak_gpu *g) {
+// In-place transforms of the rows of both channels (once per generation).
+// pack: leave FP64 rows of even length packed, for a reduction that reads them
+// so; otherwise the rows end as half spectra, packed ones of an earlier call too.
+int gpu_fft_rows(aak_gpu *g, bool pack = false) {
+  cufftHandle h;
+  int r;
   if (!g->spectral && g->rows32) {
-    int r = gpu_capacity32(g, g->count);
-    if (r != AAK_OK) return r;
-    if (cufftSetStream(g->plan32, g->stream) != CUFFT_SUCCESS) return AAK_ERR_CUDA;
-    if (cufftExecR2C(g->plan32, g->d_H32[0].ptr, reinterpret_cast<cufftComplex *>(g->d_H32[0].ptr)) != CUFFT_SUCCESS ||
-        cufftExecR2C(g->plan32, g->d_H32[1].ptr, reinterpret_cast<cufftComplex *>(g->d_H32[1].ptr)) != CUFFT_SUCCESS)
-      return AAK_ERR_CUDA;
+    if ((r = fft_plan(g, CUFFT_R2C, g->count, &h)) != AAK_OK) return r;
+    for (int ch = 0; ch < 2; ++ch)
+      if (cufftExecR2C(h, g->d_H32[ch].ptr, reinterpret_cast<cufftComplex *>(g->d_H32[ch].ptr)) != CUFFT_SUCCESS)
+        return AAK_ERR_CUDA;
     g->spectral = true;
+    g->packed = false;
     return AAK_OK;
   }
   if (!g->spectral) {
-    if (g->plan_batch != g->count) {
-      // a plan of a larger batch would transform stale rows: make one of this size
-      if (g->plan) cufftDestroy(g->plan);
-      g->plan = 0;
-      g->plan_batch = 0;
-      int r = gpu_capacity(g, g->count);
-      if (r != AAK_OK) return r;
+    g->packed = pack && g->length % 2 == 0;
+    if ((r = fft_plan(g, g->packed ? CUFFT_Z2Z : CUFFT_D2Z, g->count, &h)) != AAK_OK) return r;
+    for (int ch = 0; ch < 2; ++ch) {
+      cufftDoubleComplex *z = reinterpret_cast<cufftDoubleComplex *>(g->d_H[ch].ptr);
+      const cufftResult e = g->packed ? cufftExecZ2Z(h, z, z, CUFFT_FORWARD) : cufftExecD2Z(h, g->d_H[ch].ptr, z);
+      if (e != CUFFT_SUCCESS) return AAK_ERR_CUDA;
     }
-    if (cufftSetStream(g->plan, g->stream) != CUFFT_SUCCESS) return AAK_ERR_CUDA;
-    if (cufftExecD2Z(g->plan, g->d_H[0].ptr, reinterpret_cast<cufftDoubleComplex *>(g->d_H[0].ptr)) != CUFFT_SUCCESS ||
-        cufftExecD2Z(g->plan, g->d_H[1].ptr, reinterpret_cast<cufftDoubleComplex *>(g->d_H[1].ptr)) != CUFFT_SUCCESS)
-      return AAK_ERR_CUDA;
     g->spectral = true;
+    return AAK_OK;
+  }
+  if (g->packed && !pack) {
+    for (int ch = 0; ch < 2; ++ch) launch_unpack_rows(g->d_H[ch].ptr, g->row, g->count, g->stream);
+    g->packed = false;
+    return cuda_ok(cudaGetLastError());
   }
   return AAK_OK;
 }
@@ -2342,7 +2379,8 @@ int gpu_inner_products(aak_gpu *g) {
   a.ntemplates = g->count;
   a.partial = g->d_partial.ptr;
   a.out = g->d_out.ptr;
-  launch_inner_products(a, g->stream);
+  if (g->packed) launch_inner_products_packed(a, g->stream);
+  else launch_inner_products(a, g->stream);
   return cuda_ok(cudaGetLastError());
 }
 
@@ -2378,9 +2416,16 @@ int gpu_pipeline_ready(aak_gpu *g, int max_batch) {
   b->variant[1] = a->variant[1];
   if (!g->up_stream && (r = cuda_ok(cudaStreamCreateWithFlags(&g->up_stream, cudaStreamNonBlocking))) != AAK_OK)
     return r;
-  for (auto &row : g->pev)
-    for (auto &e : row)
-      if (!e && (r = cuda_ok(cudaEventCreate(&e))) != AAK_OK) return r;
+  auto event = [](cudaEvent_t &e) { return e ? AAK_OK : cuda_ok(cudaEventCreate(&e)); };
+  for (int p = 0; p < 2; ++p) {
+    for (auto &e : g->pev[p])
+      if ((r = event(e)) != AAK_OK) return r;
+    for (auto &e : g->uev[p])
+      if ((r = event(e)) != AAK_OK) return r;
+    for (auto &u : g->tev[p])
+      for (auto &e : u)
+        if ((r = event(e)) != AAK_OK) return r;
+  }
   if (g->stage_cap < max_batch) {
     if (g->h_stage) cudaFreeHost(g->h_stage);
     g->h_stage = nullptr;
@@ -2393,49 +2438,85 @@ int gpu_pipeline_ready(aak_gpu *g, int max_batch) {
   return AAK_OK;
 }
 
-// Chunk of B templates planned in C, result slot p: C's plan is uploaded on
-// up_stream (after the generation of the chunk two back, the last reader of
-// C's device buffers), then on the likelihood's stream the rows are
-// generated, transformed and reduced, and the results copied to slot p.
-int gpu_chunk_launch(aak_gpu *g, aak_ctx *C, int p, int B) {
-  cudaEvent_t *E = g->pev[p];
-  const bool r32 = g->precision == 2 && g->d_D32[0].ptr;
+// Plan and generate the B templates of a chunk into the rows, in units: each is planned into the context whose turn it
+// is (after the upload of the unit two back has read its plan arrays), uploaded
+// on up_stream (after the generation of that unit, the last reader of the
+// context's device buffers) and queued on the likelihood's stream, so that the
+// device starts on a chunk when its first unit is planned, not its last.  A
+// template's row does not depend on the others'.  A unit's planning costs no
+// more than its share of the chunk's where it fills the threads eight times
+// over (lane groups of four balance) or has at most three templates a thread
+// (each planned alone): 64 templates of 3.2e6 samples a chunk on 16 threads, units
+// of 48 31.6 ms for two chunks against 35.5 whole and 34.8 in units of 16; 256 of
+// 8e5, halves 51 ms against 56 whole and 69 in units of 16.  fe: the chunk's warm front end, done
+// ahead for the whole chunk, which then is one unit; between (optional): what
+// the host does after planning it and before its launch.  Adds the planning
+// time to *ms.
+int gpu_rows_launch(aak_gpu *g, const double *x, int B, int nthreads, int32_t *status, const WarmFrontEnd *fe, int p,
+                    bool r32, double *ms, const std::function<int()> &between = nullptr) {
   int r;
   if ((r = r32 ? gpu_capacity32(g, B) : gpu_capacity(g, B)) != AAK_OK) return r;
-  if ((r = cuda_ok(cudaStreamWaitEvent(g->up_stream, E[1], 0))) != AAK_OK) return r;
-  if ((r = upload(C, g->up_stream, false)) != AAK_OK) return r;
-  if ((r = cuda_ok(cudaEventRecord(E[0], g->up_stream))) != AAK_OK ||
-      (r = cuda_ok(cudaStreamWaitEvent(g->stream, E[0], 0))) != AAK_OK)
-    return r;
-  cudaEventRecord(E[2], g->stream);
-  if (r32) r = run_rows32(C, g->d_H32[0].ptr, g->d_H32[1].ptr, 1, g->stream);
-  else r = run(C, g->d_H[0].ptr, g->d_H[1].ptr, nullptr, nullptr, 0, g->precision == 0 ? 0 : 1, g->stream);
-  if (r != AAK_OK) return r;
-  cudaEventRecord(E[1], g->stream);
+  const int threads = nthreads > 0 ? nthreads : (int)std::max(1u, std::thread::hardware_concurrency());
+  const int size = (fe || B <= 2 * threads) ? B : (B >= 16 * threads) ? (B + 1) / 2 : std::max(3 * threads, (B + kUnitsMax - 1) / kUnitsMax);
+  g->units[p] = 0;
+  for (int k0 = 0; k0 < B; k0 += size) {
+    const int n = std::min(size, B - k0), q = (int)(g->unit++ & 1);
+    aak_ctx *C = q ? g->ctx2 : g->ctx;
+    double t = 0.0;
+    if ((r = cuda_ok(cudaEventSynchronize(g->uev[q][0]))) != AAK_OK ||
+        (r = gpu_plan_into(g, C, x + 14 * (int64_t)k0, n, nthreads, status ? status + k0 : nullptr, &t, fe)) != AAK_OK)
+      return r;
+    *ms += t;
+    if (between && (r = between()) != AAK_OK) return r;
+    if ((r = cuda_ok(cudaStreamWaitEvent(g->up_stream, g->uev[q][1], 0))) != AAK_OK ||
+        (r = upload(C, g->up_stream, false)) != AAK_OK ||
+        (r = cuda_ok(cudaEventRecord(g->uev[q][0], g->up_stream))) != AAK_OK ||
+        (r = cuda_ok(cudaStreamWaitEvent(g->stream, g->uev[q][0], 0))) != AAK_OK)
+      return r;
+    cudaEvent_t *T = g->tev[p][g->units[p]++];
+    const int64_t o = (int64_t)k0 * g->row;
+    cudaEventRecord(T[0], g->stream);
+    if (r32) r = run_rows32(C, g->d_H32[0].ptr + o, g->d_H32[1].ptr + o, 1, g->stream);
+    else
+      r = run(C, g->d_H[0].ptr + o, g->d_H[1].ptr + o, nullptr, nullptr, 0, g->precision == 0 ? 0 : 1, g->stream);
+    if (r != AAK_OK) return r;
+    cudaEventRecord(T[1], g->stream);
+    if ((r = cuda_ok(cudaEventRecord(g->uev[q][1], g->stream))) != AAK_OK) return r;
+  }
+  cudaEventRecord(g->pev[p][0], g->stream);
   g->count = B;
-  g->spectral = false;
+  g->spectral = g->packed = false;
   g->rows32 = r32;
-  if ((r = gpu_fft_rows(g)) != AAK_OK) return r;
-  cudaEventRecord(E[3], g->stream);
+  return AAK_OK;
+}
+
+// A chunk's device work after its rows: transform and reduction, the results
+// copied to slot p.
+int gpu_chunk_reduce(aak_gpu *g, int p, int B) {
+  cudaEvent_t *E = g->pev[p];
+  int r;
+  if ((r = gpu_fft_rows(g, true)) != AAK_OK) return r;
+  cudaEventRecord(E[1], g->stream);
   if ((r = gpu_inner_products(g)) != AAK_OK) return r;
-  cudaEventRecord(E[4], g->stream);
+  cudaEventRecord(E[2], g->stream);
   if ((r = cuda_ok(cudaMemcpyAsync(g->h_stage + 2 * (size_t)g->stage_cap * p, g->d_out.ptr,
                                    2 * (size_t)B * sizeof(double), cudaMemcpyDeviceToHost, g->stream))) != AAK_OK)
     return r;
-  return cuda_ok(cudaEventRecord(E[5], g->stream));
+  return cuda_ok(cudaEventRecord(E[3], g->stream));
 }
 
-// Wait for the chunk in slot p, copy its B results to out and add its device
-// times (generate, FFT, reduce) to ms[1..3].
-int gpu_chunk_collect(aak_gpu *g, int p, int B, double *out, double *ms) {
+// Wait for the chunk in slot p, copy its n results to out and add its device
+// times (generation kernels, transform, reduction) to ms[1..3].
+int gpu_chunk_collect(aak_gpu *g, int p, int64_t n, double *out, double *ms) {
   cudaEvent_t *E = g->pev[p];
-  const int r = cuda_ok(cudaEventSynchronize(E[5]));
+  const int r = cuda_ok(cudaEventSynchronize(E[3]));
   if (r != AAK_OK) return r;
-  std::memcpy(out, g->h_stage + 2 * (size_t)g->stage_cap * p, 2 * (size_t)B * sizeof(double));
+  std::memcpy(out, g->h_stage + 2 * (size_t)g->stage_cap * p, (size_t)n * sizeof(double));
   float f;
-  if (cudaEventElapsedTime(&f, E[2], E[1]) == cudaSuccess) ms[1] += f;
-  if (cudaEventElapsedTime(&f, E[1], E[3]) == cudaSuccess) ms[2] += f;
-  if (cudaEventElapsedTime(&f, E[3], E[4]) == cudaSuccess) ms[3] += f;
+  for (int u = 0; u < g->units[p]; ++u)
+    if (cudaEventElapsedTime(&f, g->tev[p][u][0], g->tev[p][u][1]) == cudaSuccess) ms[1] += f;
+  if (cudaEventElapsedTime(&f, E[0], E[1]) == cudaSuccess) ms[2] += f;
+  if (cudaEventElapsedTime(&f, E[1], E[2]) == cudaSuccess) ms[3] += f;
   cudaGetLastError();
   return AAK_OK;
 }
@@ -2468,7 +2549,7 @@ int gpu_fisher(aak_gpu *g, const double *x, int nd, double scale, int nthreads, 
   const int B = 2 * nd;
   int r = gpu_generate(g, x, B, nthreads, status, false);
   if (r != AAK_OK) return r;
-  if ((r = gpu_fft_rows(g)) != AAK_OK) return r;
+  if ((r = gpu_fft_rows(g, true)) != AAK_OK) return r;
   const int grid = fisher_grid(g->ctx->num_sms, g->nbins);
   const int64_t need = fisher_partial_doubles(nd, grid) + 2 * (int64_t)nd * nd;
   if ((r = g->d_fisher.reserve((size_t)need)) != AAK_OK) return r;
@@ -2482,6 +2563,7 @@ int gpu_fisher(aak_gpu *g, const double *x, int nd, double scale, int nthreads, 
   a.nbins = g->nbins;
   a.nd = nd;
   a.scale = scale;
+  a.packed = g->packed;
   a.partial = g->d_fisher.ptr;
   a.out = g->d_fisher.ptr + fisher_partial_doubles(nd, grid);
   launch_fisher_gram(a, g->ctx->num_sms, g->stream);
@@ -2499,28 +2581,13 @@ int gpu_fisher(aak_gpu *g, const double *x, int nd, double scale, int nthreads, 
   return device_status(g->ctx);
 }
 
-// The device half of one Fisher point planned in C, slot p: C's plan is
-// uploaded on up_stream (after the generation of the point two back, the
-// last reader of C's device buffers), then on the likelihood's stream the 2 nd
-// rows are generated, transformed and reduced to the Gram matrices, which are
-// copied to page-locked slot p.  Events as gpu_chunk_launch's.
-int gpu_fisher_point_launch(aak_gpu *g, aak_ctx *C, int p, int nd, double scale, int grid) {
+// One Fisher point's device work after its rows: transform and reduction to
+// the Gram matrices, which are copied to page-locked slot p.
+int gpu_fisher_reduce(aak_gpu *g, int p, int nd, double scale, int grid) {
   cudaEvent_t *E = g->pev[p];
   int r;
-  if ((r = cuda_ok(cudaStreamWaitEvent(g->up_stream, E[1], 0))) != AAK_OK) return r;
-  if ((r = upload(C, g->up_stream, false)) != AAK_OK) return r;
-  if ((r = cuda_ok(cudaEventRecord(E[0], g->up_stream))) != AAK_OK ||
-      (r = cuda_ok(cudaStreamWaitEvent(g->stream, E[0], 0))) != AAK_OK)
-    return r;
-  cudaEventRecord(E[2], g->stream);
-  if ((r = run(C, g->d_H[0].ptr, g->d_H[1].ptr, nullptr, nullptr, 0, g->precision == 0 ? 0 : 1, g->stream)) != AAK_OK)
-    return r;
+  if ((r = gpu_fft_rows(g, true)) != AAK_OK) return r;
   cudaEventRecord(E[1], g->stream);
-  g->count = 2 * nd;
-  g->spectral = false;
-  g->rows32 = false;
-  if ((r = gpu_fft_rows(g)) != AAK_OK) return r;
-  cudaEventRecord(E[3], g->stream);
   FisherArgs a;
   a.H[0] = g->d_H[0].ptr;
   a.H[1] = g->d_H[1].ptr;
@@ -2530,20 +2597,21 @@ int gpu_fisher_point_launch(aak_gpu *g, aak_ctx *C, int p, int nd, double scale,
   a.nbins = g->nbins;
   a.nd = nd;
   a.scale = scale;
+  a.packed = g->packed;
   a.partial = g->d_fisher.ptr;
   a.out = g->d_fisher.ptr + fisher_partial_doubles(nd, grid);
   launch_fisher_gram(a, g->ctx->num_sms, g->stream);
   if ((r = cuda_ok(cudaGetLastError())) != AAK_OK) return r;
-  cudaEventRecord(E[4], g->stream);
+  cudaEventRecord(E[2], g->stream);
   if ((r = cuda_ok(cudaMemcpyAsync(g->h_stage + 2 * (size_t)g->stage_cap * p, a.out, 2 * (size_t)nd * nd * sizeof(double),
                                    cudaMemcpyDeviceToHost, g->stream))) != AAK_OK)
     return r;
-  return cuda_ok(cudaEventRecord(E[5], g->stream));
+  return cuda_ok(cudaEventRecord(E[3], g->stream));
 }
 
-// Fisher matrices of npts points, pipelined as the likelihood batches are:
-// point k + 1 is planned on host threads into the other planning context while
-// the device generates, transforms and reduces point k.
+// Fisher matrices of npts points, pipelined as the likelihood batches are: the
+// next templates are planned on host threads while the device generates,
+// transforms and reduces those before them.
 int gpu_fisher_batch(aak_gpu *g, const double *x, int npts, int nd, double scale, int nthreads, double *gram,
                      int32_t *status) {
   if (npts < 1 || nd < 1 || nd > kFisherMaxDim || !x || !gram || !std::isfinite(scale)) return AAK_ERR_INVALID_PARAM;
@@ -2552,48 +2620,26 @@ int gpu_fisher_batch(aak_gpu *g, const double *x, int npts, int nd, double scale
   int r;
   // result slots of 2 nd^2 doubles (the page-locked stage holds two of 2 x stage_cap)
   if ((r = gpu_pipeline_ready(g, std::max(B, nd * nd))) != AAK_OK) return r;
-  if (g->plan_batch != B) {  // an exact-size transform plan of the rows, made once before the loop
-    if (g->plan) cufftDestroy(g->plan);
-    g->plan = 0;
-    g->plan_batch = 0;
-  }
   if ((r = gpu_capacity(g, B)) != AAK_OK) return r;
   const int grid = fisher_grid(g->ctx->num_sms, g->nbins);
   if ((r = g->d_fisher.reserve((size_t)(fisher_partial_doubles(nd, grid) + 2 * (int64_t)nd * nd))) != AAK_OK) return r;
-  aak_ctx *ctxs[2] = {g->ctx, g->ctx2};
   auto fail = [&](int e) {
     cudaStreamSynchronize(g->up_stream);
     cudaStreamSynchronize(g->stream);
     return e;
   };
-  auto collect = [&](int p, int k, double *tot) -> int {
-    cudaEvent_t *E = g->pev[p];
-    const int e = cuda_ok(cudaEventSynchronize(E[5]));
-    if (e != AAK_OK) return e;
-    std::memcpy(gram + 2 * (int64_t)nd * nd * k, g->h_stage + 2 * (size_t)g->stage_cap * p, 2 * (size_t)nd * nd * sizeof(double));
-    float f;
-    if (cudaEventElapsedTime(&f, E[2], E[1]) == cudaSuccess) tot[1] += f;
-    if (cudaEventElapsedTime(&f, E[1], E[3]) == cudaSuccess) tot[2] += f;
-    if (cudaEventElapsedTime(&f, E[3], E[4]) == cudaSuccess) tot[3] += f;
-    cudaGetLastError();
-    return AAK_OK;
-  };
-  double tot[4] = {0, 0, 0, 0}, ms = 0.0;
-  if ((r = gpu_plan_into(g, ctxs[0], x, B, nthreads, status, &ms)) != AAK_OK) return r;
-  tot[0] += ms;
+  const int64_t per = 2 * (int64_t)nd * nd;
+  double tot[4] = {0, 0, 0, 0};
   for (int c = 0; c < npts; ++c) {
     const int p = c & 1;
-    if ((r = gpu_fisher_point_launch(g, ctxs[p], p, nd, scale, grid)) != AAK_OK) return fail(r);
-    if (c + 1 < npts) {
-      const int64_t k1 = (int64_t)(c + 1) * B;
-      if ((r = cuda_ok(cudaEventSynchronize(g->pev[1 - p][0]))) != AAK_OK) return fail(r);
-      if ((r = gpu_plan_into(g, ctxs[1 - p], x + 14 * k1, B, nthreads, status ? status + k1 : nullptr, &ms)) != AAK_OK)
-        return fail(r);
-      tot[0] += ms;
-    }
-    if (c > 0 && (r = collect(1 - p, c - 1, tot)) != AAK_OK) return fail(r);
+    if (c > 1 && (r = gpu_chunk_collect(g, p, per, gram + per * (c - 2), tot)) != AAK_OK) return fail(r);
+    if ((r = gpu_rows_launch(g, x + 14 * (int64_t)c * B, B, nthreads, status ? status + (int64_t)c * B : nullptr, nullptr,
+                             p, false, &tot[0])) != AAK_OK ||
+        (r = gpu_fisher_reduce(g, p, nd, scale, grid)) != AAK_OK)
+      return fail(r);
   }
-  if ((r = collect((npts - 1) & 1, npts - 1, tot)) != AAK_OK) return fail(r);
+  for (int c = std::max(0, npts - 2); c < npts; ++c)
+    if ((r = gpu_chunk_collect(g, c & 1, per, gram + per * c, tot)) != AAK_OK) return fail(r);
   for (int q = 0; q < 4; ++q) g->ms[q] = tot[q];
   const int s1 = device_status(g->ctx), s2 = device_status(g->ctx2);
   return s1 != AAK_OK ? s1 : s2;
@@ -2649,12 +2695,12 @@ int aak_gpu_create(double T_fit, int32_t init_length, int32_t length, double ini
 
 void aak_gpu_destroy(aak_gpu *g) {
   if (!g) return;
+  while (!g->plans.empty()) drop_fft_plan(g, g->plans.size() - 1);  // they hold the stream
   if (g->stream) {
     cudaStreamSynchronize(g->stream);
     cudaStreamDestroy(g->stream);
   }
-  if (g->plan) cufftDestroy(g->plan);
-  if (g->plan32) cufftDestroy(g->plan32);
+  g->d_fft_work.release();
   for (int ch = 0; ch < 2; ++ch) {
     g->d_H32[ch].release();
     g->d_D32[ch].release();
@@ -2672,9 +2718,15 @@ void aak_gpu_destroy(aak_gpu *g) {
     cudaStreamSynchronize(g->up_stream);
     cudaStreamDestroy(g->up_stream);
   }
-  for (auto &row : g->pev)
-    for (auto &e : row)
+  for (int p = 0; p < 2; ++p) {
+    for (auto &e : g->pev[p])
       if (e) cudaEventDestroy(e);
+    for (auto &e : g->uev[p])
+      if (e) cudaEventDestroy(e);
+    for (auto &u : g->tev[p])
+      for (auto &e : u)
+        if (e) cudaEventDestroy(e);
+  }
   if (g->h_stage) cudaFreeHost(g->h_stage);
   aak_ctx_destroy(g->ctx2);
   aak_ctx_destroy(g->ctx);
@@ -2725,6 +2777,7 @@ int aak_gpu_get_waveform(aak_gpu *g, double *t, double *hI, double *hII) {
   int r;
   const size_t m = std::min(n, (size_t)g->row);
   if ((r = select_device(g->ctx->device)) != AAK_OK) return r;
+  if (g->packed && (r = gpu_fft_rows(g)) != AAK_OK) return r;  // a batch's packed rows: their half spectra
   if ((r = cuda_ok(cudaStreamSynchronize(g->stream))) != AAK_OK) return r;  // the template's generation
   double *dst[3] = {t, hI, hII};
   const double *src[3] = {g->d_t.ptr, g->d_H[0].ptr, g->d_H[1].ptr};
@@ -2754,17 +2807,15 @@ int aak_gpu_likelihood_batch(aak_gpu *g, const double *params, int32_t nsrc, int
   if (select_device(g->ctx->device) != AAK_OK) return AAK_ERR_CUDA;
   int r;
   if ((r = gpu_pipeline_ready(g, max_batch)) != AAK_OK) return r;
-  // Chunk c is planned into ctxs[c & 1]: while the device generates,
-  // transforms and reduces chunk c, the host plans chunk c + 1 into the other
-  // context (whose upload, of chunk c - 1, has finished reading its plan
-  // arrays) and then queues it, so that the device goes from one chunk to the
-  // next without waiting for the host; chunk c - 1's results are collected
-  // after that.  With a learned warm start, its prediction needs the device,
-  // which is busy with the persistent waveform kernel of the chunk in flight:
-  // the front end of chunk c + 2 (coarse inspirals, prediction, maps) is then
-  // done after chunk c + 1 is planned, so that its prediction runs between
-  // chunk c's kernels and the planning of a chunk never waits for the device.
-  aak_ctx *ctxs[2] = {g->ctx, g->ctx2};
+  // Each chunk is planned in units that the device starts on as they are
+  // planned (gpu_rows_launch); its transform and reduction follow the last
+  // one, while the host goes on to the next chunk's first unit.  A chunk's
+  // results are collected when the one two after it wants their slot.  With a
+  // learned warm start, its prediction needs the device, which is busy with the
+  // persistent waveform kernel of the chunk in flight: a chunk is then one unit,
+  // and the front end of the chunk after it (coarse inspirals, prediction, maps)
+  // is done once it is planned, before its launch, so that the prediction runs
+  // between the kernels of the chunk before and no planning waits for the device.
   const bool ahead = g->ctx->model != nullptr;
   WarmFrontEnd fe[3];
   const int32_t nch = (nsrc + max_batch - 1) / max_batch;
@@ -2774,7 +2825,6 @@ int aak_gpu_likelihood_batch(aak_gpu *g, const double *params, int32_t nsrc, int
     cudaStreamSynchronize(g->stream);
     return e;
   };
-  double ms = 0.0;
   // the warm front end of chunk c (ahead only), timed with the planning
   auto front = [&](int32_t c) {
     const auto t0 = std::chrono::steady_clock::now();
@@ -2785,29 +2835,22 @@ int aak_gpu_likelihood_batch(aak_gpu *g, const double *params, int32_t nsrc, int
     return e;
   };
   if (ahead && ((r = front(0)) != AAK_OK || (nch > 1 && (r = front(1)) != AAK_OK))) return r;
-  if ((r = gpu_plan_into(g, ctxs[0], params, chunk_size(0), nthreads, status, &ms, ahead ? &fe[0] : nullptr)) !=
-      AAK_OK)
-    return r;
-  tot[0] += ms;
+  const bool r32 = g->precision == 2 && g->d_D32[0].ptr;
+  auto collect = [&](int32_t c) {
+    return gpu_chunk_collect(g, c & 1, 2 * (int64_t)chunk_size(c), out + 2 * (int64_t)c * max_batch, tot);
+  };
   for (int32_t c = 0; c < nch; ++c) {
-    const int p = c & 1;
-    if ((r = gpu_chunk_launch(g, ctxs[p], p, chunk_size(c))) != AAK_OK) return fail(r);
-    if (c + 1 < nch) {
-      const int64_t k1 = (int64_t)(c + 1) * max_batch;
-      if ((r = cuda_ok(cudaEventSynchronize(g->pev[1 - p][0]))) != AAK_OK) return fail(r);
-      if ((r = gpu_plan_into(g, ctxs[1 - p], params + 14 * k1, chunk_size(c + 1), nthreads,
-                             status ? status + k1 : nullptr, &ms, ahead ? &fe[(c + 1) % 3] : nullptr)) != AAK_OK)
-        return fail(r);
-      tot[0] += ms;
-    }
-    if (ahead && c + 2 < nch && (r = front(c + 2)) != AAK_OK) return fail(r);
-    if (c > 0 && (r = gpu_chunk_collect(g, 1 - p, chunk_size(c - 1), out + 2 * (int64_t)(c - 1) * max_batch, tot)) !=
-                     AAK_OK)
+    const int64_t k = (int64_t)c * max_batch;
+    if (c > 1 && (r = collect(c - 2)) != AAK_OK) return fail(r);
+    std::function<int()> next_front;
+    if (ahead && c > 0 && c + 1 < nch) next_front = [&, c]() { return front(c + 1); };
+    if ((r = gpu_rows_launch(g, params + 14 * k, chunk_size(c), nthreads, status ? status + k : nullptr,
+                             ahead ? &fe[c % 3] : nullptr, c & 1, r32, &tot[0], next_front)) != AAK_OK ||
+        (r = gpu_chunk_reduce(g, c & 1, chunk_size(c))) != AAK_OK)
       return fail(r);
   }
-  if ((r = gpu_chunk_collect(g, (nch - 1) & 1, chunk_size(nch - 1), out + 2 * (int64_t)(nch - 1) * max_batch, tot)) !=
-      AAK_OK)
-    return fail(r);
+  for (int32_t c = std::max(0, nch - 2); c < nch; ++c)
+    if ((r = collect(c)) != AAK_OK) return fail(r);
   for (int q = 0; q < 4; ++q) g->ms[q] = tot[q];
   return AAK_OK;
 }

@@ -28,6 +28,14 @@ constexpr int kIpBlocksPerTemplate = 64;
 
 void launch_inner_products(const InnerProductArgs &a, cudaStream_t stream);
 
+// The same products from packed rows: for an even length N, the complex
+// transform of length M = N / 2 of the row's even and odd samples as real and
+// imaginary parts (nbins = M + 1 half-spectrum bins follow from its M values).
+void launch_inner_products_packed(const InnerProductArgs &a, cudaStream_t stream);
+
+// Packed rows to half spectra, in place (`rows` rows of row_doubles = 2 (M + 1) doubles).
+void launch_unpack_rows(double *H, int64_t row_doubles, int rows, cudaStream_t stream);
+
 // The same products from FP32 spectra (an FP32 R2C transform of FP32
 // template rows, row stride `row_floats` floats) and FP32 copies of the data
 // and weights.  Each thread accumulates its bins in FP32 with Kahan
@@ -63,6 +71,7 @@ struct FisherArgs {
   double scale;        // applied to each difference
   double *partial;     // fisher_partial_doubles(nd, num_sms) scratch
   double *out;         // 2 x nd x nd
+  bool packed = false; // the rows are packed transforms (launch_inner_products_packed)
 };
 int fisher_grid(int num_sms, int64_t nbins);
 inline int64_t fisher_partial_doubles(int nd, int grid) { return (int64_t)grid * nd * (nd + 1); }
