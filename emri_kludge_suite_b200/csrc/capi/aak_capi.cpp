@@ -13,6 +13,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <map>
 #include <memory>
 #include <string>
 #include <mutex>
@@ -594,6 +595,59 @@ int plan_sources(aak_ctx *ctx, const std::vector<aak_params> &Pv, const aak_mapp
     }
     return st;
   };
+  // Sources of one inspiral (the same masses, spin, orbit and span; the points
+  // of a Fisher matrix differ in it for 6 of 14 parameters, a sampler's
+  // extrinsic moves not at all) share their front end, where that saves a
+  // quarter of them: done once each, ahead of the tasks.
+  std::vector<int> rep;  // the source whose front end source s takes, empty: each its own
+  std::vector<MappedTrajectory> shared_map;
+  std::vector<int> shared_st;
+  if (fused && nsrc > 1 && !(ctx->evolve_device && dev >= 0)) {
+    struct Key {
+      double v[9];
+      int64_t length;
+      int32_t backint;
+      bool operator<(const Key &o) const {
+        const int c = std::memcmp(v, o.v, sizeof(v));
+        return c != 0 ? c < 0 : length != o.length ? length < o.length : backint < o.backint;
+      }
+    };
+    std::map<Key, int> seen;
+    std::vector<int> unique;
+    rep.resize(nsrc);
+    for (int s = 0; s < nsrc; ++s) {
+      const aak_params &q = Pv[s];
+      rep[s] = s;
+      if (validate(to_params(q)) != kOk) continue;  // reported by its own task
+      const Key k{{q.dt, q.p, q.T_fit, q.mu, q.M, q.s, q.e, q.iota, q.T}, q.length, q.backint};
+      const auto r = seen.emplace(k, s);
+      rep[s] = r.first->second;
+      if (r.second) unique.push_back(s);
+    }
+    if (4 * (int64_t)unique.size() > 3 * (int64_t)nsrc) {
+      rep.clear();
+    } else {
+      shared_map.resize(nsrc);
+      shared_st.assign(nsrc, kOk);
+      parallel_for((int64_t)unique.size(), nthreads, [&](int64_t i) {
+        on_device();
+        const int s = unique[i];
+        shared_st[s] = map_one(s, to_params(Pv[s]), &shared_map[s]);
+      });
+    }
+  }
+  auto front_end = [&](int s, const Params &Pp, MappedTrajectory *mt) {
+    if (rep.empty() || validate(Pp) != kOk) return map_one(s, Pp, mt);
+    const int u = rep[s];
+    if (shared_st[u] != kOk) return shared_st[u];
+    *mt = shared_map[u];
+    mt->Phi0 = initial_mean_anomaly(Pp.e, Pp.psi);
+    if (u != s) {
+      points += mt->steps;
+      iters += mt->newton_iterations;
+    }
+    return (int)kOk;
+  };
   if (ctx->evolve_device && dev >= 0) {
     // Planning in three passes around a device evolution: (a) front end, map
     // and the fit window of every source on host threads; (b) every source's
@@ -705,7 +759,7 @@ int plan_sources(aak_ctx *ctx, const std::vector<aak_params> &Pv, const aak_mapp
     for (int i = 0; i < n; ++i) {
       idx[i] = order[k + i];
       Pg[i] = to_params(Pv[idx[i]]);
-      st[i] = map_one(idx[i], Pg[i], &mg[i]);
+      st[i] = front_end(idx[i], Pg[i], &mg[i]);
       mp[i] = &mg[i];
     }
     finish_group(ctx, n, idx, Pg, mp, st, nm);

@@ -24,7 +24,7 @@ constexpr double kHmin = 1.0e-12;
 constexpr int kMaxCol = 8;
 }  // namespace
 
-KerrInspiral::KerrInspiral(double cosi0, double spin) : cosi0_(cosi0), a_(spin) {
+KerrInspiral::KerrInspiral(double cosi0, double spin) : cosi0_(cosi0), a_(spin), isco_ret_(kerr_isco_ret(spin)) {
   // The table depends on the spin alone: this thread's last one is reused
   // for the same spin (the templates of a likelihood batch share theirs).
   thread_local double last_spin = 2.0, last_table[2][2];
@@ -80,7 +80,7 @@ bool KerrInspiral::derivs(const double x[3], double dxdt[3]) const {
   KerrGeodesic g;
   g.set_constants(x[0], x[1], x[2], a_);
   KludgeFluxes f;
-  if (!f.set(x[0], x[1], g.E, g.Lz, g.Q, a_)) return false;
+  if (!f.set(x[0], x[1], g.E, g.Lz, g.Q, a_, isco_ret_)) return false;
   dxdt[0] = f.pdot;
   dxdt[1] = f.edot;
   dxdt[2] = f.cosidot;
@@ -115,13 +115,17 @@ bool KerrInspiral::midpoint(const double y[3], const double dydx[3], double h, i
 
 // Integrate y from x1 to x2.  1: done; 0: caller should shrink its step;
 // -1: the step size underflowed.
-int KerrInspiral::integrate(double y[3], double x1, double x2) const {
+int KerrInspiral::integrate(double y[3], double x1, double x2, const double *d0) const {
   double x = x1;
   double h = x2 - x1;
   double ycur[3] = {y[0], y[1], y[2]};
   for (int nstep = 0; nstep < 100000; ++nstep) {
     double dydx[3], yscal[3];
-    if (!derivs(ycur, dydx)) return 0;
+    if (nstep == 0 && d0) {
+      for (int i = 0; i < 3; ++i) dydx[i] = d0[i];
+    } else if (!derivs(ycur, dydx)) {
+      return 0;
+    }
     if ((x + h - x2) * (x + h - x1) > 0.0) h = x2 - x;
     for (int i = 0; i < 3; ++i) yscal[i] = std::fabs(ycur[i]) + std::fabs(dydx[i] * h) + 1e-30;
     // one extrapolated step of size h, shrinking h until accepted
@@ -175,10 +179,10 @@ int KerrInspiral::integrate(double y[3], double x1, double x2) const {
   return 0;
 }
 
-int KerrInspiral::take_step(double x[3], double t1, double &dt) const {
+int KerrInspiral::take_step(double x[3], double t1, double &dt, const double *d0) const {
   for (int guard = 0; guard < 64; ++guard) {
     double y[3] = {x[0], x[1], x[2]};
-    const int r = integrate(y, t1, t1 + dt);
+    const int r = integrate(y, t1, t1 + dt, d0);
     if (r == 1) {
       x[0] = y[0];
       x[1] = y[1];
@@ -211,6 +215,8 @@ int KerrInspiral::eccentric(double p0, double e0, double dt_start, int steps_max
     flag = kInspCircularised;
   }
   int i = 0;
+  double d[3] = {0, 0, 0};  // the rates at x, where have_d: they end one step and begin the next
+  bool have_d = false;
   while (!done) {
     out[i].t = t;
     out[i].p = x[0];
@@ -224,7 +230,7 @@ int KerrInspiral::eccentric(double p0, double e0, double dt_start, int steps_max
     }
     const double p_prev = x[0], e_prev = x[1];
     const double x_before[3] = {x[0], x[1], x[2]};
-    take_step(x, t, dt);
+    take_step(x, t, dt, have_d ? d : nullptr);
     if (dt * (x[0] - p_prev) > 0.) {
       done = true;
       flag = kInspInvalid;  // p growing: outside the validity of the flux kludge
@@ -233,8 +239,8 @@ int KerrInspiral::eccentric(double p0, double e0, double dt_start, int steps_max
       done = true;
       flag = kInspInvalid;
     }
-    double d[3] = {0, 0, 0};
-    derivs(x, d);
+    d[0] = d[1] = d[2] = 0.0;
+    have_d = derivs(x, d);
     while (x[0] + dt * d[0] < p_lso(x[2], x[1]) && std::fabs(dt) > 1.e-9) dt /= 2.;
     while (x[1] + dt * d[1] < 0 && std::fabs(dt) > 1.e-9) dt /= 2.;
     if (x[1] < 0.5 * ecc_ref) {

@@ -36,11 +36,13 @@ class KerrInspiral {
   bool derivs(const double x[3], double dxdt[3]) const;
 
  private:
-  int take_step(double x[3], double t1, double &dt) const;
-  int integrate(double y[3], double x1, double x2) const;
+  // d0 (optional): the rates at the starting state, if the caller has them
+  int take_step(double x[3], double t1, double &dt, const double *d0) const;
+  int integrate(double y[3], double x1, double x2, const double *d0) const;
   bool midpoint(const double y[3], const double dydx[3], double h, int nsub, double out[3]) const;
 
   double cosi0_, a_;
+  double isco_ret_;     // kerr_isco_ret(a_)
   double p_lso_[2][2];  // [cos-iota index: 0 -> +1, 1 -> -1][e index: 0 -> 0, 1 -> 0.9995]
 };
 

@@ -463,7 +463,7 @@ bool circ_fast(const CircFns &F, double c, double Elo, double Ehi, double &E_out
 }
 }  // namespace
 
-void CircularConstants::set(double r, double cosi, double a, bool bisection_only) {
+void CircularConstants::set(double r, double cosi, double a, bool bisection_only, double isco_ret) {
   const double Delta = r * r - 2. * r + a * a;
   const CircFns F{r, a, Delta};
   double En;
@@ -485,7 +485,7 @@ void CircularConstants::set(double r, double cosi, double a, bool bisection_only
     return;
   } else {
     const double Elo = kerr_e_eq_pro(r, a);
-    const double Ehi = (r >= kerr_isco_ret(a)) ? kerr_e_eq_ret(r, a) : 1.;
+    const double Ehi = (r >= (isco_ret > 0.0 ? isco_ret : kerr_isco_ret(a))) ? kerr_e_eq_ret(r, a) : 1.;
     if (bisection_only || !circ_fast(F, c, Elo, Ehi, En)) En = circ_bisect(F, c, Elo, Ehi);
   }
   E = En;
@@ -519,7 +519,7 @@ struct FluxFit {
 inline double fitc(const double *k, double sp) { return k[0] + (k[1] + k[2] / sp) / sp; }
 }  // namespace
 
-bool KludgeFluxes::set(double p, double e, double En, double L, double Qc, double a) {
+bool KludgeFluxes::set(double p, double e, double En, double L, double Qc, double a, double isco_ret) {
   if (e == 0.0) return false;
   const double ome = 1. - e, ope = 1. + e, ome2 = ome * ope;
   const double ra = p / ome, rp = p / ope;
@@ -530,7 +530,7 @@ bool KludgeFluxes::set(double p, double e, double En, double L, double Qc, doubl
   double Ecirc, Lzcirc, Qcirc, Lovercosicirc;
   if (a != 0.0) {
     CircularConstants cc;
-    cc.set(p, cosi, a);
+    cc.set(p, cosi, a, false, isco_ret);
     Ecirc = cc.E;
     Lzcirc = cc.Lz;
     Qcirc = cc.Q;
@@ -543,6 +543,8 @@ bool KludgeFluxes::set(double p, double e, double En, double L, double Qc, doubl
   }
   (void)Qcirc;
   const double sp = std::sqrt(p), p15 = p * sp, csq = cosi * cosi;
+  // each power once (a call of pow is not merged with its twin: it may set errno)
+  const double pow15 = std::pow(p, 1.5), pow35 = std::pow(p, 3.5), ome15 = std::pow(ome2, 1.5);
   const double e2 = e * e;
   const double a2 = a * a;
   const auto &C = FluxFit::c;
@@ -550,7 +552,7 @@ bool KludgeFluxes::set(double p, double e, double En, double L, double Qc, doubl
   // ---- Lz flux (GKR::Lzdot_GG)
   double Ldotcirc, Lzd;
   {
-    const double pref = -6.4 * std::pow(ome2, 1.5) / std::pow(p, 3.5);
+    const double pref = -6.4 * ome15 / pow35;
     const double term1 = 0.875 * e2;
     const double term2 = e2 * (63. / 8. + e2 * 95. / 64);
     const double term3 = e2 * (91. / 4. + e2 * 461. / 64.);
@@ -568,7 +570,7 @@ bool KludgeFluxes::set(double p, double e, double En, double L, double Qc, doubl
                        csq * csq * a2 * a * (fitc(C[7], sp) + cosi * a * fitc(C[8], sp)) + corr;
     const double circbit = cosi + a / p15 * (61. / 24. - csq * 61. / 8.) - cosi * 1247. / (336. * p) + 4. * kPi * cosi / p15 -
                            44711. * cosi / (9072. * p * p) + a2 * cosi * (-57. / 16. + 45. * csq / 8.) / (p * p) + hof / (p * p * sp);
-    Ldotcirc = -6.4 * circbit / std::pow(p, 3.5);
+    Ldotcirc = -6.4 * circbit / pow35;
     Lzd = pref * (cosi * term1 + a / p15 * (term2 - csq * term3) - cosi * term4 / p + kPi * term5 * cosi / p15 - term6 * cosi / (p * p) +
                   a2 * term7 * cosi / (p * p) + circbit);
   }
@@ -585,33 +587,33 @@ bool KludgeFluxes::set(double p, double e, double En, double L, double Qc, doubl
                        cosi * a * (fitc(C[3], sp) + a2 * fitc(C[4], sp)) +
                        csq * a2 * (fitc(C[5], sp) + a2 * fitc(C[6], sp)) +
                        csq * cosi * a2 * a * (fitc(C[7], sp) + cosi * a * fitc(C[8], sp)) + corr;
-    double circ = 1. - a / std::pow(p, 1.5) * (cosi * 61. / 8.) - 1247. / (336. * p) + 4. * kPi / std::pow(p, 1.5) -
+    double circ = 1. - a / pow15 * (cosi * 61. / 8.) - 1247. / (336. * p) + 4. * kPi / pow15 -
                   44711. / (9072. * p * p) + a2 * (-57. / 16. + 45. * csq / 8.) / (p * p) + hof / (p * p * sp);
     circ -= a2 * (FluxFit::ic3[0] + FluxFit::ic3[1] / p + FluxFit::ic3[2] / (p * sp) +
                   a * cosi * (FluxFit::ic4[0] / sp + FluxFit::ic4[1] / p + FluxFit::ic4[2] / (p * sp)) + idtc) /
             (p * p);
-    Qdotcirc = -12.8 * Lovercosicirc * sinsq * circ / std::pow(p, 3.5);
+    Qdotcirc = -12.8 * Lovercosicirc * sinsq * circ / pow35;
     Qd = -12.8 * Lovercosi * sinsq * (1. - e2) * std::sqrt(1. - e2) *
          (circ + 7. * e2 / 8. - (e2 * 425. / 336.) / p + kPi * (97. * e2 / 8.) / (p * sp) - (302893. * e2 / 6048.) / (p * p) -
           a * cosi * e2 * (91. / 4. + 461. * e2 / 64.) / (p * sp) + a2 * (95. * e2 / 16.) / (p * p)) /
-         std::pow(p, 3.5);
+         pow35;
   }
   // ---- E flux (GKR::Edot_GG)
   double Ed;
   {
-    const double pref = -6.4 * std::pow(ome2, 1.5) / std::pow(p, 5.);
+    const double pref = -6.4 * ome15 / std::pow(p, 5.);
     const double term1 = e2 * (73. / 24. + e2 * 37. / 96.);
     const double term2 = e2 * (823. / 24. + e2 * (949. / 32. + e2 * 491. / 192.));
     const double term3 = 9181. * e2 / 672.;
     const double term4 = 1375. * e2 / 48.;
     const double term5 = 172157 * e2 / 2592.;
     const double term6 = 359. * e2 / 32.;
-    const double fact = std::pow(ome2, 1.5);
+    const double fact = ome15;
     const double den = 4. * a * p * (Lzcirc - a * Ecirc) - 2. * p * p * Ecirc * (p * p + a2);
     const double dEdLz = (2. * ((p * p - 2. * p) * Lzcirc + 2. * a * p * Ecirc)) / den;
     const double dEdQ = (-2. * p + p * p + a2) / den;
     const double circbit = -(dEdLz * Ldotcirc + dEdQ * Qdotcirc);
-    Ed = pref * (term1 - a * cosi * term2 / std::pow(p, 1.5) - term3 / p + kPi * term4 / std::pow(p, 1.5) - term5 / (p * p) +
+    Ed = pref * (term1 - a * cosi * term2 / pow15 - term3 / p + kPi * term4 / pow15 - term5 / (p * p) +
                  a2 * term6 / (p * p)) +
          fact * circbit;
   }

@@ -50,8 +50,9 @@ struct KerrGeodesic {
 struct CircularConstants {
   double E = 0, Lz = 0, Q = 0, L_over_cosi = 0;
   // bisection_only: run every bisection step as written (the check of the
-  // fast path, which must give the same bits)
-  void set(double r, double cosi, double a, bool bisection_only = false);
+  // fast path, which must give the same bits).  isco_ret: kerr_isco_ret(a), for
+  // callers that hold it (three cube roots); 0: computed here.
+  void set(double r, double cosi, double a, bool bisection_only = false, double isco_ret = 0.0);
 };
 
 // Radiation-reaction rates dp/dt, de/dt, d(cos iota)/dt in radiation-reaction
@@ -60,7 +61,7 @@ struct KludgeFluxes {
   double pdot = 0, edot = 0, cosidot = 0;
   double Edot = 0, Lzdot = 0, Qdot = 0;
   // Returns false for e == 0 (the reference's circular branch is not on the AAK path).
-  bool set(double p, double e, double E, double Lz, double Q, double a);
+  bool set(double p, double e, double E, double Lz, double Q, double a, double isco_ret = 0.0);
 };
 
 // Sorted (ascending real part) roots of sum_{k=0}^{4} c[k] r^k by Laguerre's
