@@ -85,8 +85,8 @@ struct aak_ctx {
   std::vector<int64_t> queue_step;
   int32_t large_steps = 0;  // index in queue_step of the second class
   std::vector<int64_t> kofs;       // nsrc + 1 prefix of knots (the sources' knots stay in their plans)
-  std::vector<int64_t> spl_blk;    // nsrc + 1 prefix of the device spline solve's blocks
-  int spl_len = kSplineBlockShort; // knots per block of the device spline solve
+  std::vector<int64_t> spl_blk;    // nsrc + 1 prefix of the device spline solve's blocks: FP64, then split
+  bool spl_split = false;          // the coefficients on the device, and those the next upload makes: the split solve's
   bool want_pinned = true;         // plans' knot arrays in page-locked memory
   std::vector<int32_t> bessel;
   int64_t total_samples = 0, total_tiles = 0, total_knots = 0;
@@ -250,10 +250,12 @@ int pack(aak_ctx *ctx, const std::vector<aak_params> &P, int nthreads) {
     kofs[s + 1] = kofs[s] + (ok ? (int64_t)ctx->plans[s].knot_t.size() : 0);
     bofs[s + 1] = bofs[s] + (ok ? ctx->plans[s].nmodes : 0);
   }
-  ctx->spl_len = spline_block(knots);
-  ctx->spl_blk.assign(n + 1, 0);
-  for (int s = 0; s < n; ++s)
-    ctx->spl_blk[s + 1] = ctx->spl_blk[s] + (ctx->status[s] == AAK_OK ? spline_blocks((int)ctx->plans[s].knot_t.size(), ctx->spl_len) : 0);
+  ctx->spl_blk.assign(2 * (n + 1), 0);
+  for (int k = 0; k < 2; ++k) {
+    int64_t *blk = ctx->spl_blk.data() + k * (n + 1);
+    for (int s = 0; s < n; ++s)
+      blk[s + 1] = blk[s] + (ctx->status[s] == AAK_OK ? spline_blocks((int)ctx->plans[s].knot_t.size(), k != 0) : 0);
+  }
   ctx->tile_pairs.assign(2 * (size_t)n, 0);
   for (int s = 0; s < n; ++s) ctx->tile_pairs[2 * s + 1] = ctx->tile_start[s + 1] - ctx->tile_start[s];
   parallel_for(n, nthreads, [&](int64_t s64) {
@@ -783,6 +785,18 @@ int plan_common(aak_ctx *ctx, const aak_params *P, const aak_mapped *maps, int32
   return pack(ctx, Pv, nthreads);
 }
 
+// The spline coefficients of every source, by the FP64 or the split solve.
+void solve_knots(aak_ctx *ctx, bool split, cudaStream_t st) {
+  const int64_t o = split ? ctx->nsrc + 1 : 0;
+  launch_spline_coeffs(ctx->d_src.ptr, ctx->nsrc, ctx->d_spl_blk.ptr + o, ctx->spl_blk[o + ctx->nsrc], split,
+                       ctx->d_knot_t.ptr, ctx->d_knot_y.ptr, ctx->d_knot_c.ptr, st);
+  ctx->spl_split = split;
+}
+// Before a launch in `precision`: its own solve, if the upload's (that of the last launch before it) was the other one.
+void need_knots(aak_ctx *ctx, int precision, cudaStream_t st) {
+  if (ctx->spl_split != (precision == 1)) solve_knots(ctx, precision == 1, st);
+}
+
 // wait_pinned: finish the copies from page-locked plan arrays before
 // returning (callers whose next plan may refill those arrays); a caller that
 // keeps the plans untouched until it synchronises the stream passes false.
@@ -830,8 +844,7 @@ int upload(aak_ctx *ctx, cudaStream_t st, bool wait_pinned = true) {
   // the tiles' knot windows and the work queue, and the spline coefficients of every source, made on the device
   launch_tile_layout(ctx->d_src.ptr, n, ctx->d_tile_start.ptr, ctx->total_tiles, ctx->d_knot_t.ptr, ctx->d_tile_knot.ptr,
                      ctx->d_queue.ptr, ctx->d_queue_rank.ptr, ctx->d_queue_step.ptr, ctx->large_steps, st);
-  launch_spline_coeffs(ctx->d_src.ptr, n, ctx->d_spl_blk.ptr, ctx->spl_blk[n], ctx->spl_len, ctx->d_knot_t.ptr, ctx->d_knot_y.ptr,
-                       ctx->d_knot_c.ptr, st);
+  solve_knots(ctx, ctx->spl_split, st);
   if ((r = cuda_ok(cudaGetLastError())) != AAK_OK) return r;
   // copies from page-locked memory run asynchronously: finish them before the
   // host arrays can be refilled by the next plan
@@ -906,6 +919,7 @@ int run(aak_ctx *ctx, double *hI, double *hII, double *t, double *traj, int64_t 
   if (!traj && (r = tile_tables(ctx, precision, bv)) != AAK_OK) return r;
   if (ctx->profile && !ctx->ev[0])
     for (auto &e : ctx->ev) cudaEventCreate(&e);
+  need_knots(ctx, precision, st);
   launch_dense(bv, ctx->num_sms, st, ctx->profile ? ctx->ev : nullptr, precision, &ctx->side);
   ctx->last_launches = bv.tile_prep ? dense_launches(ctx, precision) : 1;
   return cuda_ok(cudaGetLastError());
@@ -921,6 +935,7 @@ int run_rows32(aak_ctx *ctx, float *hI32, float *hII32, int precision, cudaStrea
   bv.hII_f32 = hII32;
   bv.variant = ctx->variant[precision];
   if ((r = tile_tables(ctx, precision, bv)) != AAK_OK) return r;
+  need_knots(ctx, precision, st);
   launch_dense(bv, ctx->num_sms, st, nullptr, precision);
   ctx->last_launches = 3;
   return cuda_ok(cudaGetLastError());
@@ -953,8 +968,7 @@ int run_graph(aak_ctx *ctx, double *hI, double *hII, int precision, cudaStream_t
     // the whole dense stage: natural-spline solve of every source's knots
     // (idempotent: the same knots give the same coefficients), then the clears
     // and the waveform kernel
-    launch_spline_coeffs(ctx->d_src.ptr, ctx->nsrc, ctx->d_spl_blk.ptr, ctx->spl_blk[ctx->nsrc], ctx->spl_len, ctx->d_knot_t.ptr,
-                         ctx->d_knot_y.ptr, ctx->d_knot_c.ptr, ctx->cap_stream);
+    solve_knots(ctx, precision == 1, ctx->cap_stream);
     launch_dense(bv, ctx->num_sms, ctx->cap_stream, nullptr, precision, &ctx->side);
     const cudaError_t launch_err = cudaGetLastError();
     cudaGraph_t g = nullptr;
@@ -974,6 +988,7 @@ int run_graph(aak_ctx *ctx, double *hI, double *hII, int precision, cudaStream_t
     ctx->g_gen = ctx->upload_gen;
     ctx->g_variant = ctx->variant[precision];
   }
+  ctx->spl_split = precision == 1;
   ctx->last_launches = 1 + dense_launches(ctx, precision);  // with the spline solve
   return cuda_ok(cudaGraphLaunch(ctx->gexec, st));
 }
@@ -1024,6 +1039,7 @@ int run_phase(aak_ctx *ctx, double *out, int64_t stride, cudaStream_t st) {
   if ((r = tile_segments(ctx, bv)) != AAK_OK) return r;
   if (ctx->profile && !ctx->ev[0])
     for (auto &e : ctx->ev) cudaEventCreate(&e);
+  need_knots(ctx, 0, st);
   launch_phase(bv, ctx->num_sms, st, ctx->profile ? ctx->ev : nullptr, &ctx->side);
   // small sources: tile parameters, phase pass, freeze; the others: segments, carries, phase pass
   ctx->last_launches = (ctx->small_tiles > 0 ? 3 : 0) + (ctx->small_tiles < ctx->total_tiles ? 3 : 0);
@@ -1065,6 +1081,7 @@ int run_plain(aak_ctx *ctx, double *hI, double *hII, double *traj, int64_t traj_
     v.device_status = reinterpret_cast<unsigned int *>(ctx->d_counter.ptr + 1);
     v.trajectory_only = 1;
     v.max_nmodes = ctx->max_nmodes;
+    need_knots(ctx, 0, st);
     launch_dense(v, ctx->num_sms, st, nullptr, 0);
     launch_plain_waveform(ctx->d_src.ptr, s, d.vlength, traj, traj_stride, hI, hII, st);
     launches += 2;
@@ -1313,6 +1330,7 @@ int tdi_batch(aak_ctx *ctx, const aak_params *P, int32_t nsrc, int32_t nthreads,
   bv.phase_out = grid;
   bv.phase_stride = N;
   bv.trajectory_only = 1;
+  need_knots(ctx, 0, 0);
   launch_tdi_grid(bv, ctx->num_sms, 0, nullptr);
   if ((r = cuda_ok(cudaMemcpyAsync(ctx->d_tdi.ptr, td.data(), nsrc * sizeof(TdiDesc), cudaMemcpyHostToDevice, 0))) ||
       (r = cuda_ok(cudaMemcpyAsync(ctx->d_tdi_work.ptr, work.data(), (nsrc + 1) * sizeof(int64_t),
@@ -1721,8 +1739,10 @@ int aak_batch_run_noalloc(aak_ctx *ctx, void *d_plan, int64_t plan_bytes, int64_
   launch_tile_layout(reinterpret_cast<const SourceDesc *>(base), ctx->nsrc, reinterpret_cast<const int64_t *>(base + o_ts),
                      ctx->total_tiles, reinterpret_cast<const double *>(base + o_kt),
                      reinterpret_cast<int32_t *>(base + o_tk), nullptr, nullptr, nullptr, 0, st);
-  launch_spline_coeffs(reinterpret_cast<const SourceDesc *>(base), ctx->nsrc, reinterpret_cast<const int64_t *>(base + o_sb),
-                       ctx->spl_blk[ctx->nsrc], ctx->spl_len, reinterpret_cast<const double *>(base + o_kt),
+  const bool split = ctx->precision == 1;
+  const int64_t sb = split ? ctx->nsrc + 1 : 0;
+  launch_spline_coeffs(reinterpret_cast<const SourceDesc *>(base), ctx->nsrc, reinterpret_cast<const int64_t *>(base + o_sb) + sb,
+                       ctx->spl_blk[sb + ctx->nsrc], split, reinterpret_cast<const double *>(base + o_kt),
                        reinterpret_cast<const double4 *>(base + o_ky), reinterpret_cast<double4 *>(base + o_kc), st);
   if ((r = cuda_ok(cudaGetLastError())) != AAK_OK) return r;
   if (ctx->want_pinned && (r = cuda_ok(cudaStreamSynchronize(st))) != AAK_OK) return r;  // host arrays reusable on return
@@ -1871,6 +1891,7 @@ int aak_ctx_autotune(aak_ctx *ctx, double *d_hI, double *d_hII, int32_t precisio
     ms[v] = 0.0f;
     for (int rep = 0; rep < 3 && r == AAK_OK; ++rep) {  // one warm-up, then the faster of two
       cudaEventRecord(e0, st);
+      need_knots(ctx, precision, st);
       launch_dense(bv, ctx->num_sms, st, nullptr, precision);
       cudaEventRecord(e1, st);
       if ((r = cuda_ok(cudaEventSynchronize(e1))) != AAK_OK) break;

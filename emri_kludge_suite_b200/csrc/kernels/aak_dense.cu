@@ -134,8 +134,9 @@ __device__ __forceinline__ Traj4 spline4w(const BatchView &bv, const SourceDesc 
 }
 
 // Knots per unit time of the window and, for a staged window, the piece
-// coefficients (the knots are in shared memory and visible to every thread).
-__device__ __forceinline__ void finish_window(const BatchView &bv, const SourceDesc &d, KnotWin &w) {
+// coefficients (the knots are in shared memory and visible to every thread;
+// the caller's barrier publishes the coefficients).
+__device__ __forceinline__ void window_pieces(const BatchView &bv, const SourceDesc &d, KnotWin &w) {
   if (!w.staged) {
     const double *kt = bv.knot_t + d.knot_offset;
     const double span = kt[w.k0 + w.n - 1] - kt[w.k0];
@@ -155,8 +156,11 @@ __device__ __forceinline__ void finish_window(const BatchView &bv, const SourceD
       w.b[k] = b;
       w.d[k] = d;
     }
-    __syncthreads();
   }
+}
+__device__ __forceinline__ void finish_window(const BatchView &bv, const SourceDesc &d, KnotWin &w) {
+  window_pieces(bv, d, w);
+  if (w.staged) __syncthreads();
 }
 
 // Stage the knots of tile g (bracket precomputed on the host, tile_knot).
@@ -1432,7 +1436,8 @@ template <bool kSplit, int kMode = 0, bool kPre = false, int kJointT = 0, int kM
 __global__ void __launch_bounds__(kTileThreads, kMinB) k_waveform(BatchView bv) {
   constexpr bool kPhase = kMode != 0, kTdi = kMode == 2;
   static_assert(!kPre || kMode != 2, "the pre-pass serves the waveform and phase modes");
-  static_assert(!kCarry || (kPre && !kSplit && kMode != 2), "carries from the segments serve FP64 batches");
+  static_assert(!kCarry || (kPre && kMode != 2), "carries from the segments serve FP64 batches");
+  static_assert(!kPre || !kSplit, "split batches: k_wave_split");
   extern __shared__ double s_dyn[];  // [kDynVals][kTileSamples]
   __shared__ double red[2][3][kTileThreads / 32];  // warp totals of the forward and backward scans
   __shared__ long long s_tile;
@@ -1560,7 +1565,6 @@ __global__ void __launch_bounds__(kTileThreads, kMinB) k_waveform(BatchView bv) 
     }
     KnotWin w{s_wt, s_wy, s_wc, s_wb, s_wd, 0, 0, 0};
     if constexpr (kPre) {
-      using TT = typename std::conditional<kSplit, float, double>::type;
       if (tid == kTileThreads - 1) make_geom(*dp, s_geom);
       const bool ok = mbar_wait_bounded(&s_mbar[0], ph0);
       ph0 ^= 1u;
@@ -1572,8 +1576,7 @@ __global__ void __launch_bounds__(kTileThreads, kMinB) k_waveform(BatchView bv) 
         const bool tab = !kPhase && s_prep.K > 0 && nm <= kTabModes;
         if (tab) {
           fence_proxy_async_smem();
-          // FP64: one row per harmonic; FP32: one row per pair of harmonics
-          const uint32_t b1 = (uint32_t)(kSplit ? (nm + 1) >> 1 : nm) * (uint32_t)s_prep.stride * (uint32_t)sizeof(TT);
+          const uint32_t b1 = (uint32_t)nm * (uint32_t)s_prep.stride * (uint32_t)sizeof(double);  // a row a harmonic
           mbar_arrive_expect_tx(&s_mbar[1], b1);
           bulk_copy_g2s(tabD, static_cast<const unsigned char *>(bv.tile_tab) + g * bv.tab_slot, b1, &s_mbar[1]);
         }
@@ -2071,6 +2074,8 @@ __global__ void __launch_bounds__(kTileThreads, kMinB) k_waveform(BatchView bv) 
   }
 }
 
+#include "aak_split.cuh"
+
 // ------------------------------------------------------------------ plain FP64 per-source path
 // One thread per sample, everything per harmonic, as the reference's CUDA
 // port evaluates it (src/cuda/kernel.cu:374-555); the response, orientation
@@ -2243,25 +2248,26 @@ __global__ void __launch_bounds__(128) k_spline_coeffs(const SourceDesc *src, in
   }
 }
 
-// The same solve with four lanes a block, one per component, and blocks of
-// kSplineBlockShort.  One thread per 256-knot block leaves a batch of a few
-// sources waiting for a serial chain of 336 steps, each with two divisions and
-// a round trip to memory on it.  Here a step's chain is one division (each
-// lane repeats the factorisation, which depends on the knot times alone; the
-// intervals' reciprocals leave the chain, one lane dividing for each of the
-// next four), the knots are read kAhead steps before they are used, and the
-// factors wait in shared memory.  Every unknown takes the operations of the
-// long-block solve in its order.  Bound by the latency of the chain: 1e5 knots
-// 320 -> 10 us; block lengths of 32 to 96 differ by less than 10 %.
+// The same solve with four lanes a block, one per component.  A step's chain is one division
+// (each lane repeats the factorisation, which depends on the knot times alone;
+// the intervals' reciprocals leave the chain, one lane dividing for each of the
+// next four) and the knots are read kAhead steps before they are used.  The
+// factors wait in shared memory; the right-hand sides of the block's own
+// unknowns wait in c itself, so that a CTA's 16 KB leave 13 of them on an SM
+// (all in shared memory: 7).  Bound by the latency of the chain and by its
+// instructions (43 % of the issue slots, 1.2 TB/s of memory).  Block lengths,
+// 5e6 / 12e6 / 46e6 knots: 48 0.53 / 1.19 / 4.66 ms, 64 0.45 / 1.03 / 3.99, 96
+// 0.45 / 1.01 / 3.85, 128 0.49 / 1.07 / 4.08 (one thread a block of 256 knots:
+// 0.54 / 1.03 / 3.98, and 0.32 ms however few the knots; here 1e5 take 0.01).
 constexpr int kQuadThreads = 32;
 constexpr int kQuadBlocks = kQuadThreads / 4;  // knot blocks of one CTA
-constexpr int kQuadKept = kSplineBlockShort + kSplineHalo;
+constexpr int kQuadKept = kSplineBlock + kSplineHalo;
 __global__ void __launch_bounds__(kQuadThreads) k_spline_coeffs_quad(const SourceDesc *src, int nsrc,
                                                                      const int64_t *blk_start, int64_t total_blocks,
                                                                      const double *knot_t, const double4 *knot_y,
                                                                      double4 *knot_c) {
   __shared__ double s_cp[kQuadKept][kQuadBlocks];
-  __shared__ double s_dp[kQuadKept][kQuadThreads];
+  __shared__ double s_dp[kSplineHalo][kQuadThreads];  // right-hand sides of the halo; the block's own: in c
   constexpr int kAhead = 4;
   const int qd = threadIdx.x >> 2, comp = threadIdx.x & 3;
   const int64_t g = (int64_t)blockIdx.x * kQuadBlocks + qd;
@@ -2278,7 +2284,7 @@ __global__ void __launch_bounds__(kQuadThreads) k_spline_coeffs_quad(const Sourc
     return;
   }
   const int b = (int)(g - blk_start[s]);
-  const int a = 1 + b * kSplineBlockShort, e = min(a + kSplineBlockShort, n - 1);
+  const int a = 1 + b * kSplineBlock, e = min(a + kSplineBlock, n - 1);
   if (a == 1) c[0] = 0.0;
   if (e == n - 1) c[4 * (int64_t)(n - 1)] = 0.0;
   const int wa = max(1, a - kSplineHalo), wb = min(n - 1, e + kSplineHalo);
@@ -2318,7 +2324,8 @@ __global__ void __launch_bounds__(kQuadThreads) k_spline_coeffs_quad(const Sourc
       const double dd = (3.0 * ((y2 - y1) * inv_h1 - (y1 - y0) * inv_h0) - h0 * dprev) * inv;
       if (i >= a) {
         if (comp == 0) s_cp[i - a][qd] = cc;
-        s_dp[i - a][threadIdx.x] = dd;
+        if (i < e) c[4 * (int64_t)i] = dd;
+        else s_dp[i - e][threadIdx.x] = dd;
       }
       cprev = cc;
       dprev = dd;
@@ -2330,26 +2337,43 @@ __global__ void __launch_bounds__(kQuadThreads) k_spline_coeffs_quad(const Sourc
     }
   }
   __syncwarp(quad);  // lane 0's factors
-  double v = s_dp[wb - 1 - a][threadIdx.x];  // c at wb - 1 (its neighbour beyond the window taken as 0)
-  if (wb - 1 < e) c[4 * (int64_t)(wb - 1)] = v;
-  for (int i = wb - 2; i >= a; --i) {
-    v = s_dp[i - a][threadIdx.x] - s_cp[i - a][qd] * v;
-    if (i < e) c[4 * (int64_t)i] = v;
+  // back from the widened window's end (its neighbour beyond taken as 0): the halo, then the block's own unknowns
+  double v = 0.0;
+  int i = wb - 1;
+  if (i >= e) {
+    v = s_dp[i - e][threadIdx.x];
+    for (--i; i >= e; --i) v = s_dp[i - e][threadIdx.x] - s_cp[i - a][qd] * v;
+  } else {
+    v = dprev;
+    c[4 * (int64_t)i--] = v;
+  }
+  double qn[kAhead];  // unknowns i .. i - kAhead + 1
+#pragma unroll
+  for (int k = 0; k < kAhead; ++k) qn[k] = c[4 * (int64_t)max(i - k, a)];
+  for (; i >= a; i -= kAhead) {
+    double qc[kAhead];
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) {
+      qc[k] = qn[k];
+      qn[k] = c[4 * (int64_t)max(i - kAhead - k, a)];
+    }
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) {
+      if (i - k < a) break;
+      v = qc[k] - s_cp[i - k - a][qd] * v;
+      c[4 * (int64_t)(i - k)] = v;
+    }
   }
 }
 }  // namespace
 
-void launch_spline_coeffs(const SourceDesc *src, int nsrc, const int64_t *blk_start, int64_t total_blocks, int block,
+void launch_spline_coeffs(const SourceDesc *src, int nsrc, const int64_t *blk_start, int64_t total_blocks, bool split,
                           const double *knot_t, const double4 *knot_y, double4 *knot_c, cudaStream_t stream) {
   if (total_blocks <= 0) return;
-  if (block == kSplineBlockShort) {
-    k_spline_coeffs_quad<<<(unsigned)((total_blocks + kQuadBlocks - 1) / kQuadBlocks), kQuadThreads, 0, stream>>>(
-        src, nsrc, blk_start, total_blocks, knot_t, knot_y, knot_c);
-    return;
-  }
-  const int threads = 128;
-  k_spline_coeffs<<<(unsigned)((total_blocks + threads - 1) / threads), threads, 0, stream>>>(
-      src, nsrc, blk_start, total_blocks, knot_t, knot_y, knot_c);
+  const int per = split ? 128 : kQuadBlocks;  // blocks a CTA
+  const unsigned grid = (unsigned)((total_blocks + per - 1) / per);
+  if (split) k_spline_coeffs<<<grid, per, 0, stream>>>(src, nsrc, blk_start, total_blocks, knot_t, knot_y, knot_c);
+  else k_spline_coeffs_quad<<<grid, kQuadThreads, 0, stream>>>(src, nsrc, blk_start, total_blocks, knot_t, knot_y, knot_c);
 }
 
 namespace {
@@ -2421,8 +2445,7 @@ void launch_dense_fp64(const BatchView &bv, int num_sms, cudaStream_t stream, cu
 
 template <size_t... I>
 void set_variant_smem(int bytes, int seg_bytes, std::index_sequence<I...>) {
-  (cudaFuncSetAttribute(k_waveform<true, 0, wave_variant(true, (int)I).pre, wave_variant(true, (int)I).joint,
-                                   wave_variant(true, (int)I).min_blocks>,
+  (cudaFuncSetAttribute(k_wave_split<std::max(wave_variant(true, (int)I).joint, 1), wave_variant(true, (int)I).min_blocks>,
                         cudaFuncAttributeMaxDynamicSharedMemorySize, bytes),
    ...);
   (cudaFuncSetAttribute(k_wave_segments<std::max(wave_variant(false, (int)I).joint, 1), wave_variant(false, (int)I).min_blocks>,
@@ -2465,7 +2488,7 @@ void launch_persistent(K kernel, const BatchView &bv, int num_sms, size_t dyn, c
 template <int v>
 void launch_split_variant(const BatchView &bv, int num_sms, size_t dyn, cudaStream_t stream) {
   constexpr WaveVariant w = wave_variant(true, v);
-  launch_persistent(k_waveform<true, 0, w.pre, w.joint, w.min_blocks>, bv, num_sms, dyn, stream);
+  launch_persistent(k_wave_split<std::max(w.joint, 1), w.min_blocks>, bv, num_sms, dyn, stream);
 }
 template <size_t... I>
 void launch_split_index(int v, const BatchView &bv, int num_sms, size_t dyn, cudaStream_t stream,

@@ -263,24 +263,27 @@ void launch_phase(const BatchView &bv, int num_sms, cudaStream_t stream, cudaEve
 // writes with trajectory_only) of source s of the batch.
 // Natural-spline coefficients c (half second derivatives, c = 0 at both ends)
 // of every source's knots, solved on the device: the interior knots of a
-// source are cut into blocks of `block` (spline_block), each solved by Thomas
+// source are cut into blocks, each solved by Thomas
 // elimination over the block widened by kSplineHalo knots on either side,
 // taking c = 0 where the widened window is cut.  The system is diagonally
 // dominant (|h0| + |h1| = half the diagonal 2 (h0 + h1)), so the influence of
 // a cut decays at least as 0.27^k with the distance k in knots: 40 knots leave
 // it below 1e-22.  blk_start: nsrc + 1 prefix of the blocks per source
 // (spline_blocks).
-constexpr int kSplineBlockLong = 256;
-constexpr int kSplineBlockShort = 48;
+// FP64 batches: kSplineBlock knots on four lanes.  Split batches: one thread a
+// block of kSplineBlockLong.  The two contract multiply-adds differently, a
+// relative 1e-13 in c and an ulp of a phase here and there; FP64 samples differ
+// by 1e-12, but a split sample with its phase on the edge of an FP32 rounding by
+// 1e-7 of the largest, and in a single-precision likelihood that shows.
+// Measured (quad / long): 336 knots a source 0.01 / 0.32 ms, 5e6 knots 0.45 /
+// 0.54, 12e6 1.03 / 1.03.
+constexpr int kSplineBlock = 64, kSplineBlockLong = 256;
 constexpr int kSplineHalo = 40;
-// Block length for a batch of `knots` knots: short blocks on four lanes where
-// the long blocks' serial chains would leave the chip idle, long ones where the
-// halos' extra work counts.  Measured on a B200 (short / long): 0.1e6 knots
-// 0.01 / 0.32 ms, 5.3e6 0.41 / 0.52, 8.4e6 0.73 / 0.51, 20e6 1.6 / 1.06.
-constexpr int64_t kSplineShortMax = 6000000;
-inline int spline_block(int64_t knots) { return knots <= kSplineShortMax ? kSplineBlockShort : kSplineBlockLong; }
-inline int64_t spline_blocks(int n_knots, int block) { return n_knots < 3 ? 1 : (n_knots - 2 + block - 1) / block; }
-void launch_spline_coeffs(const SourceDesc *src, int nsrc, const int64_t *blk_start, int64_t total_blocks, int block,
+inline int64_t spline_blocks(int n_knots, bool split) {
+  const int block = split ? kSplineBlockLong : kSplineBlock;
+  return n_knots < 3 ? 1 : (n_knots - 2 + block - 1) / block;
+}
+void launch_spline_coeffs(const SourceDesc *src, int nsrc, const int64_t *blk_start, int64_t total_blocks, bool split,
                           const double *knot_t, const double4 *knot_y, double4 *knot_c, cudaStream_t stream);
 
 // The knot window of every tile of a batch (tile_knot, 2 per tile: the knots
