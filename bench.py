@@ -380,7 +380,7 @@ def run_fisher(g, n_points: int) -> dict:
                               "peak": hbm, "unit": "GB/s", "frac": gbs / hbm,
                               "bytes": gram_bytes, "peak_source": "measured copy bandwidth (MEASURED_PEAKS.json)"
                               if peaks.get("hbm_gbs") else "fallback"},
-            "gpu_launches_per_matrix": 6,  # spline solve, tile pre-pass (2), k_waveform, Fisher Gram (2) (+ cuFFT)
+            "gpu_launches_per_matrix": 8,  # layout, spline, segments, carries, direct tiles, waveform, Gram (2) (+ cuFFT)
             "cpu_baseline": ref_fisher_seconds()}
 
 
@@ -704,13 +704,13 @@ def run_phases(args, wb, sources, sptr, stream, N, N_all, reduce_max, local_rank
                     "of the configuration-1 batch",
         "value": N_all / (ms * 1e-3), "unit": "samples/s", "ms_per_step": ms,
         "kernel_ms": {"clears": kern[0], "phase_and_freeze": kern[2]},
-        "roofline": {"kernel": "k_tile_params + k_waveform<fp64, phase> + k_phase_freeze", "bound": "hbm", "achieved": gbs,
+        "roofline": {"kernel": "k_tile_segments + k_tile_carries + k_waveform<fp64, phase>", "bound": "hbm", "achieved": gbs,
                      "peak": hbm, "unit": "GB/s", "frac": gbs / hbm, "peak_source": hbm_src,
                      "bytes_per_sample": bytes_per_sample},
         "e2e": {"value": Np / e2e_s, "unit": "samples/s", "seconds_per_step": e2e_s, "sources": len(sub),
                 "samples": Np, "h2d_bytes_per_step": h2d,
                 "d2h_bytes_per_step": 64 * Np, "host_threads": nthreads},
-        "gpu_launches_per_step": 3,  # k_tile_params, k_waveform<fp64, phase>, k_phase_freeze
+        "gpu_launches_per_step": 3,  # k_tile_segments, k_tile_carries, k_waveform<fp64, phase>
     }
 
 
@@ -855,7 +855,7 @@ def run_gpu(args, rank, world, local_rank):
     clk = clocks.stop()
     ms = reduce_max(ev0.elapsed_time(ev1))
     # k_spline_coeffs, the tile pre-pass (two kernels, when the tuned shape uses
-    # it) and k_waveform<split> per replay; the clears are memset nodes
+    # it) and k_wave_split per replay; the clears are memset nodes
     launches = wb.launches() * args.steps
     value = N_all * args.steps / (ms * 1e-3)
     # accuracy of every source against the FP64 outputs of the same batch
@@ -878,7 +878,7 @@ def run_gpu(args, rank, world, local_rank):
     ach64 = fps * N / ((kern[1] + kern[2]) * 1e-3) / 1e12
     fp64 = {"value": value64, "unit": "samples/s", "ms_per_step": ms64 / args.steps,
             "kernel_ms": {"clears": kern[0], "tile_prepass": kern[1], "waveform_fp64": kern[2]},
-            "roofline": {"kernel": "k_tile_params + k_tile_table + k_waveform<fp64>", "bound": "fp64",
+            "roofline": {"kernel": "k_tile_segments + k_tile_carries + k_wave_segments", "bound": "fp64",
                          "achieved": ach64, "peak": fp64_peak,
                          "unit": "TFLOP/s", "frac": ach64 / fp64_peak if fp64_peak > 0 else None,
                          "peak_source": "measured FP64 FMA rate on this GPU (aak_probe_fp64_tflops)"},
@@ -1030,7 +1030,7 @@ def run_gpu(args, rank, world, local_rank):
     # ---- roofline of the dominant kernel (split harmonic sum: FP32 mode sums, FP64 phases)
     wave_ms = kern_s[1] + kern_s[2]  # the harmonic sums' Bessel tables are built in the pre-pass
     achieved = fps * N / (wave_ms * 1e-3) / 1e12
-    roofline = {"kernel": "k_waveform<split> (with its tile pre-pass k_tile_params + k_tile_table)", "bound": "fp32",
+    roofline = {"kernel": "k_wave_split (with its tile pre-pass k_tile_params + k_tile_table)", "bound": "fp32",
                 "achieved": achieved, "peak": fp32_peak,
                 "unit": "TFLOP/s", "frac": achieved / fp32_peak if fp32_peak > 0 else None,
                 "traffic": TRAFFIC_BYTES_PER_SAMPLE * N,

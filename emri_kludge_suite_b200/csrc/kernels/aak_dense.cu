@@ -11,6 +11,9 @@
 //   carry from the earlier tiles of the source, and phase 2 evaluates the
 //   harmonic sums (FP64, or split precision); h_I, h_II are written with
 //   coalesced stores.
+// k_wave_split (aak_split.cuh): the same passes for split batches.
+// k_tile_segments, k_tile_carries, k_wave_segments (aak_segments.cuh): FP64
+//   batches, from polynomials of 256 samples.
 #include <cuda_runtime.h>
 #include <math.h>
 
