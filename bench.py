@@ -957,6 +957,8 @@ def run_gpu(args, rank, world, local_rank):
             fr = x - k
             return torch.exp(-(logS[k] * (1 - fr) + logS[k + 1] * fr))
 
+        # every source has a length of its own: a plan kept for each would fill the device
+        torch.backends.cuda.cufft_plan_cache.max_size = 4
         o2 = w2.offsets
         mm2, rel2, psd2 = [], [], []
         for s_ in range(len(src2)):
