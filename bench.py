@@ -959,6 +959,7 @@ def run_gpu(args, rank, world, local_rank):
 
         # every source has a length of its own: a plan kept for each would fill the device
         torch.backends.cuda.cufft_plan_cache.max_size = 4
+        torch.cuda.empty_cache()  # a plan's tables are allocated outside torch's pool
         o2 = w2.offsets
         mm2, rel2, psd2 = [], [], []
         for s_ in range(len(src2)):
@@ -970,6 +971,7 @@ def run_gpu(args, rank, world, local_rank):
             mm2.append(1.0 - ab / math.sqrt(aa * bb) if aa > 0 and bb > 0 else 0.0)
             rel2.append(float(torch.maximum((x1 - y1).abs().max(), (x2 - y2).abs().max()) /
                               torch.maximum(x1.abs().max(), x2.abs().max())))
+            torch.cuda.empty_cache()
             w = inv_psd(len(x1), DT)
             paa = pbb = pab = 0.0
             for u, v in ((x1, y1), (x2, y2)):
