@@ -2846,7 +2846,10 @@ int aak_gpu_gen(aak_gpu *g, const double *pars14) {
 }
 
 int aak_gpu_get_waveform(aak_gpu *g, double *t, double *hI, double *hII) {
-  if (!g || !t || !hI || !hII || g->count < 1) return AAK_ERR_INVALID_PARAM;
+  if (!g || !t || !hI || !hII) return AAK_ERR_INVALID_PARAM;
+  // held over the read: packed rows are made half spectra in place, and a batch on another thread writes the rows
+  std::lock_guard<std::mutex> lk(g->ctx->mu);
+  if (g->count < 1) return AAK_ERR_INVALID_PARAM;
   const size_t n = (size_t)g->length + 2;
   std::vector<double> buf(n, 0.0);
   int r;
