@@ -2394,33 +2394,32 @@ int gpu_generate(aak_gpu *g, const double *x, int B, int nthreads, int32_t *stat
 // pack: leave FP64 rows of even length packed, for a reduction that reads them
 // so; otherwise the rows end as half spectra, packed ones of an earlier call too.
 int gpu_fft_rows(aak_gpu *g, bool pack = false) {
-  cufftHandle h;
-  int r;
-  if (!g->spectral && g->rows32) {
-    if ((r = fft_plan(g, CUFFT_R2C, g->count, &h)) != AAK_OK) return r;
-    for (int ch = 0; ch < 2; ++ch)
-      if (cufftExecR2C(h, g->d_H32[ch].ptr, reinterpret_cast<cufftComplex *>(g->d_H32[ch].ptr)) != CUFFT_SUCCESS)
-        return AAK_ERR_CUDA;
-    g->spectral = true;
-    g->packed = false;
-    return AAK_OK;
-  }
-  if (!g->spectral) {
-    g->packed = pack && g->length % 2 == 0;
-    if ((r = fft_plan(g, g->packed ? CUFFT_Z2Z : CUFFT_D2Z, g->count, &h)) != AAK_OK) return r;
-    for (int ch = 0; ch < 2; ++ch) {
-      cufftDoubleComplex *z = reinterpret_cast<cufftDoubleComplex *>(g->d_H[ch].ptr);
-      const cufftResult e = g->packed ? cufftExecZ2Z(h, z, z, CUFFT_FORWARD) : cufftExecD2Z(h, g->d_H[ch].ptr, z);
-      if (e != CUFFT_SUCCESS) return AAK_ERR_CUDA;
-    }
-    g->spectral = true;
-    return AAK_OK;
-  }
-  if (g->packed && !pack) {
+  if (g->spectral) {
+    if (!g->packed || pack) return AAK_OK;
     for (int ch = 0; ch < 2; ++ch) launch_unpack_rows(g->d_H[ch].ptr, g->row, g->count, g->stream);
     g->packed = false;
     return cuda_ok(cudaGetLastError());
   }
+  pack = pack && !g->rows32 && g->length % 2 == 0;
+  cufftHandle h;
+  // without a plan or its work area the rows stay what they are: the templates' samples
+  const int r = fft_plan(g, g->rows32 ? CUFFT_R2C : pack ? CUFFT_Z2Z : CUFFT_D2Z, g->count, &h);
+  if (r != AAK_OK) return r;
+  for (int ch = 0; ch < 2; ++ch) {
+    cufftResult e;
+    if (g->rows32) {
+      e = cufftExecR2C(h, g->d_H32[ch].ptr, reinterpret_cast<cufftComplex *>(g->d_H32[ch].ptr));
+    } else {
+      cufftDoubleComplex *z = reinterpret_cast<cufftDoubleComplex *>(g->d_H[ch].ptr);
+      e = pack ? cufftExecZ2Z(h, z, z, CUFFT_FORWARD) : cufftExecD2Z(h, g->d_H[ch].ptr, z);
+    }
+    if (e != CUFFT_SUCCESS) {
+      g->count = 0;  // a channel may be transformed and the other not: no template to be had from the rows
+      return AAK_ERR_CUDA;
+    }
+  }
+  g->spectral = true;
+  g->packed = pack;
   return AAK_OK;
 }
 
@@ -2534,6 +2533,7 @@ int gpu_rows_launch(aak_gpu *g, const double *x, int B, int nthreads, int32_t *s
   const int threads = nthreads > 0 ? nthreads : (int)std::max(1u, std::thread::hardware_concurrency());
   const int size = (fe || B <= 2 * threads) ? B : (B >= 16 * threads) ? (B + 1) / 2 : std::max(3 * threads, (B + kUnitsMax - 1) / kUnitsMax);
   g->units[p] = 0;
+  g->count = 0;  // until the last unit is queued the rows hold no chunk
   for (int k0 = 0; k0 < B; k0 += size) {
     const int n = std::min(size, B - k0), q = (int)(g->unit++ & 1);
     aak_ctx *C = q ? g->ctx2 : g->ctx;
