@@ -1819,6 +1819,8 @@ int aak_ctx_set_precision(aak_ctx *ctx, int32_t precision) {
 // sources and median length in powers of two) by timing every candidate on
 // the uploaded batch; the choice and the timings are appended to a tuning
 // cache file, and a later call with the same key reads the choice from there.
+// The key names the table of shapes (kVariantTable): an index chosen among
+// other shapes is not taken for one of these.
 static_assert(AAK_NUM_VARIANTS == kNumVariants, "the header states the number of launch shapes");
 
 namespace {
@@ -1836,8 +1838,8 @@ std::string tune_key(aak_ctx *ctx, int precision) {
   const int32_t med = len.empty() ? 0 : len[len.size() / 2];
   auto lg = [](double x) { return x > 0 ? (int)std::lround(std::log2(x)) : 0; };
   char buf[256];
-  std::snprintf(buf, sizeof(buf), "%s|sm%d|p%d|nm%d|src2^%d|len2^%d", name.c_str(), prop.multiProcessorCount, precision,
-                ctx->max_nmodes, lg((double)ctx->nsrc), lg((double)med));
+  std::snprintf(buf, sizeof(buf), "%s|sm%d|t%d|p%d|nm%d|src2^%d|len2^%d", name.c_str(), prop.multiProcessorCount,
+                kVariantTable, precision, ctx->max_nmodes, lg((double)ctx->nsrc), lg((double)med));
   return buf;
 }
 
@@ -1892,7 +1894,7 @@ int aak_ctx_autotune(aak_ctx *ctx, double *d_hI, double *d_hII, int32_t precisio
     for (int rep = 0; rep < 3 && r == AAK_OK; ++rep) {  // one warm-up, then the faster of two
       cudaEventRecord(e0, st);
       need_knots(ctx, precision, st);
-      launch_dense(bv, ctx->num_sms, st, nullptr, precision);
+      launch_dense(bv, ctx->num_sms, st, nullptr, precision, &ctx->side);  // as run() launches it
       cudaEventRecord(e1, st);
       if ((r = cuda_ok(cudaEventSynchronize(e1))) != AAK_OK) break;
       float t = 0.0f;

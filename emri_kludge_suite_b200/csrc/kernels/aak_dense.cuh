@@ -114,6 +114,9 @@ struct WaveVariant {
   int min_blocks;
 };
 constexpr int kNumVariants = 6;
+// Part of a tuning-cache key.  Raised whenever an index of wave_variant comes to mean another shape or another kernel
+// (1, which keys did not name: FP64 0 = {true, 1, 3} and 5 = {true, 2, 3} of k_waveform).
+constexpr int kVariantTable = 2;
 constexpr WaveVariant wave_variant(bool split, int v) {
   return split ? (v == 1 ? WaveVariant{false, 0, 2} : v == 2 ? WaveVariant{true, 1, 2} : v == 3 ? WaveVariant{true, 4, 2}
                   : v == 4 ? WaveVariant{true, 2, 3} : v == 5 ? WaveVariant{true, 2, 2} : WaveVariant{true, 1, 3})
