@@ -45,15 +45,17 @@ struct DevBuf {
     if (ptr) cudaFree(ptr);
     ptr = nullptr;
     cap = 0;
-    size_t want = std::max<size_t>(n, 1);
-    want += want / 4;  // growth headroom
-    if (cudaMalloc(&ptr, want * sizeof(T)) != cudaSuccess) {
+    n = std::max<size_t>(n, 1);
+    // a quarter of headroom for growth, where the memory has room for it
+    for (size_t want : {n + n / 4, n}) {
+      if (cudaMalloc(&ptr, want * sizeof(T)) == cudaSuccess) {
+        cap = want;
+        return AAK_OK;
+      }
       cudaGetLastError();
       ptr = nullptr;
-      return AAK_ERR_NO_MEMORY;
     }
-    cap = want;
-    return AAK_OK;
+    return AAK_ERR_NO_MEMORY;
   }
   void release() {
     if (ptr) cudaFree(ptr);
@@ -66,6 +68,19 @@ int cuda_ok(cudaError_t e) { return cuda_status_of(e); }
 
 
 }  // namespace
+
+// What one dense launch writes for itself.  Nothing in it outlives the launch,
+// so that contexts whose launches follow one another on one stream may share it.
+struct DenseScratch {
+  DevBuf<TilePrep> prep;       // tile pre-pass: per-tile parameters
+  DevBuf<unsigned char> tab;   //   and per-tile Taylor tables
+  DevBuf<unsigned char> seg[2];  // FP64 polynomial segments of the waveform and of the phase product (seg_parts)
+  void release() {
+    prep.release();
+    tab.release();
+    for (auto &s : seg) s.release();
+  }
+};
 
 struct aak_ctx {
   int device = 0;
@@ -105,12 +120,8 @@ struct aak_ctx {
   DevBuf<TileLink> d_link;                // look-back records, one per tile
   DevBuf<int32_t> d_flag;                 // look-back flags, one per tile
   DevBuf<unsigned long long> d_counter;   // [0] work-queue head, [1] device status word
-  DevBuf<TilePrep> d_tile_prep;           // tile pre-pass: per-tile parameters
-  DevBuf<unsigned char> d_tile_tab;       //   and per-tile Taylor tables
-  DevBuf<unsigned char> d_tile_seg;       // FP64: polynomial segments, one slot per tile
-  DevBuf<SegAgg> d_seg_agg;               //   the tiles' phase increments,
-  DevBuf<int32_t> d_direct, d_seg_ctl;    //   the direct tiles, counters,
-  DevBuf<double> d_frozen;                //   and the phases at i_plunge, 3 per source
+  DenseScratch own_scratch, *scratch = &own_scratch;
+  bool no_segments = false;               // the segments found no memory: not asked for again before the next upload
   DevBuf<double> d_out;  // outputs for the host-buffer entry points
   // batched device solve of the Kerr -> AK map (opt-in: parmap_device)
   bool parmap_device = false;
@@ -140,7 +151,7 @@ struct aak_ctx {
   double *g_hI = nullptr, *g_hII = nullptr;
   int g_prec = -1;
   uint64_t g_gen = ~0ull;
-  int g_variant = -1;
+  int g_variant = -1, g_launches = 0;
   int variant[2] = {0, 0};  // launch shape of the waveform stage per precision (autotuner; 0: default)
   int64_t newton_points = 0, newton_iters = 0, newton_fallbacks = 0;
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -797,6 +808,63 @@ void need_knots(aak_ctx *ctx, int precision, cudaStream_t st) {
   if (ctx->spl_split != (precision == 1)) solve_knots(ctx, precision == 1, st);
 }
 
+void drop_graph(aak_ctx *ctx);
+
+// The memory of the FP64 polynomial segments of a launch, one allocation:
+// counters, the phases at i_plunge (phase product, 3 per source), the tiles'
+// phase increments, the direct tiles, and a slot per tile.
+struct SegParts {
+  size_t frozen, agg, direct, slots, total;
+};
+SegParts seg_parts(int64_t tiles, int nsrc, bool phase) {
+  const auto al = [](size_t x) { return (x + 255) / 256 * 256; };
+  SegParts p;
+  p.frozen = al(seg_ctl_words(nsrc) * sizeof(int32_t));
+  p.agg = p.frozen + al(phase ? 3 * (size_t)nsrc * sizeof(double) : 0);
+  p.direct = p.agg + al((size_t)tiles * sizeof(SegAgg));
+  p.slots = p.direct + al((size_t)tiles * sizeof(int32_t));
+  p.total = p.slots + (size_t)tiles * (phase ? kSegSlotBytesPhase : kSegSlotBytes);
+  return p;
+}
+
+// Give the segments' memory back (a launch without them takes the in-tile kernels).
+void drop_segments(aak_ctx *ctx) {
+  drop_graph(ctx);
+  for (auto &s : ctx->scratch->seg) s.release();
+}
+
+// The segments' memory, grown as needed, set in bv.  Where the device has none
+// left (4.5 KB a tile for the waveform, 2.1 KB for the phase product), the
+// launch does without: every source then takes the in-tile kernels.
+void tile_segments(aak_ctx *ctx, BatchView &bv, bool phase) {
+  if (ctx->no_segments) return;
+  const int64_t tiles = std::max<int64_t>(ctx->total_tiles, 1);
+  const SegParts p = seg_parts(tiles, ctx->nsrc, phase);
+  DevBuf<unsigned char> &buf = ctx->scratch->seg[phase];
+  const void *old = buf.ptr;
+  if (buf.reserve(p.total) != AAK_OK) {
+    drop_segments(ctx);
+    ctx->no_segments = true;
+    return;
+  }
+  if (buf.ptr != old) drop_graph(ctx);
+  unsigned char *b = buf.ptr;
+  bv.seg_ctl = reinterpret_cast<int32_t *>(b);
+  bv.frozen = phase ? reinterpret_cast<double *>(b + p.frozen) : nullptr;
+  bv.tile_agg = reinterpret_cast<SegAgg *>(b + p.agg);
+  bv.direct_list = reinterpret_cast<int32_t *>(b + p.direct);
+  bv.tile_seg = b + p.slots;
+}
+
+// Run `f`, which reserves device memory; where there is none left, once more without the segments'.
+template <typename F>
+int with_room(aak_ctx *ctx, F f) {
+  int r = f();
+  if (r != AAK_ERR_NO_MEMORY || (!ctx->scratch->seg[0].ptr && !ctx->scratch->seg[1].ptr)) return r;
+  drop_segments(ctx);
+  return f();
+}
+
 // wait_pinned: finish the copies from page-locked plan arrays before
 // returning (callers whose next plan may refill those arrays); a caller that
 // keeps the plans untouched until it synchronises the stream passes false.
@@ -804,20 +872,23 @@ int upload(aak_ctx *ctx, cudaStream_t st, bool wait_pinned = true) {
   int r;
   if ((r = select_device(ctx->device)) != AAK_OK) return r;
   const int n = ctx->nsrc;
-  if ((r = ctx->d_src.reserve(n)) || (r = ctx->d_tile_start.reserve(n + 1)) ||
-      (r = ctx->d_tile_knot.reserve(2 * std::max<int64_t>(ctx->total_tiles, 1))) ||
-      (r = ctx->d_tile_pairs.reserve(ctx->tile_pairs.size())) ||
-      (r = ctx->d_queue.reserve(std::max<int64_t>(ctx->total_tiles, 1))) ||
-      (r = ctx->d_queue_rank.reserve(ctx->queue_rank.size())) || (r = ctx->d_queue_step.reserve(ctx->queue_step.size())) ||
-      (r = ctx->d_spl_blk.reserve(ctx->spl_blk.size())) ||
-      // knot times: two entries of slack past the last knot (a window's bulk
-      // copy starts on a 16-byte boundary and may read one element beyond it)
-      (r = ctx->d_knot_t.reserve(std::max<int64_t>(ctx->total_knots, 1) + 2)) ||
-      (r = ctx->d_knot_y.reserve(std::max<int64_t>(ctx->total_knots, 1))) ||
-      (r = ctx->d_knot_c.reserve(std::max<int64_t>(ctx->total_knots, 1))) || (r = ctx->d_bessel.reserve(ctx->bessel.size())) ||
-      (r = ctx->d_link.reserve(std::max<int64_t>(ctx->total_tiles, 1))) ||
-      (r = ctx->d_flag.reserve(std::max<int64_t>(ctx->total_tiles, 1))) || (r = ctx->d_counter.reserve(2)))
-    return r;
+  ctx->no_segments = false;
+  r = with_room(ctx, [&] {
+    const size_t tiles = (size_t)std::max<int64_t>(ctx->total_tiles, 1), knots = (size_t)std::max<int64_t>(ctx->total_knots, 1);
+    int e;
+    if ((e = ctx->d_src.reserve(n)) || (e = ctx->d_tile_start.reserve(n + 1)) || (e = ctx->d_tile_knot.reserve(2 * tiles)) ||
+        (e = ctx->d_tile_pairs.reserve(ctx->tile_pairs.size())) || (e = ctx->d_queue.reserve(tiles)) ||
+        (e = ctx->d_queue_rank.reserve(ctx->queue_rank.size())) || (e = ctx->d_queue_step.reserve(ctx->queue_step.size())) ||
+        (e = ctx->d_spl_blk.reserve(ctx->spl_blk.size())) ||
+        // knot times: two entries of slack past the last knot (a window's bulk
+        // copy starts on a 16-byte boundary and may read one element beyond it)
+        (e = ctx->d_knot_t.reserve(knots + 2)) || (e = ctx->d_knot_y.reserve(knots)) || (e = ctx->d_knot_c.reserve(knots)) ||
+        (e = ctx->d_bessel.reserve(ctx->bessel.size())) || (e = ctx->d_link.reserve(tiles)) ||
+        (e = ctx->d_flag.reserve(tiles)) || (e = ctx->d_counter.reserve(2)))
+      return e;
+    return (int)AAK_OK;
+  });
+  if (r != AAK_OK) return r;
   // the work-queue head is cleared by every launch; the status word here
   if ((r = cuda_ok(cudaMemsetAsync(ctx->d_counter.ptr, 0, 2 * sizeof(unsigned long long), st))) != AAK_OK) return r;
   auto cp = [&](void *dst, const void *src, size_t bytes) {
@@ -856,54 +927,38 @@ int upload(aak_ctx *ctx, cudaStream_t st, bool wait_pinned = true) {
 
 BatchView batch_view(aak_ctx *ctx, double *hI, double *hII, double *t, double *traj, int64_t traj_stride);
 
-// The tile pre-pass buffers of a waveform launch in `precision` (one
-// TilePrep and one Taylor-table slot per tile), grown as needed, set in bv.
-void drop_graph(aak_ctx *ctx);
-
-// The buffers of the FP64 polynomial segments, grown as needed, set in bv.
-int tile_segments(aak_ctx *ctx, BatchView &bv) {
-  const int64_t tiles = std::max<int64_t>(ctx->total_tiles, 1);
-  const void *s0 = ctx->d_tile_seg.ptr, *c0 = ctx->d_seg_ctl.ptr, *a0 = ctx->d_seg_agg.ptr, *l0 = ctx->d_direct.ptr,
-             *f0 = ctx->d_frozen.ptr;
-  int r;
-  if ((r = ctx->d_tile_seg.reserve(tiles * kSegSlotBytes)) != AAK_OK || (r = ctx->d_seg_agg.reserve(tiles)) != AAK_OK ||
-      (r = ctx->d_direct.reserve(tiles)) != AAK_OK ||
-      (r = ctx->d_seg_ctl.reserve(seg_ctl_words(ctx->nsrc))) != AAK_OK || (r = ctx->d_frozen.reserve(3 * (size_t)ctx->nsrc)) != AAK_OK)
-    return r;
-  if (ctx->d_tile_seg.ptr != s0 || ctx->d_seg_ctl.ptr != c0 || ctx->d_seg_agg.ptr != a0 || ctx->d_direct.ptr != l0 ||
-      ctx->d_frozen.ptr != f0)
-    drop_graph(ctx);
-  bv.tile_seg = ctx->d_tile_seg.ptr;
-  bv.seg_ctl = ctx->d_seg_ctl.ptr;
-  bv.frozen = ctx->d_frozen.ptr;
-  bv.tile_agg = ctx->d_seg_agg.ptr;
-  bv.direct_list = ctx->d_direct.ptr;
-  return AAK_OK;
-}
-
 // Kernels of one dense launch: the in-tile kernel alone; with the pre-pass,
 // split: tile parameters, tables, waveform; FP64: the in-tile kernel for the
 // small sources, and for the others segments, carries (with the tables), the
 // direct tiles and the segments' waveform.
-int dense_launches(const aak_ctx *ctx, int precision) {
-  if (!wave_variant(precision == 1, ctx->variant[precision]).pre) return 1;
+int dense_launches(const aak_ctx *ctx, int precision, const BatchView &bv) {
+  if (!bv.tile_prep || !wave_variant(precision == 1, ctx->variant[precision]).pre) return 1;
   if (precision == 1) return 3;
+  if (!bv.tile_seg) return 1;
   return (ctx->small_tiles > 0 ? 1 : 0) + (ctx->small_tiles < ctx->total_tiles ? 4 : 0);
 }
 
+// The tile pre-pass buffers of a waveform launch in `precision` (one
+// TilePrep and one Taylor-table slot per tile), grown as needed, set in bv.
 int tile_tables(aak_ctx *ctx, int precision, BatchView &bv) {
+  // sources inside the in-tile kernel's sizes only: it needs none of this
+  if (precision == 0 && ctx->small_tiles == ctx->total_tiles) return AAK_OK;
   const int64_t tiles = std::max<int64_t>(ctx->total_tiles, 1);
   const int64_t slot = tile_table_slot_bytes(ctx->max_nmodes, precision == 1);
-  const void *p0 = ctx->d_tile_prep.ptr, *t0 = ctx->d_tile_tab.ptr;
-  int r;
-  if ((r = ctx->d_tile_prep.reserve(tiles)) != AAK_OK || (r = ctx->d_tile_tab.reserve(tiles * slot)) != AAK_OK)
-    return r;
+  DenseScratch &S = *ctx->scratch;
+  const void *p0 = S.prep.ptr, *t0 = S.tab.ptr;
+  const int r = with_room(ctx, [&] {
+    const int e = S.prep.reserve(tiles);
+    return e != AAK_OK ? e : S.tab.reserve(tiles * slot);
+  });
+  if (r != AAK_OK) return r;
   // a captured dense graph holds the old buffers: recapture on its next use
-  if (ctx->d_tile_prep.ptr != p0 || ctx->d_tile_tab.ptr != t0) drop_graph(ctx);
-  bv.tile_prep = ctx->d_tile_prep.ptr;
-  bv.tile_tab = ctx->d_tile_tab.ptr;
+  if (S.prep.ptr != p0 || S.tab.ptr != t0) drop_graph(ctx);
+  bv.tile_prep = S.prep.ptr;
+  bv.tile_tab = S.tab.ptr;
   bv.tab_slot = slot;
-  return precision == 0 ? tile_segments(ctx, bv) : AAK_OK;
+  if (precision == 0) tile_segments(ctx, bv, false);
+  return AAK_OK;
 }
 
 int run(aak_ctx *ctx, double *hI, double *hII, double *t, double *traj, int64_t traj_stride, int precision,
@@ -921,7 +976,7 @@ int run(aak_ctx *ctx, double *hI, double *hII, double *t, double *traj, int64_t 
     for (auto &e : ctx->ev) cudaEventCreate(&e);
   need_knots(ctx, precision, st);
   launch_dense(bv, ctx->num_sms, st, ctx->profile ? ctx->ev : nullptr, precision, &ctx->side);
-  ctx->last_launches = bv.tile_prep ? dense_launches(ctx, precision) : 1;
+  ctx->last_launches = dense_launches(ctx, precision, bv);
   return cuda_ok(cudaGetLastError());
 }
 
@@ -987,9 +1042,10 @@ int run_graph(aak_ctx *ctx, double *hI, double *hII, int precision, cudaStream_t
     ctx->g_prec = precision;
     ctx->g_gen = ctx->upload_gen;
     ctx->g_variant = ctx->variant[precision];
+    ctx->g_launches = 1 + dense_launches(ctx, precision, bv);  // with the spline solve
   }
   ctx->spl_split = precision == 1;
-  ctx->last_launches = 1 + dense_launches(ctx, precision);  // with the spline solve
+  ctx->last_launches = ctx->g_launches;
   return cuda_ok(cudaGraphLaunch(ctx->gexec, st));
 }
 
@@ -1032,17 +1088,18 @@ int run_phase(aak_ctx *ctx, double *out, int64_t stride, cudaStream_t st) {
   bv.phase_stride = stride;
   bv.trajectory_only = 1;
   // the tile pre-pass's parameters (no tables in the phase product)
-  const void *p0 = ctx->d_tile_prep.ptr;
-  if ((r = ctx->d_tile_prep.reserve(std::max<int64_t>(ctx->total_tiles, 1))) != AAK_OK) return r;
-  if (ctx->d_tile_prep.ptr != p0) drop_graph(ctx);
-  bv.tile_prep = ctx->d_tile_prep.ptr;
-  if ((r = tile_segments(ctx, bv)) != AAK_OK) return r;
+  DenseScratch &S = *ctx->scratch;
+  const void *p0 = S.prep.ptr;
+  if ((r = with_room(ctx, [&] { return S.prep.reserve(std::max<int64_t>(ctx->total_tiles, 1)); })) != AAK_OK) return r;
+  if (S.prep.ptr != p0) drop_graph(ctx);
+  bv.tile_prep = S.prep.ptr;
+  if (ctx->small_tiles < ctx->total_tiles) tile_segments(ctx, bv, true);
   if (ctx->profile && !ctx->ev[0])
     for (auto &e : ctx->ev) cudaEventCreate(&e);
   need_knots(ctx, 0, st);
   launch_phase(bv, ctx->num_sms, st, ctx->profile ? ctx->ev : nullptr, &ctx->side);
   // small sources: tile parameters, phase pass, freeze; the others: segments, carries, phase pass
-  ctx->last_launches = (ctx->small_tiles > 0 ? 3 : 0) + (ctx->small_tiles < ctx->total_tiles ? 3 : 0);
+  ctx->last_launches = bv.tile_seg ? (ctx->small_tiles > 0 ? 3 : 0) + 3 : 3;
   return cuda_ok(cudaGetLastError());
 }
 
@@ -1581,14 +1638,9 @@ void aak_ctx_destroy(aak_ctx *c) {
     c->d_tile_pairs.release();
     c->d_queue.release();
     c->d_spl_blk.release();
-    c->d_tile_seg.release();
-    c->d_seg_ctl.release();
-    c->d_seg_agg.release();
-    c->d_direct.release();
     if (c->side.stream) cudaStreamDestroy(c->side.stream);
     for (cudaEvent_t e : {c->side.fork[0], c->side.fork[1], c->side.join})
       if (e) cudaEventDestroy(e);
-    c->d_frozen.release();
     c->d_knot_t.release();
     c->d_knot_y.release();
     c->d_knot_c.release();
@@ -1596,8 +1648,7 @@ void aak_ctx_destroy(aak_ctx *c) {
     c->d_link.release();
     c->d_flag.release();
     c->d_counter.release();
-    c->d_tile_prep.release();
-    c->d_tile_tab.release();
+    c->own_scratch.release();
     c->d_out.release();
     c->d_tdi.release();
     c->d_tdi_work.release();
@@ -2183,19 +2234,23 @@ struct aak_gpu {
 namespace {
 
 int gpu_capacity(aak_gpu *g, int B) {
-  int r;
-  if ((r = g->d_H[0].reserve((size_t)B * g->row)) || (r = g->d_H[1].reserve((size_t)B * g->row)) ||
-      (r = g->d_partial.reserve((size_t)B * kIpBlocksPerTemplate * 2)) || (r = g->d_out.reserve((size_t)B * 2)))
-    return r;
-  return AAK_OK;
+  return with_room(g->ctx, [&] {
+    int r;
+    if ((r = g->d_H[0].reserve((size_t)B * g->row)) || (r = g->d_H[1].reserve((size_t)B * g->row)) ||
+        (r = g->d_partial.reserve((size_t)B * kIpBlocksPerTemplate * 2)) || (r = g->d_out.reserve((size_t)B * 2)))
+      return r;
+    return (int)AAK_OK;
+  });
 }
 
 int gpu_capacity32(aak_gpu *g, int B) {
-  int r;
-  if ((r = g->d_H32[0].reserve((size_t)B * g->row)) || (r = g->d_H32[1].reserve((size_t)B * g->row)) ||
-      (r = g->d_partial.reserve((size_t)B * kIpBlocksPerTemplate * 2)) || (r = g->d_out.reserve((size_t)B * 2)))
-    return r;
-  return AAK_OK;
+  return with_room(g->ctx, [&] {
+    int r;
+    if ((r = g->d_H32[0].reserve((size_t)B * g->row)) || (r = g->d_H32[1].reserve((size_t)B * g->row)) ||
+        (r = g->d_partial.reserve((size_t)B * kIpBlocksPerTemplate * 2)) || (r = g->d_out.reserve((size_t)B * 2)))
+      return r;
+    return (int)AAK_OK;
+  });
 }
 
 // The in-place transform of the rows for a batch of B, ready on the
@@ -2232,7 +2287,7 @@ int fft_plan(aak_gpu *g, cufftType kind, int B, cufftHandle *out) {
   }
   aak_gpu::FftPlan &p = g->plans[k];
   p.used = ++g->plan_clock;
-  const int r = g->d_fft_work.reserve(std::max<size_t>(p.work, 1));
+  const int r = with_room(g->ctx, [&] { return g->d_fft_work.reserve(p.work); });
   if (r != AAK_OK) return r;
   if (cufftSetWorkArea(p.handle, g->d_fft_work.ptr) != CUFFT_SUCCESS ||
       cufftSetStream(p.handle, g->stream) != CUFFT_SUCCESS)
@@ -2482,6 +2537,7 @@ int gpu_pipeline_ready(aak_gpu *g, int max_batch) {
   int r;
   if (!g->ctx2 && (r = aak_ctx_create(g->ctx->device, &g->ctx2)) != AAK_OK) return r;
   aak_ctx *a = g->ctx, *b = g->ctx2;
+  b->scratch = a->scratch;  // their launches follow one another on g->stream
   b->want_pinned = a->want_pinned;
   b->parmap_device = a->parmap_device;
   b->evolve_device = a->evolve_device;
@@ -2498,9 +2554,6 @@ int gpu_pipeline_ready(aak_gpu *g, int max_batch) {
       if ((r = event(e)) != AAK_OK) return r;
     for (auto &e : g->uev[p])
       if ((r = event(e)) != AAK_OK) return r;
-    for (auto &u : g->tev[p])
-      for (auto &e : u)
-        if ((r = event(e)) != AAK_OK) return r;
   }
   if (g->stage_cap < max_batch) {
     if (g->h_stage) cudaFreeHost(g->h_stage);
@@ -2551,6 +2604,8 @@ int gpu_rows_launch(aak_gpu *g, const double *x, int B, int nthreads, int32_t *s
         (r = cuda_ok(cudaStreamWaitEvent(g->stream, g->uev[q][0], 0))) != AAK_OK)
       return r;
     cudaEvent_t *T = g->tev[p][g->units[p]++];
+    for (int k = 0; k < 2; ++k)
+      if (!T[k] && (r = cuda_ok(cudaEventCreate(&T[k]))) != AAK_OK) return r;
     const int64_t o = (int64_t)k0 * g->row;
     cudaEventRecord(T[0], g->stream);
     if (r32) r = run_rows32(C, g->d_H32[0].ptr + o, g->d_H32[1].ptr + o, 1, g->stream);

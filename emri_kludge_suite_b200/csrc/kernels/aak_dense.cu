@@ -1282,7 +1282,7 @@ __global__ void __launch_bounds__(128) k_tile_params(BatchView bv) {
   if (g >= bv.total_tiles) return;
   const int s = find_source(bv.tile_start, bv.nsrc, g);
   const SourceDesc &d = bv.src[s];
-  if (!kSplit && d.n_tiles > kSmallTiles) return;  // (the phase product's small sources)
+  if (!kSplit && bv.tile_seg && d.n_tiles > kSmallTiles) return;  // (the phase product's small sources)
   TilePrep P;
   P.ec = 0.0;
   P.K = -1;
@@ -2614,12 +2614,12 @@ void launch_dense(const BatchView &bv, int num_sms, cudaStream_t stream, cudaEve
 // i.e. the samples from max(i_plunge + i_buffer + 2, i0 + 1) on.  Rows 1-3 of
 // phase_out are sums of those three phases, so they take their own values at
 // i_plunge.  y strides over sources, x over each source's frozen samples.
-// (Small sources; the segments' phase pass writes them itself.)
-__global__ void __launch_bounds__(256) k_phase_freeze(const SourceDesc *__restrict__ src, int nsrc,
+// (Sources of at most max_tiles tiles; the segments' phase pass writes them itself.)
+__global__ void __launch_bounds__(256) k_phase_freeze(const SourceDesc *__restrict__ src, int nsrc, int max_tiles,
                                                       double *__restrict__ out, int64_t st) {
   for (int s = blockIdx.y; s < nsrc; s += gridDim.y) {
     const SourceDesc &d = src[s];
-    if (d.n_tiles > kSmallTiles || d.status != 0 || d.i_plunge < 0 || d.i_plunge >= d.vlength) continue;
+    if (d.n_tiles > max_tiles || d.status != 0 || d.i_plunge < 0 || d.i_plunge >= d.vlength) continue;
     const long long first = max((long long)d.i_plunge + (long long)d.i_buffer + 2, (long long)d.i0 + 1);
     if (first >= d.vlength) continue;
     const int64_t o = d.out_offset;
@@ -2635,32 +2635,34 @@ __global__ void __launch_bounds__(256) k_phase_freeze(const SourceDesc *__restri
 }
 
 void launch_phase(const BatchView &bv, int num_sms, cudaStream_t stream, cudaEvent_t *ev, const DenseSide *side) {
-  if (bv.total_tiles <= 0 || !bv.phase_out || !bv.tile_prep || !bv.tile_seg || !bv.frozen) return;
+  if (bv.total_tiles <= 0 || !bv.phase_out || !bv.tile_prep) return;
+  const int64_t small = bv.tile_seg ? bv.small_tiles : bv.total_tiles;  // without segments: every source as a small one
   if (ev) cudaEventRecord(ev[0], stream);
   prepare_dense_launch();
-  if (bv.small_tiles > 0) {
+  if (small > 0) {
     // the tile parameters from the pre-pass, each tile's inputs staged by bulk copies, carries by look-back
-    const bool only = bv.small_tiles == bv.total_tiles;
+    const bool only = small == bv.total_tiles;
     const cudaStream_t st = only ? stream : fork_side(side, 0, stream);
     BatchView sm = bv;
-    sm.total_tiles = bv.small_tiles;
+    sm.total_tiles = small;
     cudaMemsetAsync(bv.work_counter, 0, sizeof(unsigned long long), st);
     cudaMemsetAsync(bv.link_flag, 0, (size_t)bv.total_tiles * sizeof(int32_t), st);
     k_tile_params<false><<<(unsigned)((bv.total_tiles + 127) / 128), 128, 0, st>>>(bv);
     launch_persistent(k_waveform<false, 1, true, 0, 3>, sm, num_sms, kWaveDynSmem, st);
     const dim3 fgrid(64, (unsigned)std::min(std::max(bv.nsrc, 1), 1024));
-    k_phase_freeze<<<fgrid, 256, 0, st>>>(bv.src, bv.nsrc, bv.phase_out, bv.phase_stride);
+    k_phase_freeze<<<fgrid, 256, 0, st>>>(bv.src, bv.nsrc, bv.tile_seg ? kSmallTiles : 0x7fffffff, bv.phase_out,
+                                          bv.phase_stride);
   }
   if (ev) cudaEventRecord(ev[1], stream);
   if (ev) cudaEventRecord(ev[2], stream);
-  if (bv.small_tiles < bv.total_tiles) {
+  if (small < bv.total_tiles) {
     BatchView lg = bv;
-    lg.queue += bv.small_tiles;
-    lg.total_tiles -= bv.small_tiles;
+    lg.queue += small;
+    lg.total_tiles -= small;
     launch_segments<true>(lg, num_sms, 0, stream, nullptr);
     if (ev) cudaEventRecord(ev[2], stream);
     launch_persistent(k_waveform<false, 1, true, 0, 3, true>, lg, num_sms, kWaveDynSmem, stream);
-    if (bv.small_tiles > 0) join_side(side, stream);
+    if (small > 0) join_side(side, stream);
   }
   if (ev) cudaEventRecord(ev[3], stream);
 }

@@ -68,7 +68,8 @@ struct alignas(16) TileHead {
   int32_t pad[2];
 };
 static_assert(sizeof(TileHead) == 96, "the coefficients after the head stay 16-byte aligned");
-constexpr int64_t kSegSlotBytes = 96 + 4 * 108 * 8;  // head, 4 segments of at most 108 doubles
+constexpr int64_t kSegSlotBytes = 96 + 4 * 108 * 8;      // head, 4 segments of at most 108 doubles
+constexpr int64_t kSegSlotBytesPhase = 96 + 4 * 60 * 8;  // the phase product's: at most 60
 // Phase increments of one tile: forward and backward sums, and the clamped
 // Phidot after its last forward sample.
 struct SegAgg {

@@ -33,13 +33,16 @@ constexpr double kSegTol = 4e-15;
 constexpr int kSegWarps = 8;  // tiles of one CTA of k_tile_segments
 
 __device__ __forceinline__ TileHead *tile_head(const BatchView &bv, int64_t g) {
-  return reinterpret_cast<TileHead *>(bv.tile_seg + g * kSegSlotBytes);
+  return reinterpret_cast<TileHead *>(bv.tile_seg + g * (bv.phase_out ? kSegSlotBytesPhase : kSegSlotBytes));
 }
 
 // doubles of one segment's coefficients
 __host__ __device__ constexpr int seg_doubles(int D, bool phase) {
   return (3 * (D + 2) + (phase ? kPolyQPhase : kPolyQ) * (D + 1) + 1) / 2 * 2;
 }
+
+static_assert(kSegSlotBytes == sizeof(TileHead) + 4 * sizeof(double) * seg_doubles(7, false), "a slot of the waveform");
+static_assert(kSegSlotBytesPhase == sizeof(TileHead) + 4 * sizeof(double) * seg_doubles(7, true), "a slot of the phase product");
 
 struct SegTables {
   double fit4t[kSegNodes][kSegNodes];  // five rows of the cut fit, then the three dropped Chebyshev coefficients

@@ -51,7 +51,7 @@ def test_rows_after_a_call_without_memory():
         del hog
         torch.cuda.empty_cache()
         if out is not None:
-            assert np.array_equal(out, full), k
+            assert np.max(np.abs(out - full)) <= 1e-9 * full[:, 1].max(), k
         try:
             got = g.GetWaveform()[1:]
         except AAKError:
@@ -59,9 +59,9 @@ def test_rows_after_a_call_without_memory():
             got = None
         for c in range(2) if got is not None else ():
             s = got[c][0::2] + 1j * got[c][1::2]
-            is_spec = np.max(np.abs(s - spec[c])) <= 1e-12 * np.sum(np.abs(h[c]))
+            is_spec = np.max(np.abs(s - spec[c])) <= 1e-10 * np.sum(np.abs(h[c]))
             if out is None:
-                assert np.array_equal(got[c][:LENGTH], h[c][:LENGTH]), (k, is_spec)
+                assert np.max(np.abs(got[c] - h[c])[:LENGTH]) <= 1e-10 * np.max(np.abs(h[c][:LENGTH])), (k, is_spec)
             else:
                 assert is_spec, k
         # the handle goes on: a template of its own, and the batch
