@@ -1481,10 +1481,19 @@ __global__ void __launch_bounds__(kTileThreads, kMinB) k_waveform(BatchView bv) 
     else if constexpr (kCarry) return atomicAdd(bv.seg_ctl + kCtlQueue, 1);
     else return (long long)atomicAdd(bv.work_counter, 1ull);
   };
-  // direct tiles: an entry for each chunk of samples (the phase pass is done again for each; a few tiles a batch)
-  const long long items =
-      (kCarry && !kPhase) ? (long long)bv.seg_ctl[kCtlDirectCount] * kTileChunks : (long long)bv.total_tiles;
-  int part = 0;
+  // Direct tiles: first those without a table, an entry for each chunk of samples (the phase pass done again for each is
+  // little beside the chunk's recurrences); then the others, cut in four or two as long as all entries run at once.
+  // 2344 direct tiles: whole 0.55 ms for the launch, in quarters 0.88; 300 without a table: in quarters 0.48, whole 1.13.
+  int n_slow = 0, n_direct = 0, direct_parts = 1;
+  if constexpr (kCarry && !kPhase) {
+    n_slow = bv.seg_ctl[kCtlDirectSlow];
+    n_direct = bv.seg_ctl[kCtlDirectCount];
+    const int room = (int)gridDim.x;
+    direct_parts = 4 * n_direct <= room ? 4 : 2 * n_direct <= room ? 2 : 1;
+  }
+  static_assert(kTileChunks == 4, "a direct tile in four, two or one");
+  const long long items = (kCarry && !kPhase) ? 4ll * n_slow + (long long)n_direct * direct_parts : (long long)bv.total_tiles;
+  int part = 0, parts = 1;
   if (tid == 0) s_tile = fetch();
   __syncthreads();
   for (;;) {
@@ -1492,8 +1501,11 @@ __global__ void __launch_bounds__(kTileThreads, kMinB) k_waveform(BatchView bv) 
     __syncthreads();
     if (j >= items) break;
     if constexpr (kCarry && !kPhase) {
-      part = (int)(j % kTileChunks);
-      j = bv.direct_list[j / kTileChunks];
+      const bool slow = j < 4ll * n_slow;
+      const int e = (int)(slow ? j : j - 4ll * n_slow);
+      parts = slow ? 4 : direct_parts;
+      part = e % parts;
+      j = bv.direct_list[slow ? bv.total_tiles - 1 - e / 4 : e / parts];
     }
     if constexpr (kCarry && kPhase) {
       // a tile of polynomial segments: its record, head and coefficients by
@@ -2000,9 +2012,10 @@ __global__ void __launch_bounds__(kTileThreads, kMinB) k_waveform(BatchView bv) 
     const T *tab = kSplit ? reinterpret_cast<const T *>(tabF) : reinterpret_cast<const T *>(tabD);
     const int rs = kPre ? (int)s_prep.stride : (kSplit ? 2 * kRowF : kRowD);  // table row (FP32: pair row) stride
     constexpr bool kParts = kCarry && !kPhase;
-    static_assert(!kParts || kJoint == 1, "a direct entry is one chunk");
+    static_assert(!kParts || kJoint == 1, "a direct entry may be one chunk");
+    const int chunks = kParts ? kTileChunks / parts : kTileChunks;  // of this entry
 #pragma unroll 1
-    for (int g0 = kParts ? part : 0; g0 < (kParts ? part + 1 : kTileChunks); g0 += kJoint) {
+    for (int g0 = part * chunks; g0 < (part + 1) * chunks; g0 += kJoint) {
       SamplePrep<T> P[kJoint];
       T dl[kJoint], c1[kJoint], s1[kJoint], cD[kJoint], sD[kJoint], Sa[kJoint], Sb[kJoint], Sc[kJoint], d0[kJoint];
       double ph[kJoint];
@@ -2480,11 +2493,11 @@ void prepare_dense_launch() {
 // Launch one waveform-kernel instantiation as a persistent grid: every CTA
 // that fits on the device at once.
 template <typename K>
-void launch_persistent(K kernel, const BatchView &bv, int num_sms, size_t dyn, cudaStream_t stream) {
+void launch_persistent(K kernel, const BatchView &bv, int num_sms, size_t dyn, cudaStream_t stream, int entries = 1) {
   int resident = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, kTileThreads, dyn);
   resident = std::max(resident, 1);
-  const int grid = (int)std::min<int64_t>(bv.total_tiles, (int64_t)num_sms * resident);
+  const int grid = (int)std::min<int64_t>(bv.total_tiles * entries, (int64_t)num_sms * resident);  // entries of a tile
   kernel<<<grid, kTileThreads, dyn, stream>>>(bv);
 }
 
@@ -2526,8 +2539,8 @@ void launch_segments(const BatchView &bv, int num_sms, int rows, cudaStream_t st
   if (ev) cudaEventRecord(ev[1], stream);
   const int64_t tiles = bv.total_tiles, blocks = (tiles + kSegWarps - 1) / kSegWarps;
   k_tile_segments<kPhase><<<(unsigned)std::min<int64_t>(blocks, 3 * (int64_t)num_sms), kSegWarps * 32, 0, stream>>>(bv);
-  // a block a source, and one an SM for the direct tiles
-  const int carry = std::min(std::max(bv.nsrc, num_sms), 4096);
+  // a block a source, and two an SM (as many as fit) for the direct tiles
+  const int carry = std::min(std::max(bv.nsrc, 2 * num_sms), 4096);
   const int64_t table = (tiles * rows + kSegWarps * 32 - 1) / (kSegWarps * 32);
   k_tile_carries<<<(unsigned)(carry + table), kSegWarps * 32, 0, stream>>>(bv, carry, std::max(rows, 1));
 }
@@ -2580,7 +2593,7 @@ void launch_dense_t(const BatchView &bv, int num_sms, cudaStream_t stream, cudaE
       lg.total_tiles -= bv.small_tiles;
       launch_segments<false>(lg, num_sms, rows, stream, ev);
       if (ev) cudaEventRecord(ev[2], stream);
-      launch_persistent(k_waveform<false, 0, true, 1, 3, true>, lg, num_sms, dyn, fork_side(side, 1, stream));
+      launch_persistent(k_waveform<false, 0, true, 1, 3, true>, lg, num_sms, dyn, fork_side(side, 1, stream), kTileChunks);
       launch_seg_index(v, lg, num_sms, rows, stream, std::make_index_sequence<kNumVariants>{});
       sided = true;
     }

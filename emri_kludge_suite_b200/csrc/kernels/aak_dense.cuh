@@ -75,11 +75,14 @@ constexpr int64_t kSegSlotBytesPhase = 96 + 4 * 60 * 8;  // the phase product's:
 struct SegAgg {
   double f[3], b[3];
   double lastP;
-  int32_t hasP, needC;  // lastP was set in the tile; the sums wait for the clamped Phidot before the tile
+  double wC;            // needC: f[1] lacks wC times the clamped Phidot before the tile
+  int32_t hasP, needC;  // lastP is known from the tile itself; the one before the tile enters its sums
 };
-// words of seg_ctl, cleared before every launch: queue heads, direct tiles,
-// then per source its direct tiles, and per source those of them summed
-constexpr int kCtlQueue = 0, kCtlDirectQueue = 1, kCtlDirectCount = 2, kCtlSource = 4;
+static_assert(sizeof(SegAgg) == 72 && offsetof(SegAgg, hasP) == 64, "the two flags are one 8-byte load");
+// words of seg_ctl, cleared before every launch: queue heads, direct tiles
+// (with a Bessel table, without one), then per source its direct tiles, and per
+// source those of them summed
+constexpr int kCtlQueue = 0, kCtlDirectQueue = 1, kCtlDirectCount = 2, kCtlDirectSlow = 3, kCtlSource = 4;
 inline size_t seg_ctl_words(int nsrc) { return kCtlSource + 2 * (size_t)nsrc; }
 
 // Taylor-table rows: FP64 terms at most (K <= 10) and FP32 terms at most

@@ -91,60 +91,6 @@ __device__ __forceinline__ void lisa_response(const SourceDesc &d, double co, do
   F[3] = kHalfSqrt3 * (cosq1 * sin2phi * sin2psi - cosq * cos2phi * cos2psi);
 }
 
-// Phase increments of a tile sample by sample (one warp): the forward sums
-// with the clamped Phidot (Cin: its value before the tile where the raw one is
-// not positive) and the backward ones, as the phase pass of k_waveform forms
-// them, a rate's weights in its own and its neighbour's AB2 step taken together.
-__device__ void direct_aggregate(const BatchView &bv, const SourceDesc &d, const KnotWin &w, int start, int end, int lim,
-                                 const double rb[3], const double ra[3], double Cin, SegAgg &A) {
-  const int lane = threadIdx.x & 31;
-  double f[3] = {0, 0, 0}, b[3] = {0, 0, 0};
-  double P = (rb[1] > 0.0) ? rb[1] : Cin;  // clamped Phidot before the chunk
-  if (lane == 0 && start > d.i0 && start < lim) {  // the sample before the tile in its first step
-    f[0] -= .5 * rb[0];
-    f[1] -= .5 * P;
-    f[2] -= .5 * rb[2];
-  }
-  if (lane == 0 && end - 1 < d.i0 && end - 1 >= 1 && end - 1 < lim)  // the sample after it in its last backward step
-    for (int q = 0; q < 3; ++q) b[q] -= .5 * ra[q];
-  for (int s0 = start; s0 < lim; s0 += 32) {
-    const int i = s0 + lane;
-    const bool in = i < lim;
-    double r[3] = {0, 0, 0};
-    if (in) phase_rates(d, spline4w(bv, d, sample_time(d, i), w), r);
-    const bool fwd = in && i >= d.i0;
-    const unsigned pos = __ballot_sync(0xffffffffu, fwd && r[1] > 0.0);
-    const unsigned below = pos & (0xffffffffu >> (31 - lane));
-    const double up = __shfl_sync(0xffffffffu, r[1], below ? 31 - __clz(below) : 0);
-    const double Pi = below ? up : P;
-    if (fwd) {
-      const double wt = (i == d.i0 ? 1.0 : 1.5) - ((i + 1 < lim) ? .5 : 0.0);
-      f[0] = fma(wt, r[0], f[0]);
-      f[1] = fma(wt, Pi, f[1]);
-      f[2] = fma(wt, r[2], f[2]);
-    }
-    if (in && i <= d.i0) {
-      const double own = (i == d.i0) ? (i >= 1 ? 1.0 : 0.0) : (i >= 1 ? 1.5 : 0.0);
-      const double wt = own - ((i - 1 >= start && i - 1 >= 1) ? .5 : 0.0);
-      for (int q = 0; q < 3; ++q) b[q] = fma(wt, r[q], b[q]);
-    }
-    P = __shfl_sync(0xffffffffu, Pi, 31);  // lanes past lim repeat the last value
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-    for (int q = 0; q < 3; ++q) {
-      f[q] += __shfl_xor_sync(0xffffffffu, f[q], o);
-      b[q] += __shfl_xor_sync(0xffffffffu, b[q], o);
-    }
-  for (int q = 0; q < 3; ++q) {
-    A.f[q] = f[q] * d.dt;
-    A.b[q] = b[q] * d.dt;
-  }
-  A.lastP = P;
-  A.hasP = lim - 1 >= max(start, d.i0);
-}
-
 // Block-wide sum of N values of every thread (in every thread), for blocks of kSegWarps warps.
 template <int N>
 __device__ __forceinline__ void block_sum(double *v, double (*red)[8]) {
@@ -164,65 +110,137 @@ __device__ __forceinline__ void block_sum(double *v, double (*red)[8]) {
   }
 }
 
-// A direct tile by the whole CTA: the rates either side of the tile, and its
-// sums, which take every raw Phidot as it is; where one is not positive, one
-// warp sums the tile again with the clamp.
-__device__ void direct_tile(const BatchView &bv, const QueueItem &it, int lim, double (*red)[8]) {
-  const SourceDesc &d = bv.src[it.s];
-  const int tid = threadIdx.x;
-  const int start = it.lt * kTileSamples, end = min(start + kTileSamples, d.vlength);
-  KnotWin w{nullptr, nullptr, nullptr, nullptr, nullptr, it.k0, it.nk, 0, 0.0};
-  const double *kt = bv.knot_t + d.knot_offset;
-  const double span = kt[w.k0 + w.n - 1] - kt[w.k0];
-  w.inv_h = (span > 0.0) ? (double)(w.n - 1) / span : 0.0;
-  double v[7] = {0, 0, 0, 0, 0, 0, 0};  // forward sums, backward sums, non-positive raw Phidot
-  double rb[3] = {0, 0, 0}, ra[3] = {0, 0, 0};
-  const bool okb = start - 1 >= 0 && start - 1 < d.vlength;
-  if (okb) phase_rates(d, spline4w(bv, d, sample_time(d, start - 1), w), rb);
-  else rb[1] = -1.0;
-  if (end - 1 < d.i0 && end < d.vlength) phase_rates(d, spline4w(bv, d, sample_time(d, end), w), ra);
+// Shared scratch of a CTA that sums direct tiles and scans carries.
+struct CarryShared {
+  double red[8][8];
+  double last[kTileChunks * kSegWarps];  // per 32 samples, their last positive Phidot (-1: none)
+  double side[2][3];                     // the rates of the samples either side of the tile
+  double lastP;
+  int before[kSegWarps];
+  int is_last;
+};
+
+// Phase increments of the samples [start, lim) of a direct tile, by the whole
+// CTA: forward sums with the clamped Phidot (the last positive raw one; before
+// any in the tile that of the sample before, or C where haveC) and backward
+// ones, as the phase pass of k_waveform forms them, a rate's weights in its own
+// and its neighbour's AB2 step taken together.  Where the value before the tile
+// is not known, f[1] lacks C wC.
+//
+// Bound by latency: a sample's chain is a search, loads of the piece's knots and
+// the rates.  A thread's four samples, and the two either side, go through it
+// side by side.  Where the clamp acts over whole tiles (eight sources of 293 tiles
+// past their plunge) the phase product takes 0.23 ms; with one warp a tile, each
+// waiting for the tiles before it, 3.07.
+__device__ void direct_sums(const BatchView &bv, const SourceDesc &d, const KnotWin &w, int start, int end, int lim,
+                            bool haveC, double C, SegAgg &A, CarryShared &sh) {
+  const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
+  double r[kTileChunks + 1][3];
+#pragma unroll
+  for (int ch = 0; ch <= kTileChunks; ++ch) {  // the last one: warp 0 the sample before the tile, the others the one after
+    const int i = (ch < kTileChunks) ? min(start + ch * kTileThreads + tid, lim - 1) : (wp == 0) ? start - 1 : end;
+    phase_rates(d, spline4w(bv, d, sample_time(d, min(max(i, 0), d.vlength - 1)), w), r[ch]);
+  }
+  if (lane == 0 && wp < 2) {
+    const bool ok = (wp == 0) ? start >= 1 : (end - 1 < d.i0 && end < d.vlength);
+    for (int q = 0; q < 3; ++q) sh.side[wp][q] = ok ? r[kTileChunks][q] : (wp == 0 && q == 1) ? -1.0 : 0.0;
+  }
+  int clamp = 0;
 #pragma unroll
   for (int ch = 0; ch < kTileChunks; ++ch) {
     const int i = start + ch * kTileThreads + tid;
-    if (i >= lim) break;
-    double r[3];
-    phase_rates(d, spline4w(bv, d, sample_time(d, i), w), r);
-    if (i >= d.i0) {
+    if (i >= d.i0 && i < lim && !(r[ch][1] > 0.0)) clamp = 1;
+  }
+  clamp = __syncthreads_or(clamp);
+  const double *rb = sh.side[0], *ra = sh.side[1];
+  const double P0 = (rb[1] > 0.0) ? rb[1] : haveC ? C : -1.0;  // clamped Phidot before the tile (-1: not known)
+  double P[kTileChunks];  // clamped Phidot of the forward samples (-1: that of before the tile, not known)
+#pragma unroll
+  for (int ch = 0; ch < kTileChunks; ++ch) P[ch] = r[ch][1];
+  if (clamp) {
+    unsigned pos[kTileChunks];
+#pragma unroll
+    for (int ch = 0; ch < kTileChunks; ++ch) {
+      const int i = start + ch * kTileThreads + tid;
+      pos[ch] = __ballot_sync(0xffffffffu, i >= d.i0 && i < lim && r[ch][1] > 0.0);
+      const double x = __shfl_sync(0xffffffffu, r[ch][1], pos[ch] ? 31 - __clz(pos[ch]) : 0);
+      if (lane == 0) sh.last[ch * kSegWarps + wp] = pos[ch] ? x : -1.0;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int ch = 0; ch < kTileChunks; ++ch) {
+      const unsigned below = pos[ch] & (0xffffffffu >> (31 - lane));
+      const double up = __shfl_sync(0xffffffffu, r[ch][1], below ? 31 - __clz(below) : 0);
+      P[ch] = P0;
+      for (int k = ch * kSegWarps + wp - 1; k >= 0; --k)
+        if (sh.last[k] > 0.0) {
+          P[ch] = sh.last[k];
+          break;
+        }
+      if (below) P[ch] = up;
+    }
+  }
+  double v[7] = {0, 0, 0, 0, 0, 0, 0};  // forward sums, backward sums, weight of the Phidot before the tile
+#pragma unroll
+  for (int ch = 0; ch < kTileChunks; ++ch) {
+    const int i = start + ch * kTileThreads + tid;
+    if (i < lim && i >= d.i0) {
       const double wt = (i == d.i0 ? 1.0 : 1.5) - ((i + 1 < lim) ? .5 : 0.0);
-      for (int q = 0; q < 3; ++q) v[q] = fma(wt, r[q], v[q]);
-      if (!(r[1] > 0.0)) v[6] = 1.0;
+      v[0] = fma(wt, r[ch][0], v[0]);
+      if (clamp && P[ch] < 0.0) v[6] += wt;
+      else v[1] = fma(wt, P[ch], v[1]);
+      v[2] = fma(wt, r[ch][2], v[2]);
     }
-    if (i <= d.i0) {
+    if (i < lim && i <= d.i0) {
       const double wt = (i >= 1 ? (i == d.i0 ? 1.0 : 1.5) : 0.0) - ((i - 1 >= start && i - 1 >= 1) ? .5 : 0.0);
-      for (int q = 0; q < 3; ++q) v[3 + q] = fma(wt, r[q], v[3 + q]);
+      for (int q = 0; q < 3; ++q) v[3 + q] = fma(wt, r[ch][q], v[3 + q]);
     }
-    if (i == lim - 1) red[7][0] = r[1];
+    if (i == lim - 1) sh.lastP = P[ch];
   }
-  block_sum<7>(v, red);
+  block_sum<7>(v, sh.red);
+  if (start > d.i0 && start < lim) {
+    v[0] -= .5 * rb[0];
+    v[2] -= .5 * rb[2];
+    if (P0 < 0.0) v[6] -= .5;
+    else v[1] -= .5 * P0;
+  }
+  if (end - 1 < d.i0 && end - 1 >= max(start, 1) && end - 1 < lim)
+    for (int q = 0; q < 3; ++q) v[3 + q] -= .5 * ra[q];
+  for (int q = 0; q < 3; ++q) {
+    A.f[q] = v[q] * d.dt;
+    A.b[q] = v[3 + q] * d.dt;
+  }
+  A.wC = v[6] * d.dt;
+  A.lastP = sh.lastP;
+  A.hasP = lim - 1 >= max(start, d.i0) && !(clamp && sh.lastP < 0.0);
+  A.needC = P0 < 0.0;
+}
+
+// The window of tile g in global memory.
+__device__ __forceinline__ KnotWin tile_window(const BatchView &bv, const SourceDesc &d, int k0, int nk) {
+  KnotWin w{nullptr, nullptr, nullptr, nullptr, nullptr, k0, nk, 0, 0.0};
+  const double *kt = bv.knot_t + d.knot_offset;
+  const double span = kt[k0 + nk - 1] - kt[k0];
+  w.inv_h = (span > 0.0) ? (double)(nk - 1) / span : 0.0;
+  return w;
+}
+
+// A direct tile by the whole CTA: the rates either side of it, and its sums.
+__device__ void direct_tile(const BatchView &bv, const QueueItem &it, int lim, CarryShared &sh) {
+  const SourceDesc &d = bv.src[it.s];
+  const int start = it.lt * kTileSamples, end = min(start + kTileSamples, d.vlength);
   const int head = (d.i0 <= 0) ? 0 : min(d.i0 / kTileSamples, d.n_tiles - 1);
-  SegAgg A{};
-  A.needC = it.lt > head && !(rb[1] > 0.0);
-  if (v[6] != 0.0 || A.needC) {
-    if (tid < 32) direct_aggregate(bv, d, w, start, end, lim, rb, ra, 0.0, A);
-  } else {
-    for (int q = 0; q < 3; ++q) {
-      const double before = (start > d.i0 && start < lim) ? .5 * rb[q] : 0.0;
-      const double after = (end - 1 < d.i0 && end - 1 >= 1 && end - 1 < lim) ? .5 * ra[q] : 0.0;
-      A.f[q] = (v[q] - before) * d.dt;
-      A.b[q] = (v[3 + q] - after) * d.dt;
-    }
-    A.lastP = red[7][0];
-    A.hasP = lim - 1 >= max(start, d.i0);
-  }
-  if (tid == 0) {
+  SegAgg A;
+  direct_sums(bv, d, tile_window(bv, d, it.k0, it.nk), start, end, lim, it.lt <= head, 0.0, A, sh);
+  if (threadIdx.x == 0) {
     TilePrep &P = bv.tile_prep[it.g];
     for (int q = 0; q < 3; ++q) {
-      P.rb[q] = rb[q];
-      P.ra[q] = ra[q];
+      P.rb[q] = sh.side[0][q];
+      P.ra[q] = sh.side[1][q];
     }
     bv.tile_agg[it.g] = A;
   }
-  __syncthreads();  // red is free again
+  __syncthreads();  // sh is free again
 }
 
 // The phase at a tile's head modulo 2 pi, x0 + (h, l) as a double-double: the
@@ -237,7 +255,7 @@ __device__ __forceinline__ void reduced_base(double x0, double &h, double &l) {
 }
 
 // The phases that GenPhase keeps after the plunge buffer, those of sample
-// i_plunge (AAKPhase.cc:253-257), into the source's slot of frozen (one warp,
+// i_plunge (AAKPhase.cc:253-257), into the source's slot of frozen (the whole CTA,
 // after the carries).  first_frozen: the first sample that takes them.
 __device__ __forceinline__ long long first_frozen(const SourceDesc &d) {
   if (d.status != 0 || d.i_plunge < 0 || d.i_plunge >= d.vlength) return (long long)d.vlength;
@@ -248,11 +266,10 @@ __device__ __forceinline__ bool is_frozen(const SourceDesc &d, int i) {
   const long long first = first_frozen(d);
   return first < d.vlength && (i >= first || i == d.i_plunge);
 }
-__device__ void frozen_phases(const BatchView &bv, int s, const SourceDesc &d) {
+__device__ void frozen_phases(const BatchView &bv, int s, const SourceDesc &d, CarryShared &sh) {
   if (first_frozen(d) >= d.vlength) return;
-  const int lane = threadIdx.x & 31, i = d.i_plunge, lt = i / kTileSamples;
+  const int i = d.i_plunge, lt = i / kTileSamples;
   const int64_t g = bv.tile_start[s] + lt;
-  __syncwarp();
   const TileHead *H = tile_head(bv, g);
   const int mode = __ldcg(&H->mode);
   double v[3] = {0, 0, 0};
@@ -267,27 +284,19 @@ __device__ void frozen_phases(const BatchView &bv, int s, const SourceDesc &d) {
         v[q] = (i < d.i0) ? -p : p;
       }
     } else {
-      KnotWin w{nullptr, nullptr, nullptr, nullptr, nullptr, bv.tile_knot[2 * g], bv.tile_knot[2 * g + 1], 0, 0.0};
-      const double *kt = bv.knot_t + d.knot_offset;
-      const double span = kt[w.k0 + w.n - 1] - kt[w.k0];
-      w.inv_h = (span > 0.0) ? (double)(w.n - 1) / span : 0.0;
+      const KnotWin w = tile_window(bv, d, bv.tile_knot[2 * g], bv.tile_knot[2 * g + 1]);
       const int start = lt * kTileSamples, end = min(start + kTileSamples, d.vlength);
-      double rb[3], ra[3];
-      for (int q = 0; q < 3; ++q) {
-        rb[q] = __ldcg(&bv.tile_prep[g].rb[q]);
-        ra[q] = __ldcg(&bv.tile_prep[g].ra[q]);
-      }
-      SegAgg A{};
+      SegAgg A;
       if (i > d.i0) {  // the forward sum of the tile's samples before i
-        direct_aggregate(bv, d, w, start, i, i, rb, ra, __ldcg(&H->C), A);
+        direct_sums(bv, d, w, start, end, i, true, __ldcg(&H->C), A, sh);
         for (int q = 0; q < 3; ++q) v[q] = A.f[q];
       } else {  // the backward sum of those after i
-        direct_aggregate(bv, d, w, i + 1, end, end, rb, ra, 0.0, A);
+        direct_sums(bv, d, w, i + 1, end, end, true, 0.0, A, sh);
         for (int q = 0; q < 3; ++q) v[q] = -A.b[q];
       }
     }
   }
-  if (lane == 0) {
+  if (threadIdx.x == 0) {
     const double X0[3] = {d.gim0, d.Phi0, d.alp0};
     for (int q = 0; q < 3; ++q)
       bv.frozen[3 * s + q] = (i == d.i0) ? X0[q] : X0[q] + (__ldcg(&H->hi[q]) + (__ldcg(&H->lo[q]) + v[q]));
@@ -296,62 +305,67 @@ __device__ void frozen_phases(const BatchView &bv, int s, const SourceDesc &d) {
 
 // The carries of one source's tiles (the whole CTA): every tile's aggregates of the
 // tiles between it and the head, in double-double, forward and backward; a
-// forward tile whose Phidot clamp reaches back past its first sample is summed
-// again with the value that the tiles before it leave.  The waveform gets the
-// phases at the tile's head modulo 2 pi, the phase product the signed sums.
-__device__ void scan_source(const BatchView &bv, int s, double (*red)[8]) {
+// forward tile whose Phidot clamp reaches back past its first sample gets the
+// value that the tiles before it leave, the last one known, times its weight.
+// The waveform gets the phases at the tile's head modulo 2 pi, the phase product
+// the signed sums.
+__device__ void scan_source(const BatchView &bv, int s, CarryShared &sh) {
   const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
   const SourceDesc &d = bv.src[s];
   const int64_t t0 = bv.tile_start[s];
   const int T = d.n_tiles, i0 = d.i0;
   const int head = (i0 <= 0) ? 0 : min(i0 / kTileSamples, T - 1);
-  SegAgg *A = bv.tile_agg + t0;
-  // tiles that wait for the clamped Phidot, in order (one warp)
-  for (int k0 = head + 1; wp == 0 && k0 < T; k0 += 32) {
-    const int k = k0 + lane;
-    unsigned m = __ballot_sync(0xffffffffu, k < T && __ldcg(&A[k].needC) != 0);
-    for (; m; m &= m - 1) {
-      const int t = k0 + __ffs(m) - 1;
-      double C = 0.0;
-      for (int q = t - 1; q >= head; --q)
-        if (__ldcg(&A[q].hasP)) {
-          C = __ldcg(&A[q].lastP);
-          break;
-        }
-      const int64_t g = t0 + t;
-      KnotWin w{nullptr, nullptr, nullptr, nullptr, nullptr, bv.tile_knot[2 * g], bv.tile_knot[2 * g + 1], 0, 0.0};
-      const double *kt = bv.knot_t + d.knot_offset;
-      const double span = kt[w.k0 + w.n - 1] - kt[w.k0];
-      w.inv_h = (span > 0.0) ? (double)(w.n - 1) / span : 0.0;
-      const int start = t * kTileSamples, end = min(start + kTileSamples, d.vlength);
-      const int lim = bv.phase_out ? end : min(end, n_eff(d));
-      double rb[3], ra[3];  // written in this launch
-      for (int q = 0; q < 3; ++q) {
-        rb[q] = __ldcg(&bv.tile_prep[g].rb[q]);
-        ra[q] = __ldcg(&bv.tile_prep[g].ra[q]);
-      }
-      SegAgg R{};
-      direct_aggregate(bv, d, w, start, end, lim, rb, ra, C, R);
-      if (lane == 0) {
-        A[t] = R;
-        tile_head(bv, g)->C = C;
-        __threadfence();
-      }
-      __syncwarp();
-    }
-  }
+  const SegAgg *A = bv.tile_agg + t0;  // written in this launch by other CTAs
   __syncthreads();
 #pragma unroll 1
   for (int dir = 1; dir >= -1; dir -= 2) {
     const int n = (dir > 0) ? T - head : head + 1;  // tiles of the chain, the head first
     if (dir < 0 && n == 1) break;
     const int per = (n + kSegWarps * 32 - 1) / (kSegWarps * 32), k0 = min(tid * per, n), k1 = min(k0 + per, n);
-    double hi[3] = {0, 0, 0}, lo[3] = {0, 0, 0};
+    bool clamp = false;
+    double C0 = 0.0;  // the clamped Phidot that the tiles before the thread's leave
+    if (dir > 0) {
+      bool need = false;
+      int last = -1;  // the thread's last tile that leaves one
 #pragma unroll 8
-    for (int k = k0; k < k1; ++k) {
-      const double *x = (dir > 0) ? A[head + k].f : A[head - k].b;
+      for (int k = k0; k < k1; ++k) {
+        const int2 f = __ldcg(reinterpret_cast<const int2 *>(&A[head + k].hasP));
+        if (f.x) last = k;
+        need = need || f.y;
+      }
+      clamp = __syncthreads_or(need);
+      if (clamp) {
 #pragma unroll
-      for (int q = 0; q < 3; ++q) dd_add(hi[q], lo[q], __ldcg(x + q));
+        for (int o = 1; o < 32; o <<= 1) {
+          const int b = __shfl_up_sync(0xffffffffu, last, o);
+          if (lane >= o) last = max(last, b);
+        }
+        if (lane == 31) sh.before[wp] = last;
+        int before = __shfl_up_sync(0xffffffffu, last, 1);
+        if (lane == 0) before = -1;
+        __syncthreads();
+        for (int k = 0; k < wp; ++k) before = max(before, sh.before[k]);
+        if (before >= 0) C0 = __ldcg(&A[head + before].lastP);
+      }
+    }
+    double C = C0;
+    // the increments of tile k of the chain, C the clamped Phidot before it and then after it
+    const auto increments = [&](int k, double x[3]) {
+      const SegAgg &a = A[(dir > 0) ? head + k : head - k];
+#pragma unroll
+      for (int q = 0; q < 3; ++q) x[q] = __ldcg(((dir > 0) ? a.f : a.b) + q);
+      if (clamp) {
+        if (__ldcg(&a.needC)) x[1] = fma(C, __ldcg(&a.wC), x[1]);
+        if (__ldcg(&a.hasP)) C = __ldcg(&a.lastP);
+      }
+    };
+    double hi[3] = {0, 0, 0}, lo[3] = {0, 0, 0};
+#pragma unroll 4
+    for (int k = k0; k < k1; ++k) {
+      double x[3];
+      increments(k, x);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) dd_add(hi[q], lo[q], x[q]);
     }
     // exclusive scan of the threads' sums: inside the warp, then over the warps before
     double ph[3], pl[3];
@@ -368,23 +382,24 @@ __device__ void scan_source(const BatchView &bv, int s, double (*red)[8]) {
       pl[q] = __shfl_up_sync(0xffffffffu, l, 1);
       if (lane == 0) ph[q] = pl[q] = 0.0;
       if (lane == 31) {
-        red[q][wp] = h;
-        red[3 + q][wp] = l;
+        sh.red[q][wp] = h;
+        sh.red[3 + q][wp] = l;
       }
     }
     __syncthreads();
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
       double h = 0.0, l = 0.0;
-      for (int k = 0; k < wp; ++k) dd_add_dd(h, l, red[q][k], red[3 + q][k]);
+      for (int k = 0; k < wp; ++k) dd_add_dd(h, l, sh.red[q][k], sh.red[3 + q][k]);
       dd_add_dd(h, l, ph[q], pl[q]);
       ph[q] = h;
       pl[q] = l;
     }
-#pragma unroll 8
+    C = C0;
+#pragma unroll 4
     for (int k = k0; k < k1; ++k) {
+      TileHead *H = tile_head(bv, t0 + head + dir * k);
       if (dir > 0 || k > 0) {  // the head's own, of sum 0, is set once
-        TileHead *H = tile_head(bv, t0 + head + dir * k);
         const double X0[3] = {d.gim0, d.Phi0, d.alp0};
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
@@ -393,15 +408,17 @@ __device__ void scan_source(const BatchView &bv, int s, double (*red)[8]) {
           H->hi[q] = h;
           H->lo[q] = l;
         }
+        if (clamp) H->C = C;
       }
-      const double *x = (dir > 0) ? A[head + k].f : A[head - k].b;
+      double x[3];
+      increments(k, x);
 #pragma unroll
-      for (int q = 0; q < 3; ++q) dd_add(ph[q], pl[q], __ldcg(x + q));
+      for (int q = 0; q < 3; ++q) dd_add(ph[q], pl[q], x[q]);
     }
   }
   if (bv.phase_out) {
     __syncthreads();
-    if (tid < 32) frozen_phases(bv, s, d);
+    frozen_phases(bv, s, d, sh);
   }
 }
 
@@ -577,12 +594,7 @@ __global__ void __launch_bounds__(kSegWarps * 32, 3) k_tile_segments(BatchView b
       }
       const bool fail = __any_sync(0xffffffffu, bad7);
       mode = fail ? 0 : (__any_sync(0xffffffffu, bad4) ? 7 : 4);
-      if (mode == 0) {
-        if (lane == 0) {
-          bv.direct_list[atomicAdd(bv.seg_ctl + kCtlDirectCount, 1)] = (int32_t)jq;
-          atomicAdd(bv.seg_ctl + kCtlSource + it.s, 1);
-        }
-      } else {
+      if (mode != 0) {
         double tot[3];
         if (mode == 4) {
           phase_segments<4, SD4>(tb, s_dv[wp], v, out, nseg, bwd, dir == 0, d.dt, tot);
@@ -619,6 +631,11 @@ __global__ void __launch_bounds__(kSegWarps * 32, 3) k_tile_segments(BatchView b
       }
     }
     if (lane == 0) {
+      if (mode == 0) {  // direct tiles from the list's front; those whose sums have no table, and take longest, from its end
+        if (P.K == 0) bv.direct_list[bv.total_tiles - 1 - atomicAdd(bv.seg_ctl + kCtlDirectSlow, 1)] = (int32_t)jq;
+        else bv.direct_list[atomicAdd(bv.seg_ctl + kCtlDirectCount, 1)] = (int32_t)jq;
+        atomicAdd(bv.seg_ctl + kCtlSource + it.s, 1);
+      }
       bv.tile_prep[it.g] = P;
       if (mode != 0) bv.tile_agg[it.g] = A;
       H->C = 0.0;
@@ -638,28 +655,27 @@ __global__ void __launch_bounds__(kSegWarps * 32, 3) k_tile_segments(BatchView b
 // at once, another by the CTA that finishes its last one); the other blocks
 // build the tiles' Taylor tables, one thread a (tile,
 // harmonic).  The small sources are not the segments'.
-__global__ void __launch_bounds__(kSegWarps * 32) k_tile_carries(BatchView bv, int carry_blocks, int rows) {
-  __shared__ double s_red[8][8];
-  __shared__ int s_last;
+__global__ void __launch_bounds__(kSegWarps * 32, 2) k_tile_carries(BatchView bv, int carry_blocks, int rows) {
+  __shared__ CarryShared sh;
   if ((int)blockIdx.x >= carry_blocks) {
     table_row<false>(bv, rows, (int64_t)(blockIdx.x - carry_blocks) * blockDim.x + threadIdx.x);
     return;
   }
   for (int s = blockIdx.x; s < bv.nsrc; s += carry_blocks)
-    if (bv.seg_ctl[kCtlSource + s] == 0 && bv.src[s].n_tiles > kSmallTiles) scan_source(bv, s, s_red);
-  const int n = bv.seg_ctl[kCtlDirectCount];
-  for (int m = blockIdx.x; m < n; m += carry_blocks) {
-    const QueueItem it = bv.queue[bv.direct_list[m]];
+    if (bv.seg_ctl[kCtlSource + s] == 0 && bv.src[s].n_tiles > kSmallTiles) scan_source(bv, s, sh);
+  const int n = bv.seg_ctl[kCtlDirectCount], slow = bv.seg_ctl[kCtlDirectSlow];
+  for (int m = blockIdx.x; m < n + slow; m += carry_blocks) {
+    const QueueItem it = bv.queue[bv.direct_list[m < n ? m : bv.total_tiles - 1 - (m - n)]];
     const SourceDesc &d = bv.src[it.s];
     const int end = min((it.lt + 1) * kTileSamples, d.vlength);
-    direct_tile(bv, it, bv.phase_out ? end : min(end, n_eff(d)), s_red);
+    direct_tile(bv, it, bv.phase_out ? end : min(end, n_eff(d)), sh);
     if (threadIdx.x == 0) {
       __threadfence();
-      s_last = atomicAdd(bv.seg_ctl + kCtlSource + bv.nsrc + it.s, 1) == bv.seg_ctl[kCtlSource + it.s] - 1;
+      sh.is_last = atomicAdd(bv.seg_ctl + kCtlSource + bv.nsrc + it.s, 1) == bv.seg_ctl[kCtlSource + it.s] - 1;
       __threadfence();
     }
     __syncthreads();
-    if (s_last) scan_source(bv, it.s, s_red);
+    if (sh.is_last) scan_source(bv, it.s, sh);
     __syncthreads();
   }
 }
