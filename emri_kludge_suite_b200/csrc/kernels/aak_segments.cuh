@@ -15,8 +15,9 @@
 // k_tile_segments (one warp a tile, a lane a node) tests the cut by the
 // Chebyshev coefficients it drops: they must lie at the rounding noise of the
 // node values (kSegTol).  A tile that fails -- a frozen or clamped trajectory,
-// the end of a plunge, an irregular sample time -- is marked direct and goes
-// through k_waveform's per-sample phase pass with its carry given.
+// the end of a plunge, an irregular sample time, either end of the source -- is
+// marked direct and goes through k_waveform's per-sample phase pass with its
+// carry given.
 #pragma once
 
 // quantities sampled at the nodes: gamma~dot, Phidot, alphadot, then (waveform)
@@ -565,7 +566,10 @@ __global__ void __launch_bounds__(kSegWarps * 32, 3) k_tile_segments(BatchView b
       }
       // a forward tile's Phidot is positive throughout, and its sample times are evenly spaced
       const bool even = (start > 0 || (i0 == 0 && d.t_first == 0.0)) && (dir != 0 || (i0 == 0 && start == 0));
-      bool bad7 = !even || (used && dir >= 0 && !(v[1] > 0.0)), bad4 = false;
+      // The source's first and last samples lie outside the nodes, where a boundary layer of the natural spline shorter
+      // than two samples (knots closer than the samples: a fast inspiral) would go unseen: their tiles are direct.
+      const bool ends = it.lt == 0 || it.lt == T - 1;
+      bool bad7 = !even || ends || (used && dir >= 0 && !(v[1] > 0.0)), bad4 = false;
 #pragma unroll
       for (int q = 0; q < NQ; ++q) {  // v becomes the value at the segment's reference node
         const double r = __shfl_sync(0xffffffffu, v[q], (lane & 24) | kSegRef);

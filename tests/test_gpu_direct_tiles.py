@@ -101,9 +101,10 @@ def test_whole_and_quartered_entries_give_the_same_samples():
         assert np.array_equal(h[:, s * n:(s + 1) * n], h1) and np.array_equal(r[:, s * n:(s + 1) * n], r1)
 
 
-@pytest.mark.parametrize("k", [7])
+# k = 2: knots closer than the samples, so that only sample 0 is in the spline's boundary layer
+@pytest.mark.parametrize("k", [2, 7])
 def test_phases_past_a_plunge(k):
-    """A plunge at sample 88272 of 100000, and the tiles past it."""
+    """Plunges at sample 85679 and 88272 of 100000, and the tiles past them."""
     pars = _fast(k)
     _, maps, _, rows = _run([pars], [3])
     _check_phase(pars, maps[0], rows)
