@@ -123,28 +123,31 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float v[16]) {
 }
 
 // ------------------------------------------------------------------ activation
-// Sigmoids of a pair.  Training (kFast false): the library's exp and an IEEE
-// division, so that the activations and their BF16 roundings do not move.
-// Inference: one exponential each (ex2.approx of the FP32 product, 2 ulp) and
-// one reciprocal for the two, 1 / a = b / (a b); the argument is bounded at
-// 2^60, so that the product of the two stays finite: below z = -41 the sigmoid
-// is 1e-18, not less.
+// Sigmoids of a pair by the library's exp and an IEEE division (training, whose
+// activations and BF16 roundings do not move), and silu = z times the sigmoid.
+__device__ __forceinline__ float2 sigm2(float2 z) {
+  return make_float2(1.0f / (1.0f + expf(-z.x)), 1.0f / (1.0f + expf(-z.y)));
+}
+// silu of a pair for inference: one exponential each (ex2.approx of the FP32
+// product, 2 ulp) and one reciprocal for the two, 1 / a = b / (a b).  The
+// exponential is bounded at 2^90, so that a sigmoid is at least 8e-28 and silu
+// within 1e-7 of 0 down to z = -1e20; where a b overflows, the reciprocal and
+// both sigmoids are 0, the larger of them no more than 2^-38 before.  (Bounding z
+// itself, exact to -inf, costs 3 %: the pairs of values are packed again.)
 __device__ __forceinline__ float ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
 template <bool kFast>
-__device__ __forceinline__ float2 sigm2(float2 z) {
-  if constexpr (!kFast) return make_float2(1.0f / (1.0f + expf(-z.x)), 1.0f / (1.0f + expf(-z.y)));
+__device__ __forceinline__ float2 silu2(float2 z) {
+  if constexpr (!kFast) return __fmul2_rn(z, sigm2(z));
   const float2 t = __fmul2_rn(z, make_float2(-1.44269504f, -1.44269504f));
-  const float a = 1.0f + ex2(fminf(t.x, 60.0f)), b = 1.0f + ex2(fminf(t.y, 60.0f));
+  const float a = 1.0f + ex2(fminf(t.x, 90.0f)), b = 1.0f + ex2(fminf(t.y, 90.0f));
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a * b));
-  return __fmul2_rn(make_float2(r, r), make_float2(b, a));
+  return __fmul2_rn(z, __fmul2_rn(make_float2(r, r), make_float2(b, a)));
 }
-template <bool kFast>
-__device__ __forceinline__ float2 silu2(float2 z) { return __fmul2_rn(z, sigm2<kFast>(z)); }
 // silu' = s (1 + z (1 - s))
 __device__ __forceinline__ float2 dsilu2(float2 z, float2 s) {
   const float2 one = make_float2(1.0f, 1.0f);
@@ -269,7 +272,7 @@ struct FwdSmem {
 };
 
 // The activations cost two special-function operations a value with the
-// library's exp and division beside them; with sigm2 they cost one and a half,
+// library's exp and division beside them; with silu2 they cost one and a half,
 // and sixteen warps an SM on four tiles keep that pipe busy while a tile waits
 // for its product.  Bound by that pipe (69 % of its rate): 1e6 points 1027 us on
 // 128-thread CTAs, two an SM, 199 us here.
@@ -512,7 +515,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gradients(DeviceModel md, const
         for (int j = 0; j < 8; ++j) {
           const float4 u = S.L.w4[o0 + 16 * c + 2 * j], w = S.L.w4[o0 + 16 * c + 2 * j + 1];
           const float2 z = __fadd2_rn(make_float2(v[2 * j], v[2 * j + 1]), make_float2(u.w, w.w));
-          const float2 sg = sigm2<false>(z);
+          const float2 sg = sigm2(z);
           ds[8 * c + j] = dsilu2(z, sg);
           q[j] = pack_bf16(__fmul2_rn(z, sg));
           const float a0 = __uint_as_float(q[j] << 16), a1 = __uint_as_float(q[j] & 0xFFFF0000u);
@@ -612,7 +615,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gradients(DeviceModel md, const
       for (int j = 0; j < 8; ++j) {
         const int o = o0 + 16 * c + 2 * j;
         const float2 zz = __fadd2_rn(make_float2(z[2 * j], z[2 * j + 1]), make_float2(S.L.b2[o], S.L.b2[o + 1]));
-        q[j] = valid ? pack_bf16(__fmul2_rn(make_float2(da[2 * j], da[2 * j + 1]), dsilu2(zz, sigm2<false>(zz)))) : 0u;
+        q[j] = valid ? pack_bf16(__fmul2_rn(make_float2(da[2 * j], da[2 * j + 1]), dsilu2(zz, sigm2(zz)))) : 0u;
       }
       put_row8(S.D, t, o0 + 16 * c, q);
       put_row8(S.D, t, o0 + 16 * c + 8, q + 4);
@@ -649,7 +652,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gradients(DeviceModel md, const
       for (int j = 0; j < 8; ++j) {
         const int o = o0 + 16 * c + 2 * j;
         const float2 z = layer1_pair(S.L.w1[o / 2], f);
-        const float2 d = __fmul2_rn(__fmul2_rn(make_float2(v[2 * j], v[2 * j + 1]), dsilu2(z, sigm2<false>(z))), on2);
+        const float2 d = __fmul2_rn(__fmul2_rn(make_float2(v[2 * j], v[2 * j + 1]), dsilu2(z, sigm2(z))), on2);
         scr[o * kScrStride + t] = d.x;
         scr[(o + 1) * kScrStride + t] = d.y;
       }
