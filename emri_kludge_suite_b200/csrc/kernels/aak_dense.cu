@@ -1483,7 +1483,8 @@ __global__ void __launch_bounds__(kTileThreads, kMinB) k_waveform(BatchView bv) 
   };
   // Direct tiles: first those without a table, an entry for each chunk of samples (the phase pass done again for each is
   // little beside the chunk's recurrences); then the others, cut in four or two as long as all entries run at once.
-  // 2344 direct tiles: whole 0.55 ms for the launch, in quarters 0.88; 300 without a table: in quarters 0.48, whole 1.13.
+  // 2344 direct tiles: whole 0.55 ms for the launch, in quarters 0.88; 64 beside 1984 of segments: whole 0.29, in
+  // quarters 0.26; 300 without a table: whole 1.13, in quarters 0.48.
   int n_slow = 0, n_direct = 0, direct_parts = 1;
   if constexpr (kCarry && !kPhase) {
     n_slow = bv.seg_ctl[kCtlDirectSlow];
@@ -2537,12 +2538,15 @@ template <bool kPhase>
 void launch_segments(const BatchView &bv, int num_sms, int rows, cudaStream_t stream, cudaEvent_t *ev) {
   cudaMemsetAsync(bv.seg_ctl, 0, seg_ctl_words(bv.nsrc) * sizeof(int32_t), stream);
   if (ev) cudaEventRecord(ev[1], stream);
-  const int64_t tiles = bv.total_tiles, blocks = (tiles + kSegWarps - 1) / kSegWarps;
-  k_tile_segments<kPhase><<<(unsigned)std::min<int64_t>(blocks, 3 * (int64_t)num_sms), kSegWarps * 32, 0, stream>>>(bv);
-  // a block a source, and two an SM (as many as fit) for the direct tiles
-  const int carry = std::min(std::max(bv.nsrc, 2 * num_sms), 4096);
+  const int64_t tiles = bv.total_tiles;
+  // a warp a tile: few of them spread over the SMs, whose FP64 units eight warps share
+  const int warps = (int)std::min<int64_t>(kSegWarps, std::max<int64_t>(1, (tiles + num_sms - 1) / num_sms));
+  k_tile_segments<kPhase><<<(unsigned)std::min<int64_t>((tiles + warps - 1) / warps, 3 * (int64_t)num_sms), warps * 32, 0, stream>>>(bv);
+  // a block a source and one an SM for the direct tiles, and after the tables one more an SM (two fit)
+  const int carry = std::min(std::max(bv.nsrc, num_sms), 4096);
   const int64_t table = (tiles * rows + kSegWarps * 32 - 1) / (kSegWarps * 32);
-  k_tile_carries<<<(unsigned)(carry + table), kSegWarps * 32, 0, stream>>>(bv, carry, std::max(rows, 1));
+  const int more = tiles > carry ? num_sms : 0;
+  k_tile_carries<<<(unsigned)(carry + table + more), kSegWarps * 32, 0, stream>>>(bv, carry, (int)table, std::max(rows, 1));
 }
 
 // Let work queued on the side stream from here on follow what is on `stream`.
