@@ -1268,14 +1268,16 @@ __device__ __forceinline__ void finish(const SamplePrep<T> &P, T Sa, T Sb, T Sc,
 
 
 // ------------------------------------------------------------------ tile pre-pass
-// The per-tile work of the waveform kernel that does not depend on the phase
-// scan, done for every tile of the batch before it: (1) k_tile_params, one
-// thread per tile: e at the tile's first, middle and last output samples
-// (the Taylor-table centre e_c and term count K), and the raw rates of the
-// samples just before and after the tile; (2) k_tile_table, one thread per
-// (tile, harmonic): the tile's Taylor row of that harmonic.  Both evaluate
-// the spline with the same window, search and arithmetic as the waveform
-// kernel, so the values equal the ones it would compute itself.
+// The per-tile work of the split waveform kernel and of the small sources' phase
+// pass that does not depend on the phase scan, done for every tile before them:
+// (1) k_tile_params, one thread per tile: the raw rates of the samples just
+// before and after the tile and, for the waveform, e at the tile's first, middle
+// and last output samples (the Taylor-table centre e_c and term count K); (2)
+// k_tile_table, one thread per (tile, harmonic): the tile's Taylor row of that
+// harmonic.  Both evaluate the spline with the same window, search and
+// arithmetic as those kernels, so the values equal the ones they would compute
+// themselves.  (FP64 waveforms: the segments' pre-pass, or everything inside the
+// tiles.)
 template <bool kSplit>
 __global__ void __launch_bounds__(128) k_tile_params(BatchView bv) {
   const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -1319,7 +1321,7 @@ __global__ void __launch_bounds__(128) k_tile_params(BatchView bv) {
       P.ra[2] = r[2];
     }
   }
-  if (d.status == 0 && lim > start) {  // lim <= end: the window above is set
+  if constexpr (kSplit) if (d.status == 0 && lim > start) {  // lim <= end: the window above is set
     const double e0 = spline4w(bv, d, sample_time(d, start), w).e;
     const double em = spline4w(bv, d, sample_time(d, (start + lim - 1) / 2), w).e;
     const double e1 = spline4w(bv, d, sample_time(d, lim - 1), w).e;
@@ -1330,12 +1332,12 @@ __global__ void __launch_bounds__(128) k_tile_params(BatchView bv) {
       const double de = fmax(fabs(e0 - ec), fabs(e1 - ec));
       if (ec > 1e-6) {
         const double q = d.nmodes * (1.25 * de + 1e-15);  // bounds n |e - e_c| over the tile
-        K = kSplit ? taylor_terms_fp32(q, d.nmodes) : taylor_terms_fp64(q, d.nmodes);
+        K = taylor_terms_fp32(q, d.nmodes);
       }
     }
     P.ec = ec;
     P.K = (int16_t)K;
-    P.stride = (int16_t)(K > 0 ? (kSplit ? row_stride<float>(K) : row_stride<double>(K)) : 0);
+    P.stride = (int16_t)(K > 0 ? row_stride<float>(K) : 0);
   }
   bv.tile_prep[g] = P;
 }
@@ -1357,9 +1359,8 @@ __device__ __forceinline__ void table_row(const BatchView &bv, int rows, int64_t
   T *tab = reinterpret_cast<T *>(static_cast<unsigned char *>(bv.tile_tab) + g * bv.tab_slot);
   build_taylor_row<T>(tab, P.stride, n, d.nmodes, P.ec, K, (n <= d.nmodes) ? bv.bessel_start[d.bessel_offset + n - 1] : 0);
 }
-template <bool kSplit>
 __global__ void __launch_bounds__(128) k_tile_table(BatchView bv, int rows) {
-  table_row<kSplit>(bv, rows, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
+  table_row<true>(bv, rows, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
 
 #include "aak_segments.cuh"
@@ -2456,10 +2457,6 @@ void launch_plain_waveform(const SourceDesc *src, int s, int vlength, const doub
   k_plain_waveform<<<(vlength + 255) / 256, 256, 0, stream>>>(src, s, traj, traj_stride, hI, hII);
 }
 
-void launch_dense_fp64(const BatchView &bv, int num_sms, cudaStream_t stream, cudaEvent_t *ev) {
-  launch_dense(bv, num_sms, stream, ev, 0);
-}
-
 template <size_t... I>
 void set_variant_smem(int bytes, int seg_bytes, std::index_sequence<I...>) {
   (cudaFuncSetAttribute(k_wave_split<std::max(wave_variant(true, (int)I).joint, 1), wave_variant(true, (int)I).min_blocks>,
@@ -2610,7 +2607,7 @@ void launch_dense_t(const BatchView &bv, int num_sms, cudaStream_t stream, cudaE
   if (ev) cudaEventRecord(ev[1], stream);
   if (kSplit && pre) {
     k_tile_params<true><<<(unsigned)((tiles + 127) / 128), 128, 0, stream>>>(bv);
-    k_tile_table<true><<<(unsigned)((tiles * rows + 127) / 128), 128, 0, stream>>>(bv, rows);
+    k_tile_table<<<(unsigned)((tiles * rows + 127) / 128), 128, 0, stream>>>(bv, rows);
   }
   if (ev) cudaEventRecord(ev[2], stream);
   if (kSplit && pre) launch_split_index(v, bv, num_sms, dyn, stream, std::make_index_sequence<kNumVariants>{});

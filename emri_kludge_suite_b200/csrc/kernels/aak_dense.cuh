@@ -211,7 +211,6 @@ struct DenseSide {
   cudaStream_t stream = nullptr;
   cudaEvent_t fork[2] = {nullptr, nullptr}, join = nullptr;
 };
-void launch_dense_fp64(const BatchView &bv, int num_sms, cudaStream_t stream, cudaEvent_t *ev);
 // precision 0: FP64 throughout; 1: split (FP64 phases and reductions, FP32
 // geometry, response, Bessel evaluation and harmonic recurrence).
 void launch_dense(const BatchView &bv, int num_sms, cudaStream_t stream, cudaEvent_t *ev, int precision,
