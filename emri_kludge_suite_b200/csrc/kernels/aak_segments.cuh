@@ -718,38 +718,6 @@ __global__ void __launch_bounds__(kSegWarps * 32, 2) k_tile_carries(BatchView bv
   }
 }
 
-// ------------------------------------------------------------------ sine and cosine
-// sin x and cos x in FP64 for |x| up to about 1e9: x = k pi/2 + r by a two-term
-// Cody-Waite reduction (fma keeps the product exact; the second term leaves
-// 1e-32 k), then the Taylor polynomials through r^15 and r^16, whose remainders
-// on |r| <= pi/4 are (pi/4)^16 / 17! = 6e-17 of sin and (pi/4)^18 / 18! = 2e-18.
-// The library's sincos takes its slow reduction above 1e5 rad, where the
-// orbital phase of a year-long source spends most of its samples.
-__device__ __forceinline__ void sincos_cw(double x, double &sn, double &cs) {
-  const double t = fma(x, 0.63661977236758134308, 6755399441055744.0);  // 1.5 x 2^52: k in the low bits
-  const int k = __double2loint(t);
-  const double kd = t - 6755399441055744.0;
-  const double r = fma(-kd, 6.123233995736766e-17, fma(-kd, 1.5707963267948966, x));
-  const double z = r * r;
-  double p = fma(z, -1. / 1307674368000., 1. / 6227020800.);
-  p = fma(z, p, -1. / 39916800.);
-  p = fma(z, p, 1. / 362880.);
-  p = fma(z, p, -1. / 5040.);
-  p = fma(z, p, 1. / 120.);
-  p = fma(z, p, -1. / 6.);
-  const double s = fma(r * z, p, r);
-  double q = fma(z, 1. / 20922789888000., -1. / 87178291200.);
-  q = fma(z, q, 1. / 479001600.);
-  q = fma(z, q, -1. / 3628800.);
-  q = fma(z, q, 1. / 40320.);
-  q = fma(z, q, -1. / 720.);
-  q = fma(z, q, 1. / 24.);
-  const double c = fma(z * z, q, fma(z, -.5, 1.0));
-  const double a = (k & 1) ? c : s, b = (k & 1) ? s : c;
-  sn = (k & 2) ? -a : a;
-  cs = ((k + 1) & 2) ? -b : b;
-}
-
 // Horner evaluation of coefficients at index OFF .. OFF + N - 1 of a segment (16-byte loads)
 template <int OFF, int N>
 __device__ __forceinline__ double seg_poly(const double2 *c, double x) {
@@ -762,7 +730,9 @@ __device__ __forceinline__ double seg_poly(const double2 *c, double x) {
 
 // ------------------------------------------------------------------ waveform kernel of the segments
 // What a sample needs before its mode sums, and after them.  w: the chain's
-// sign, 0 for the sample at t = 0, whose phases are the initial ones.
+// sign, 0 for the sample at t = 0, whose phases are the initial ones.  The
+// phases are those of the tile's head modulo 2 pi plus at most 1024 samples', so
+// that sincos stays in its fast range (below 1e5 rad).
 struct SegRotor {
   double c1, s1, cD, sD, dl;
 };
@@ -774,8 +744,8 @@ __device__ __forceinline__ SegRotor seg_rotor(const double2 *c, double x, double
   const double gd = seg_poly<Q, D + 1>(c, x), Pd = seg_poly<Q + (D + 1), D + 1>(c, x);
   const double e = seg_poly<Q + 4 * (D + 1), D + 1>(c, x), arm = seg_poly<Q + 9 * (D + 1), D + 1>(c, x);
   R.dl = e - H.ec;
-  sincos_cw(fma(Pd, arm, Phi), R.s1, R.c1);
-  sincos_cw(2.0 * gd * arm, R.sD, R.cD);
+  sincos(fma(Pd, arm, Phi), &R.s1, &R.c1);
+  sincos(2.0 * gd * arm, &R.sD, &R.cD);
   return R;
 }
 // h_I, h_II from the mode sums: the orientation (AAK.cc:425-440, RotCoeff
@@ -788,8 +758,8 @@ __device__ __forceinline__ void seg_output(const double2 *c, double x, double w,
   const double gim = H.hi[0] + fma(w, seg_poly<0, D + 2>(c, x), H.lo[0]);
   const double alp = H.hi[2] + fma(w, seg_poly<2 * (D + 2), D + 2>(c, x), H.lo[2]);
   double sa, ca, s2g, c2g;
-  sincos_cw(alp, sa, ca);
-  sincos_cw(2.0 * gim, s2g, c2g);
+  sincos(alp, &sa, &ca);
+  sincos(2.0 * gim, &s2g, &c2g);
   const double L0 = d.Lc[0] + sa * d.Ls[0] + ca * d.Lq[0];
   const double L1 = d.Lc[1] + sa * d.Ls[1] + ca * d.Lq[1];
   const double L2 = d.Lc[2] + ca * d.Lq[2];
