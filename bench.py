@@ -251,10 +251,10 @@ def cpu_likelihood_reference(procs: int = 0, sample_len: int = 200000) -> dict:
 
 # ----------------------------------------------------------------------------- likelihood (config 4)
 FIDUCIAL = np.array([0.785, 0.5, 8.0, 0.2, 1e6, 10.0, 0.0, 0.0, 0.0, 0.5, 1.0, 0.8, 2.0, 1.0])  # gpu_gen_AAK order
-# DRAM bytes (read + write) per sample of the split waveform kernel, from an ncu
-# capture of that kernel on all 512 sources of the configuration-1 draw cut to
-# an eighth of their length (bench.py --profile waveform512)
-TRAFFIC_BYTES_PER_SAMPLE = (923.200768e6 + 1849.097e6) / 108_999_922
+# DRAM bytes (read + write) per sample of k_wave_split, from an ncu capture of it
+# on all 512 sources of the configuration-1 draw cut to an eighth of their length
+# (bench.py --profile waveform512)
+TRAFFIC_BYTES_PER_SAMPLE = (924.052224e6 + 1894.4128e6) / 108_999_922
 LIKE_LENGTH = 3_200_000  # 1 yr at dt = 10 s rounded up to the 5-smooth FFT length 2^10 * 5^5
 
 
@@ -797,10 +797,10 @@ def run_gpu(args, rank, world, local_rank):
     for prec, name in ((0, "fp64"), (1, "split")):
         v, ms_v = wb.autotune(hI.data_ptr(), hII.data_ptr(), precision=prec)
         tune[name] = {"choice": v, "ms_per_variant": ms_v}
-    tune["variants"] = ["pre-pass, joint 1, 3 CTAs/SM", "tables inside the tiles, 2 CTAs/SM",
+    tune["variants"] = ["pre-pass, joint 1 (split) / 2 (FP64), 3 CTAs/SM", "everything inside the tiles, 2 CTAs/SM",
                         "pre-pass, joint 1 (split) / 2 (FP64), 2 CTAs/SM", "pre-pass, joint 4, 2 CTAs/SM",
-                        "pre-pass, joint 2 / 1, 3 CTAs/SM (split) / 2 CTAs/SM (FP64)",
-                        "pre-pass, joint 2, 2 CTAs/SM (split) / 3 CTAs/SM (FP64)"]
+                        "pre-pass, joint 2, 3 CTAs/SM (split) / joint 1, 2 CTAs/SM (FP64)",
+                        "pre-pass, joint 2, 2 CTAs/SM (split) / joint 1, 3 CTAs/SM (FP64)"]
 
     # ---- plain FP64 batched path (precision 0): per-kernel times
     for _ in range(args.warmup):
@@ -1038,7 +1038,7 @@ def run_gpu(args, rank, world, local_rank):
                 "achieved": achieved, "peak": fp32_peak,
                 "unit": "TFLOP/s", "frac": achieved / fp32_peak if fp32_peak > 0 else None,
                 "traffic": TRAFFIC_BYTES_PER_SAMPLE * N,
-                "traffic_source": "dram read+write per sample of one ncu capture of the same kernel on the 512 "
+                "traffic_source": "dram read+write per sample of one ncu capture of k_wave_split on the 512 "
                                   "sources of this draw cut to an eighth of their length (108,999,922 samples), "
                                   "scaled to this launch",
                 "peak_source": "measured FP32 FMA rate on this GPU (aak_probe_fp32_tflops)",
@@ -1111,11 +1111,10 @@ def run_gpu(args, rank, world, local_rank):
 #   python bench.py --profile likelihood # 32 config-4 templates, FP64 and FP32 transform + products
 def profile_waveform():
     """16 of the 512 configuration-1 sources (every 32nd; 28,332,971 samples,
-    n = 1..30): per precision the earlier default launch shape (FP64: 2
-    CTAs/SM; split: 2 samples per thread, 2 CTAs/SM) and the autotuner's
-    choice on the full batch (pre-pass, 1 sample per thread, 3 CTAs/SM: shape
-    0, the default now), twice each, in the order FP64 v4, FP64 v0, split v5,
-    split v0 (16 B/sample of outputs: 453 MB, above the 126 MB L2)."""
+    n = 1..30): per precision a shape with 2 CTAs/SM (FP64: one sample per
+    thread; split: two) and the default, shape 0 (3 CTAs/SM; FP64: two samples
+    per thread; split: one), twice each, in the order FP64 v4, FP64 v0, split
+    v5, split v0 (16 B/sample of outputs: 453 MB, above the 126 MB L2)."""
     import torch
 
     from emri_kludge_suite_b200.aak import WaveBatch

@@ -2273,7 +2273,7 @@ __global__ void __launch_bounds__(128) k_spline_coeffs(const SourceDesc *src, in
 // factors wait in shared memory; the right-hand sides of the block's own
 // unknowns wait in c itself, so that a CTA's 16 KB leave 13 of them on an SM
 // (all in shared memory: 7).  Bound by the latency of the chain and by its
-// instructions (43 % of the issue slots, 1.2 TB/s of memory).  Block lengths,
+// instructions (44 % of the issue slots, shared-memory and load pipe 61 %).  Block lengths,
 // 5e6 / 12e6 / 46e6 knots: 48 0.53 / 1.19 / 4.66 ms, 64 0.45 / 1.03 / 3.99, 96
 // 0.45 / 1.01 / 3.85, 128 0.49 / 1.07 / 4.08 (one thread a block of 256 knots:
 // 0.54 / 1.03 / 3.98, and 0.32 ms however few the knots; here 1e5 take 0.01).

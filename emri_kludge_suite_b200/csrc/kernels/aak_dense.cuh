@@ -130,10 +130,13 @@ constexpr WaveVariant wave_variant(bool split, int v) {
 
 // FP64 sources of at most this many tiles keep the single kernel that does
 // everything inside the tiles (one launch, the chain carried by look-back):
-// the segments' four launches one after another cost more than the few
-// tiles.  Four sources of 4 to 20 tiles: 41 us against 77; one of 100: 80
-// and 85.  The line is drawn by the source, not by the batch, so that a
-// source's samples do not depend on the batch it comes in.
+// the segments' four launches one after another cost more than the few tiles.
+// In the tile / as segments, us, caches flushed: one source of 25 tiles 55 / 92,
+// of 128 49 / 104; 4 of 64 75 / 123; 8 of 64 127 / 139; 16 of 25 121 / 118; 32 of
+// 25 188 / 156, of 64 399 / 256.  So up to about 500 tiles in all the single
+// kernel is the faster one, but the line is drawn by the source and not by the
+// launch, so that a source's samples do not depend on the batch it comes in, and
+// low enough that batches of sources just above it gain.
 constexpr int kSmallTiles = 24;
 
 // One work-queue item: a tile, its place in its source, and what staging it

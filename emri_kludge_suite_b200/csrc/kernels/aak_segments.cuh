@@ -667,7 +667,7 @@ __global__ void __launch_bounds__(kSegWarps * 32, 3) k_tile_segments(BatchView b
     }
     if (lane == 0) {
       if (mode == 0) {  // direct tiles from the list's front; those whose sums have no table, and take longest, from its end
-        if (P.K == 0) bv.direct_list[bv.total_tiles - 1 - atomicAdd(bv.seg_ctl + kCtlDirectSlow, 1)] = (int32_t)jq;
+        if (!kPhase && P.K <= 0) bv.direct_list[bv.total_tiles - 1 - atomicAdd(bv.seg_ctl + kCtlDirectSlow, 1)] = (int32_t)jq;
         else bv.direct_list[atomicAdd(bv.seg_ctl + kCtlDirectCount, 1)] = (int32_t)jq;
         atomicAdd(bv.seg_ctl + kCtlSource + it.s, 1);
       }
@@ -691,7 +691,7 @@ __global__ void __launch_bounds__(kSegWarps * 32, 3) k_tile_segments(BatchView b
 // build the tiles' Taylor tables, one thread a (tile, harmonic); the last ones
 // help with the direct tiles where there are more of those than carry blocks
 // (they come last so that the tables need not wait for them: 2344 direct tiles
-// 0.24 -> 0.13 ms).  The small sources are not the segments'.
+// 0.24 -> 0.15 ms).  The small sources are not the segments'.
 __global__ void __launch_bounds__(kSegWarps * 32, 2) k_tile_carries(BatchView bv, int carry_blocks, int table_blocks, int rows) {
   __shared__ CarryShared sh;
   const int blk = blockIdx.x, carriers = gridDim.x - table_blocks;

@@ -4,9 +4,9 @@
 //
 // A CTA takes one tile at a time from the work queue, in the passes of the
 // kernel that does everything inside the tile (the same operations and sums in
-// the same order), arranged for what bounded it: waits.  No pipe is saturated
-// (issue 63 %, FMA 30, FP64 20, LSU 32); the barriers and the copies at a
-// tile's start were 30 % of the time.  So
+// the same order), arranged for what bounds it: waits.  No pipe is saturated
+// (issue 64 % of the cycles, FMA 32, FP64 21, LSU 33); the barriers and the copies
+// at a tile's start were 30 % of that kernel's time.  So
 // - the next tile's record, parameters and knot window are requested while the
 //   last quarter of this tile's sums runs, and five barriers a tile stand for
 //   the ten of before;

@@ -169,7 +169,10 @@ int aak_batch_upload(aak_ctx *ctx, void *stream);
  * trajectory e, v, M, S, gamma~, Phi, alpha, nu, gamma~dot; diagnostic).
  * precision: 0 = FP64 throughout; 1 = split precision (FP64 spline, phases
  * and angle reductions; FP32 geometry, LISA response, Bessel evaluation and
- * harmonic recurrence). */
+ * harmonic recurrence).  FP64 sources of more than 24 tiles (1024 samples each)
+ * go through polynomial segments, which take 3.6 KB of device memory a tile on
+ * first use (the phase product 2.1 KB); where the device has none left they are
+ * generated inside the tiles, with the same values to rounding (1e-12). */
 int aak_batch_run(aak_ctx *ctx, double *d_hI, double *d_hII, double *d_t, double *d_traj, int64_t traj_stride,
                   int32_t precision, void *stream);
 
@@ -234,16 +237,18 @@ int aak_batch_last_launches(aak_ctx *ctx);
 int aak_batch_device_status(aak_ctx *ctx);
 
 /* Autotuner of the waveform stage's launch shape.  The candidates
- * (AAK_NUM_VARIANTS of them, per precision) are the tile pre-pass with bulk
- * copies or tables built inside the tiles, 1, 2 or 4 samples per thread in the
- * harmonic loop, and 2 or 3 resident CTAs per SM; tiles are 1024 samples in
+ * (AAK_NUM_VARIANTS of them, per precision) are the kernels with a tile
+ * pre-pass (FP64: polynomial segments, split: tables and bulk copies) or the
+ * one that does everything inside the tiles, 1, 2 or 4 samples per thread in
+ * the harmonic loop, and 2 or 3 resident CTAs per SM; tiles are 1024 samples in
  * every candidate (the host plan is laid out per tile).  On the context's
  * uploaded batch, with the caller's output buffers d_hI, d_hII, every
  * candidate runs once as a warm-up and twice timed (CUDA events); the fastest
  * becomes the context's choice for `precision`, used by aak_batch_run,
  * aak_batch_run_graph and the host-buffer entry points.  Key: device name and
- * SM count, precision, largest harmonic count, and the numbers of sources and
- * of samples of the median source in powers of two.  cache_path (optional): a
+ * SM count, the table of shapes that the index counts in, precision, largest
+ * harmonic count, and the numbers of sources and of samples of the median
+ * source in powers of two.  cache_path (optional): a
  * text file of "key variant ms_0 .. ms_5" lines; an entry for the key is used
  * without timing, a new choice is appended.  variant (optional) receives the
  * choice, ms_per_variant (optional, AAK_NUM_VARIANTS entries) the timings in
@@ -271,8 +276,9 @@ int aak_selftest_lookback_timeout(int64_t cycles);
 
 /* Per-kernel timing of aak_batch_run with CUDA events on its stream: after
  * aak_batch_set_profiling(ctx, 1), aak_batch_kernel_ms returns the durations
- * of (work-queue and look-back flag clears, the tile pre-pass -- 0 without
- * it --, the waveform kernel) of the last run in ms. */
+ * of (the clears, the tile pre-pass -- 0 without it; FP64: segments, carries
+ * and tables, with the small sources beside them --, the waveform kernels) of
+ * the last run in ms. */
 int aak_batch_set_profiling(aak_ctx *ctx, int32_t on);
 int aak_batch_kernel_ms(aak_ctx *ctx, float *ms3);
 
@@ -288,8 +294,8 @@ int aak_batch_run_plain(aak_ctx *ctx, double *d_hI, double *d_hII, double *d_tra
 
 /* The whole dense stage in one CUDA graph: the natural-spline solve of every
  * source's knots (as aak_batch_upload runs it; the same knots give the same
- * coefficients) and the three launches of aak_batch_run (no t / trajectory
- * outputs), captured on the first call for a given (d_hI, d_hII, precision,
+ * coefficients) and the launches of aak_batch_run (no t / trajectory outputs;
+ * FP64: two streams, forked and joined inside the graph), captured on the first call for a given (d_hI, d_hII, precision,
  * upload) and replayed on later calls; a new upload or other outputs
  * recapture.  Capture runs on a stream of the context, so `stream`
  * may be the legacy default stream.  No reference counterpart: the
