@@ -101,10 +101,10 @@ struct aak_ctx {
   int32_t large_steps = 0;  // index in queue_step of the second class
   std::vector<int64_t> kofs;       // nsrc + 1 prefix of knots (the sources' knots stay in their plans)
   std::vector<int64_t> spl_blk;    // nsrc + 1 prefix of the device spline solve's blocks: FP64, then split
-  // spline coefficients by the FP64 solve and by the split one, each made when its precision needs it; the next upload
+  // the spline coefficients on the device: by the FP64 solve (0) or the split one (1); -1: not known.  The next upload
   // makes those of the last launch
-  bool have_knot_c[2] = {false, false};
-  int last_knot_c = 0;
+  int knots = 0, last_knots = 0;
+  bool knots_captured = false;  // a graph of the caller's may write them whenever it runs: every launch solves for itself
   bool want_pinned = true;         // plans' knot arrays in page-locked memory
   std::vector<int32_t> bessel;
   int64_t total_samples = 0, total_tiles = 0, total_knots = 0;
@@ -118,7 +118,7 @@ struct aak_ctx {
   DevBuf<QueueItem> d_queue;
   DevBuf<int32_t> d_tile_knot, d_queue_rank;
   DevBuf<double> d_knot_t;
-  DevBuf<double4> d_knot_y, d_knot_c[2];
+  DevBuf<double4> d_knot_y, d_knot_c;
   DevBuf<int32_t> d_bessel;
   DevBuf<TileLink> d_link;                // look-back records, one per tile
   DevBuf<int32_t> d_flag;                 // look-back flags, one per tile
@@ -860,35 +860,25 @@ int with_room(aak_ctx *ctx, F f) {
 void solve_knots(aak_ctx *ctx, int k, cudaStream_t st) {
   const int64_t o = k ? ctx->nsrc + 1 : 0;
   launch_spline_coeffs(ctx->d_src.ptr, ctx->nsrc, ctx->d_spl_blk.ptr + o, ctx->spl_blk[o + ctx->nsrc], k != 0,
-                       ctx->d_knot_t.ptr, ctx->d_knot_y.ptr, ctx->d_knot_c[k].ptr, st);
+                       ctx->d_knot_t.ptr, ctx->d_knot_y.ptr, ctx->d_knot_c.ptr, st);
 }
-// After a solve was queued on `st`: the coefficients are there for later launches, unless the caller is capturing (they
-// are made when the caller's graph runs, and each capture makes its own).
+// After a solve (or a graph that holds one) was queued on `st`.  Where the caller is capturing it has not run.
 void note_knots(aak_ctx *ctx, int k, cudaStream_t st) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) ctx->have_knot_c[k] = true;
+  const bool runs = cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+  if (!runs) ctx->knots_captured = true;
+  ctx->knots = runs ? k : -1;
+  ctx->last_knots = k;
 }
-int reserve_knots(aak_ctx *ctx, int k) {
-  const size_t n = (size_t)std::max<int64_t>(ctx->total_knots, 1);
-  const int r = with_room(ctx, [&] { return ctx->d_knot_c[k].reserve(n); });
-  if (r != AAK_ERR_NO_MEMORY || !ctx->d_knot_c[1 - k].ptr) return r;
-  drop_graph(ctx);  // no room for both: the other precision's are made again when they are needed
-  ctx->d_knot_c[1 - k].release();
-  ctx->have_knot_c[1 - k] = false;
-  return ctx->d_knot_c[k].reserve(n);
-}
-// Before a launch in `precision`: its coefficients, set in bv.
-int need_knots(aak_ctx *ctx, int precision, cudaStream_t st, BatchView &bv) {
+// Before a launch in `precision`: its coefficients, solved for again where those on the device may be the other ones.
+// (Two arrays would spare the second solve, but a chunk of 256 templates has 1.5 GB of coefficients in each context.)
+void need_knots(aak_ctx *ctx, int precision, cudaStream_t st) {
   const int k = precision == 1;
-  if (!ctx->have_knot_c[k]) {
-    const int r = reserve_knots(ctx, k);
-    if (r != AAK_OK) return r;
-    solve_knots(ctx, k, st);
-    note_knots(ctx, k, st);
-  }
-  ctx->last_knot_c = k;
-  bv.knot_c = ctx->d_knot_c[k].ptr;
-  return AAK_OK;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  const bool capturing = cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;
+  if (ctx->knots == k && !ctx->knots_captured && !capturing) return;
+  solve_knots(ctx, k, st);
+  note_knots(ctx, k, st);
 }
 
 // wait_pinned: finish the copies from page-locked plan arrays before
@@ -908,8 +898,8 @@ int upload(aak_ctx *ctx, cudaStream_t st, bool wait_pinned = true) {
         (e = ctx->d_spl_blk.reserve(ctx->spl_blk.size())) ||
         // knot times: two entries of slack past the last knot (a window's bulk
         // copy starts on a 16-byte boundary and may read one element beyond it)
-        (e = ctx->d_knot_t.reserve(knots + 2)) || (e = ctx->d_knot_y.reserve(knots)) ||
-        (e = ctx->d_knot_c[ctx->last_knot_c].reserve(knots)) || (e = ctx->d_bessel.reserve(ctx->bessel.size())) ||
+        (e = ctx->d_knot_t.reserve(knots + 2)) || (e = ctx->d_knot_y.reserve(knots)) || (e = ctx->d_knot_c.reserve(knots)) ||
+        (e = ctx->d_bessel.reserve(ctx->bessel.size())) ||
         (e = ctx->d_link.reserve(tiles)) || (e = ctx->d_flag.reserve(tiles)) || (e = ctx->d_counter.reserve(2)))
       return e;
     return (int)AAK_OK;
@@ -941,9 +931,9 @@ int upload(aak_ctx *ctx, cudaStream_t st, bool wait_pinned = true) {
   // the tiles' knot windows and the work queue, and the spline coefficients of every source, made on the device
   launch_tile_layout(ctx->d_src.ptr, n, ctx->d_tile_start.ptr, ctx->total_tiles, ctx->d_knot_t.ptr, ctx->d_tile_knot.ptr,
                      ctx->d_queue.ptr, ctx->d_queue_rank.ptr, ctx->d_queue_step.ptr, ctx->large_steps, st);
-  ctx->have_knot_c[0] = ctx->have_knot_c[1] = false;
-  solve_knots(ctx, ctx->last_knot_c, st);
-  note_knots(ctx, ctx->last_knot_c, st);
+  ctx->knots_captured = false;
+  solve_knots(ctx, ctx->last_knots, st);
+  note_knots(ctx, ctx->last_knots, st);
   if ((r = cuda_ok(cudaGetLastError())) != AAK_OK) return r;
   // copies from page-locked memory run asynchronously: finish them before the
   // host arrays can be refilled by the next plan
@@ -1002,7 +992,7 @@ int run(aak_ctx *ctx, double *hI, double *hII, double *t, double *traj, int64_t 
   if (!traj && (r = tile_tables(ctx, precision, bv)) != AAK_OK) return r;
   if (ctx->profile && !ctx->ev[0])
     for (auto &e : ctx->ev) cudaEventCreate(&e);
-  if ((r = need_knots(ctx, precision, st, bv)) != AAK_OK) return r;
+  need_knots(ctx, precision, st);
   launch_dense(bv, ctx->num_sms, st, ctx->profile ? ctx->ev : nullptr, precision, &ctx->side);
   ctx->last_launches = dense_launches(ctx, precision, bv);
   return cuda_ok(cudaGetLastError());
@@ -1018,7 +1008,7 @@ int run_rows32(aak_ctx *ctx, float *hI32, float *hII32, int precision, cudaStrea
   bv.hII_f32 = hII32;
   bv.variant = ctx->variant[precision];
   if ((r = tile_tables(ctx, precision, bv)) != AAK_OK) return r;
-  if ((r = need_knots(ctx, precision, st, bv)) != AAK_OK) return r;
+  need_knots(ctx, precision, st);
   launch_dense(bv, ctx->num_sms, st, nullptr, precision);
   ctx->last_launches = 3;
   return cuda_ok(cudaGetLastError());
@@ -1047,8 +1037,7 @@ int run_graph(aak_ctx *ctx, double *hI, double *hII, int precision, cudaStream_t
     BatchView bv = batch_view(ctx, hI, hII, nullptr, nullptr, 0);
     bv.variant = ctx->variant[precision];
     const int k = precision == 1;
-    if ((r = tile_tables(ctx, precision, bv)) != AAK_OK || (r = reserve_knots(ctx, k)) != AAK_OK) return r;
-    bv.knot_c = ctx->d_knot_c[k].ptr;
+    if ((r = tile_tables(ctx, precision, bv)) != AAK_OK) return r;
     if ((r = cuda_ok(cudaStreamBeginCapture(ctx->cap_stream, cudaStreamCaptureModeThreadLocal))) != AAK_OK) return r;
     // the whole dense stage: natural-spline solve of every source's knots
     // (idempotent: the same knots give the same coefficients), then the clears
@@ -1074,9 +1063,8 @@ int run_graph(aak_ctx *ctx, double *hI, double *hII, int precision, cudaStream_t
     ctx->g_variant = ctx->variant[precision];
     ctx->g_launches = 1 + dense_launches(ctx, precision, bv);  // with the spline solve
   }
-  ctx->last_knot_c = precision == 1;
   ctx->last_launches = ctx->g_launches;
-  if ((r = cuda_ok(cudaGraphLaunch(ctx->gexec, st))) == AAK_OK) note_knots(ctx, ctx->last_knot_c, st);
+  if ((r = cuda_ok(cudaGraphLaunch(ctx->gexec, st))) == AAK_OK) note_knots(ctx, precision == 1, st);
   return r;
 }
 
@@ -1091,7 +1079,7 @@ BatchView batch_view(aak_ctx *ctx, double *hI, double *hII, double *t, double *t
   bv.tile_knot = ctx->d_tile_knot.ptr;
   bv.knot_t = ctx->d_knot_t.ptr;
   bv.knot_y = ctx->d_knot_y.ptr;
-  bv.knot_c = nullptr;  // need_knots
+  bv.knot_c = ctx->d_knot_c.ptr;
   bv.bessel_start = ctx->d_bessel.ptr;
   bv.link = ctx->d_link.ptr;
   bv.link_flag = ctx->d_flag.ptr;
@@ -1127,7 +1115,7 @@ int run_phase(aak_ctx *ctx, double *out, int64_t stride, cudaStream_t st) {
   if (ctx->small_tiles < ctx->total_tiles) tile_segments(ctx, bv, true);
   if (ctx->profile && !ctx->ev[0])
     for (auto &e : ctx->ev) cudaEventCreate(&e);
-  if ((r = need_knots(ctx, 0, st, bv)) != AAK_OK) return r;
+  need_knots(ctx, 0, st);
   launch_phase(bv, ctx->num_sms, st, ctx->profile ? ctx->ev : nullptr, &ctx->side);
   // small sources: tile parameters, phase pass, freeze; the others: segments, carries, phase pass
   ctx->last_launches = bv.tile_seg ? (ctx->small_tiles > 0 ? 3 : 0) + 3 : 3;
@@ -1156,6 +1144,7 @@ int run_plain(aak_ctx *ctx, double *hI, double *hII, double *traj, int64_t traj_
     v.tile_knot = ctx->d_tile_knot.ptr + 2 * d.tile_offset;
     v.knot_t = ctx->d_knot_t.ptr;
     v.knot_y = ctx->d_knot_y.ptr;
+    v.knot_c = ctx->d_knot_c.ptr;
     v.bessel_start = ctx->d_bessel.ptr;
     v.link = ctx->d_link.ptr + d.tile_offset;
     v.link_flag = ctx->d_flag.ptr + d.tile_offset;
@@ -1168,7 +1157,7 @@ int run_plain(aak_ctx *ctx, double *hI, double *hII, double *traj, int64_t traj_
     v.device_status = reinterpret_cast<unsigned int *>(ctx->d_counter.ptr + 1);
     v.trajectory_only = 1;
     v.max_nmodes = ctx->max_nmodes;
-    if ((r = need_knots(ctx, 0, st, v)) != AAK_OK) return r;
+    need_knots(ctx, 0, st);
     launch_dense(v, ctx->num_sms, st, nullptr, 0);
     launch_plain_waveform(ctx->d_src.ptr, s, d.vlength, traj, traj_stride, hI, hII, st);
     launches += 2;
@@ -1417,7 +1406,7 @@ int tdi_batch(aak_ctx *ctx, const aak_params *P, int32_t nsrc, int32_t nthreads,
   bv.phase_out = grid;
   bv.phase_stride = N;
   bv.trajectory_only = 1;
-  if ((r = need_knots(ctx, 0, 0, bv)) != AAK_OK) return r;
+  need_knots(ctx, 0, 0);
   launch_tdi_grid(bv, ctx->num_sms, 0, nullptr);
   if ((r = cuda_ok(cudaMemcpyAsync(ctx->d_tdi.ptr, td.data(), nsrc * sizeof(TdiDesc), cudaMemcpyHostToDevice, 0))) ||
       (r = cuda_ok(cudaMemcpyAsync(ctx->d_tdi_work.ptr, work.data(), (nsrc + 1) * sizeof(int64_t),
@@ -1673,7 +1662,7 @@ void aak_ctx_destroy(aak_ctx *c) {
       if (e) cudaEventDestroy(e);
     c->d_knot_t.release();
     c->d_knot_y.release();
-    for (auto &k : c->d_knot_c) k.release();
+    c->d_knot_c.release();
     c->d_bessel.release();
     c->d_link.release();
     c->d_flag.release();
@@ -1974,7 +1963,7 @@ int aak_ctx_autotune(aak_ctx *ctx, double *d_hI, double *d_hII, int32_t precisio
     ms[v] = 0.0f;
     for (int rep = 0; rep < 3 && r == AAK_OK; ++rep) {  // one warm-up, then the faster of two
       cudaEventRecord(e0, st);
-      if ((r = need_knots(ctx, precision, st, bv)) != AAK_OK) break;
+      need_knots(ctx, precision, st);
       launch_dense(bv, ctx->num_sms, st, nullptr, precision, &ctx->side);  // as run() launches it
       cudaEventRecord(e1, st);
       if ((r = cuda_ok(cudaEventSynchronize(e1))) != AAK_OK) break;
