@@ -72,7 +72,7 @@ int cuda_ok(cudaError_t e) { return cuda_status_of(e); }
 // What one dense launch writes for itself.  Nothing in it outlives the launch,
 // so that contexts whose launches follow one another on one stream may share it.
 struct DenseScratch {
-  DevBuf<TilePrep> prep;       // tile pre-pass: per-tile parameters
+  DevBuf<TilePrep> prep;       // tile pre-pass: per-tile parameters (with segments: in their memory)
   DevBuf<unsigned char> tab;   //   and per-tile Taylor tables
   DevBuf<unsigned char> seg[2];  // FP64 polynomial segments of the waveform and of the phase product (seg_parts)
   void release() {
@@ -803,15 +803,16 @@ void drop_graph(aak_ctx *ctx);
 
 // The memory of the FP64 polynomial segments of a launch, one allocation:
 // counters, the phases at i_plunge (phase product, 3 per source), the tiles'
-// phase increments, the direct tiles, and a slot per tile.
+// parameters and phase increments, the direct tiles, and a slot per tile.
 struct SegParts {
-  size_t frozen, agg, direct, slots, total;
+  size_t frozen, prep, agg, direct, slots, total;
 };
 SegParts seg_parts(int64_t tiles, int nsrc, bool phase) {
   const auto al = [](size_t x) { return (x + 255) / 256 * 256; };
   SegParts p;
   p.frozen = al(seg_ctl_words(nsrc) * sizeof(int32_t));
-  p.agg = p.frozen + al(phase ? 3 * (size_t)nsrc * sizeof(double) : 0);
+  p.prep = p.frozen + al(phase ? 3 * (size_t)nsrc * sizeof(double) : 0);
+  p.agg = p.prep + al((size_t)tiles * sizeof(TilePrep));
   p.direct = p.agg + al((size_t)tiles * sizeof(SegAgg));
   p.slots = p.direct + al((size_t)tiles * sizeof(int32_t));
   p.total = p.slots + (size_t)tiles * (phase ? kSegSlotBytesPhase : kSegSlotBytes);
@@ -842,6 +843,7 @@ void tile_segments(aak_ctx *ctx, BatchView &bv, bool phase) {
   unsigned char *b = buf.ptr;
   bv.seg_ctl = reinterpret_cast<int32_t *>(b);
   bv.frozen = phase ? reinterpret_cast<double *>(b + p.frozen) : nullptr;
+  bv.tile_prep = reinterpret_cast<TilePrep *>(b + p.prep);
   bv.tile_agg = reinterpret_cast<SegAgg *>(b + p.agg);
   bv.direct_list = reinterpret_cast<int32_t *>(b + p.direct);
   bv.tile_seg = b + p.slots;
@@ -959,23 +961,28 @@ int dense_launches(const aak_ctx *ctx, int precision, const BatchView &bv) {
 // The tile pre-pass buffers of a waveform launch in `precision` (one
 // TilePrep and one Taylor-table slot per tile), grown as needed, set in bv.
 int tile_tables(aak_ctx *ctx, int precision, BatchView &bv) {
-  // sources inside the in-tile kernel's sizes only: it needs none of this
-  if (precision == 0 && ctx->small_tiles == ctx->total_tiles) return AAK_OK;
+  const bool fp64 = precision == 0;
+  // FP64 inside the tiles only (the sources' sizes, the launch shape): none of this is used
+  if (fp64 && (ctx->small_tiles == ctx->total_tiles || !wave_variant(false, bv.variant).pre)) return AAK_OK;
   const int64_t tiles = std::max<int64_t>(ctx->total_tiles, 1);
   const int64_t slot = tile_table_slot_bytes(ctx->max_nmodes, precision == 1);
   DenseScratch &S = *ctx->scratch;
   const void *p0 = S.prep.ptr, *t0 = S.tab.ptr;
   const int r = with_room(ctx, [&] {
-    const int e = S.prep.reserve(tiles);
+    const int e = fp64 ? AAK_OK : S.prep.reserve(tiles);
     return e != AAK_OK ? e : S.tab.reserve(tiles * slot);
   });
-  if (r != AAK_OK) return r;
   // a captured dense graph holds the old buffers: recapture on its next use
   if (S.prep.ptr != p0 || S.tab.ptr != t0) drop_graph(ctx);
-  bv.tile_prep = S.prep.ptr;
+  if (r != AAK_OK) return fp64 && r == AAK_ERR_NO_MEMORY ? AAK_OK : r;  // FP64: inside the tiles then, without tables
+  if (fp64) {
+    tile_segments(ctx, bv, false);
+    if (!bv.tile_seg) return AAK_OK;
+  } else {
+    bv.tile_prep = S.prep.ptr;
+  }
   bv.tile_tab = S.tab.ptr;
   bv.tab_slot = slot;
-  if (precision == 0) tile_segments(ctx, bv, false);
   return AAK_OK;
 }
 
@@ -1107,12 +1114,14 @@ int run_phase(aak_ctx *ctx, double *out, int64_t stride, cudaStream_t st) {
   bv.phase_stride = stride;
   bv.trajectory_only = 1;
   // the tile pre-pass's parameters (no tables in the phase product)
-  DenseScratch &S = *ctx->scratch;
-  const void *p0 = S.prep.ptr;
-  if ((r = with_room(ctx, [&] { return S.prep.reserve(std::max<int64_t>(ctx->total_tiles, 1)); })) != AAK_OK) return r;
-  if (S.prep.ptr != p0) drop_graph(ctx);
-  bv.tile_prep = S.prep.ptr;
   if (ctx->small_tiles < ctx->total_tiles) tile_segments(ctx, bv, true);
+  if (!bv.tile_seg) {
+    DenseScratch &S = *ctx->scratch;
+    const void *p0 = S.prep.ptr;
+    if ((r = with_room(ctx, [&] { return S.prep.reserve(std::max<int64_t>(ctx->total_tiles, 1)); })) != AAK_OK) return r;
+    if (S.prep.ptr != p0) drop_graph(ctx);
+    bv.tile_prep = S.prep.ptr;
+  }
   if (ctx->profile && !ctx->ev[0])
     for (auto &e : ctx->ev) cudaEventCreate(&e);
   need_knots(ctx, 0, st);
